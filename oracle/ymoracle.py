@@ -31,7 +31,7 @@ def reference_tree():
     """The reference's source tree: $YM_REFERENCE, else a checkout named
     `reference` beside this repository; None where neither exists."""
     p = Path(os.environ["YM_REFERENCE"]) if os.environ.get("YM_REFERENCE") else HERE.parent.parent / "reference"
-    return p if p.is_dir() else None
+    return p if (p / "src").is_dir() else None
 
 
 def build() -> None:
