@@ -254,13 +254,8 @@ __device__ __forceinline__ void split_link_update_to(const F& in, const F& out,
         const R sg = mu < nu ? R(1) : R(-1);
         const int y = g.hop_rt(s, g.coord(c, nu), nu, -1);
         const M3<R> v = in.load(nu, y);
-        const Herm8<R> lower = herm_conj_by(v, hf.load_ro(p, y));
-        const Herm8<R> upper = hf.load_ro(p, s);
-        d.d0 = fma(sg, upper.d0 - lower.d0, d.d0);
-        d.d1 = fma(sg, upper.d1 - lower.d1, d.d1);
-        d.z01 = cx(fma(sg, upper.z01.re - lower.z01.re, d.z01.re), fma(sg, upper.z01.im - lower.z01.im, d.z01.im));
-        d.z02 = cx(fma(sg, upper.z02.re - lower.z02.re, d.z02.re), fma(sg, upper.z02.im - lower.z02.im, d.z02.im));
-        d.z12 = cx(fma(sg, upper.z12.re - lower.z12.re, d.z12.re), fma(sg, upper.z12.im - lower.z12.im, d.z12.im));
+        d = h8_axpy(sg, hf.load_ro(p, s), d);
+        herm_conj_add(v, h8_scale(-sg, hf.load_ro(p, y)), d);
     }
     const M3<R> uu = in.load(mu, s);
     const Rows2<R> un = rk_finish<F, STAGE>(out, zf, eps, s, mu, d, uu);

@@ -218,12 +218,8 @@ __device__ __forceinline__ void tile_unit(const F& in, const F& out, const Force
                 }
                 const int y = g.hop_rt(s, g.coord(c, nu), nu, -1);
                 const M3<R> v = in.load(nu, y);
-                const Herm8<R> lower = herm_conj_by(v, HV::get(lb + li, ln));
-                d.d0 = fma(sg, upper.d0 - lower.d0, d.d0);
-                d.d1 = fma(sg, upper.d1 - lower.d1, d.d1);
-                d.z01 = cx(fma(sg, upper.z01.re - lower.z01.re, d.z01.re), fma(sg, upper.z01.im - lower.z01.im, d.z01.im));
-                d.z02 = cx(fma(sg, upper.z02.re - lower.z02.re, d.z02.re), fma(sg, upper.z02.im - lower.z02.im, d.z02.im));
-                d.z12 = cx(fma(sg, upper.z12.re - lower.z12.re, d.z12.re), fma(sg, upper.z12.im - lower.z12.im, d.z12.im));
+                d = h8_axpy(sg, upper, d);
+                herm_conj_add(v, h8_scale(-sg, HV::get(lb + li, ln)), d);
             }
             const M3<R> uu = in.load(mu, s);
             rk_finish<F, STAGE>(out, zf, eps, s, mu, d, uu);

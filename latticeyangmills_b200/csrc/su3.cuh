@@ -123,17 +123,23 @@ __device__ __forceinline__ R re_trace_mul(const M3<R>& a, const M3<R>& b) {
     return s;
 }
 
-// Row 2 of an SU(3) matrix from rows 0 and 1: r2 = conj(r0 x r1).
+// Entry k of row 2 of the SU(3) matrix whose rows 0 and 1 are those of a
+// (M3 or Rows2): conj(r0 x r1).  Every multiply-add is written out, so every
+// kernel rebuilds the same row 2 bit for bit.
+template <class R, class M>
+__device__ __forceinline__ Cx<R> row2_entry_of(const M& a, int k) {
+    const int i = (k + 1) % 3, j = (k + 2) % 3;
+    const Cx<R> p = a.e[0][i], q = a.e[1][j], r = a.e[0][j], s = a.e[1][i];
+    const R re = fma(p.re, q.re, fma(-p.im, q.im, -fma(r.re, s.re, -r.im * s.im)));
+    const R im = fma(p.re, q.im, fma(p.im, q.re, -fma(r.re, s.im, r.im * s.re)));
+    return cx(re, -im);
+}
+
+// Row 2 of an SU(3) matrix from rows 0 and 1.
 template <class R>
 __device__ __forceinline__ void reconstruct_row2(M3<R>& a) {
 #pragma unroll
-    for (int k = 0; k < 3; k++) {
-        const int i = (k + 1) % 3, j = (k + 2) % 3;
-        const Cx<R> p = a.e[0][i], q = a.e[1][j], r = a.e[0][j], s = a.e[1][i];
-        R re = p.re * q.re - p.im * q.im - (r.re * s.re - r.im * s.im);
-        R im = p.re * q.im + p.im * q.re - (r.re * s.im + r.im * s.re);
-        a.e[2][k] = cx(re, -im);
-    }
+    for (int k = 0; k < 3; k++) a.e[2][k] = row2_entry_of<R>(a, k);
 }
 
 // ---------------------------------------------------------------------------
@@ -173,14 +179,10 @@ __device__ __forceinline__ void mmul_rows2(const MA& a, const M3<R>& b, Rows2<R>
     }
 }
 
-// row 2 of an SU(3) matrix given by its first two rows: conj(r0 x r1), entry k
+// row 2 of an SU(3) matrix given by its first two rows, entry k
 template <class R>
 __device__ __forceinline__ Cx<R> row2_entry(const Rows2<R>& a, int k) {
-    const int i = (k + 1) % 3, j = (k + 2) % 3;
-    const Cx<R> p = a.e[0][i], q = a.e[1][j], r = a.e[0][j], s = a.e[1][i];
-    const R re = fma(p.re, q.re, fma(-p.im, q.im, -fma(r.re, s.re, -r.im * s.im)));
-    const R im = fma(p.re, q.im, fma(p.im, q.re, -fma(r.re, s.im, r.im * s.re)));
-    return cx(re, -im);
+    return row2_entry_of<R>(a, k);
 }
 
 // acc += the SU(3) matrix whose first two rows are a
@@ -366,53 +368,57 @@ __device__ __forceinline__ Herm8<R> force_from_b2_cdag(const Rows2<R>& b, const 
     return z;
 }
 
-// v^+ h v for a Hermitian traceless h: Hermitian and traceless again, so only
-// its diagonal d0, d1 and upper triangle are formed.  W = h v uses h's real
-// diagonal (h22 = -d0 - d1) and conjugate lower triangle.
+// acc += v^+ h v for a Hermitian traceless h and v in SU(3) (Hermitian and
+// traceless again: its diagonal d0, d1 and upper triangle are formed).  With
+// d2 = h22, v^+ h v = v^+ (h - d2) v + d2, and h - d2 = A + A^+ for the upper
+// triangular A with half its diagonal, whose third row is zero: w = A v has
+// two rows, and v^+ (h - d2) v = v^+ w + (v^+ w)^+ sums over two rows of v.
+// 113 multiply-adds, against 139 for h v and the needed entries of v^+ (h v).
+// The stage kernel that makes three of these per link is bound by its issue
+// slots: at 32^4 on B200 0.165 -> 0.148 ms per launch (FP32-12, with the row 2
+// of the links in four multiply-adds per component instead of five), 0.167 ->
+// 0.160 (FP32-18), 0.350 -> 0.337 (FP64).
 template <class R>
-__device__ __forceinline__ Herm8<R> herm_conj_by(const M3<R>& v, const Herm8<R>& h) {
+__device__ __forceinline__ void herm_conj_add(const M3<R>& v, const Herm8<R>& h, Herm8<R>& acc) {
     const R d2 = -(h.d0 + h.d1);
-    M3<R> w;
+    const R a0 = R(0.5) * (h.d0 - d2), a1 = R(0.5) * (h.d1 - d2);
+    Rows2<R> w;
 #pragma unroll
     for (int j = 0; j < 3; j++) {
         const Cx<R> a = v.e[0][j], b = v.e[1][j], c = v.e[2][j];
-        // row 0: d0 a + z01 b + z02 c
-        w.e[0][j].re = fma(h.d0, a.re, fma(h.z01.re, b.re, fma(-h.z01.im, b.im, fma(h.z02.re, c.re, -h.z02.im * c.im))));
-        w.e[0][j].im = fma(h.d0, a.im, fma(h.z01.re, b.im, fma(h.z01.im, b.re, fma(h.z02.re, c.im, h.z02.im * c.re))));
-        // row 1: conj(z01) a + d1 b + z12 c
-        w.e[1][j].re = fma(h.z01.re, a.re, fma(h.z01.im, a.im, fma(h.d1, b.re, fma(h.z12.re, c.re, -h.z12.im * c.im))));
-        w.e[1][j].im = fma(h.z01.re, a.im, fma(-h.z01.im, a.re, fma(h.d1, b.im, fma(h.z12.re, c.im, h.z12.im * c.re))));
-        // row 2: conj(z02) a + conj(z12) b + d2 c
-        w.e[2][j].re = fma(h.z02.re, a.re, fma(h.z02.im, a.im, fma(h.z12.re, b.re, fma(h.z12.im, b.im, d2 * c.re))));
-        w.e[2][j].im = fma(h.z02.re, a.im, fma(-h.z02.im, a.re, fma(h.z12.re, b.im, fma(-h.z12.im, b.re, d2 * c.im))));
+        // row 0: a0 a + z01 b + z02 c
+        w.e[0][j].re = fma(a0, a.re, fma(h.z01.re, b.re, fma(-h.z01.im, b.im, fma(h.z02.re, c.re, -h.z02.im * c.im))));
+        w.e[0][j].im = fma(a0, a.im, fma(h.z01.re, b.im, fma(h.z01.im, b.re, fma(h.z02.re, c.im, h.z02.im * c.re))));
+        // row 1: a1 b + z12 c
+        w.e[1][j].re = fma(a1, b.re, fma(h.z12.re, c.re, -h.z12.im * c.im));
+        w.e[1][j].im = fma(a1, b.im, fma(h.z12.re, c.im, h.z12.im * c.re));
     }
-    auto entry = [&](int i, int j) {  // (v^+ w)_ij = sum_k conj(v_ki) w_kj
-        R re = R(0), im = R(0);
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            re = fma(v.e[k][i].re, w.e[k][j].re, re);
-            re = fma(v.e[k][i].im, w.e[k][j].im, re);
-            im = fma(v.e[k][i].re, w.e[k][j].im, im);
-            im = fma(-v.e[k][i].im, w.e[k][j].re, im);
-        }
-        return cx(re, im);
+    auto diag = [&](int i, R& out) {  // out += d2 + 2 Re (v^+ w)_ii
+        R re = v.e[0][i].re * w.e[0][i].re;
+        re = fma(v.e[0][i].im, w.e[0][i].im, re);
+        re = fma(v.e[1][i].re, w.e[1][i].re, re);
+        re = fma(v.e[1][i].im, w.e[1][i].im, re);
+        out = fma(R(2), re, out + d2);
     };
-    auto diag_re = [&](int i) {
-        R re = R(0);
+    auto entry = [&](int i, int j, Cx<R>& out) {  // out += (v^+ w)_ij + conj((v^+ w)_ji)
 #pragma unroll
-        for (int k = 0; k < 3; k++) {
-            re = fma(v.e[k][i].re, w.e[k][i].re, re);
-            re = fma(v.e[k][i].im, w.e[k][i].im, re);
+        for (int k = 0; k < 2; k++) {
+            const Cx<R> vi = v.e[k][i], vj = v.e[k][j], wi = w.e[k][i], wj = w.e[k][j];
+            out.re = fma(vi.re, wj.re, out.re);
+            out.re = fma(vi.im, wj.im, out.re);
+            out.re = fma(vj.re, wi.re, out.re);
+            out.re = fma(vj.im, wi.im, out.re);
+            out.im = fma(vi.re, wj.im, out.im);
+            out.im = fma(-vi.im, wj.re, out.im);
+            out.im = fma(vj.im, wi.re, out.im);
+            out.im = fma(-vj.re, wi.im, out.im);
         }
-        return re;
     };
-    Herm8<R> r;
-    r.d0 = diag_re(0);
-    r.d1 = diag_re(1);
-    r.z01 = entry(0, 1);
-    r.z02 = entry(0, 2);
-    r.z12 = entry(1, 2);
-    return r;
+    diag(0, acc.d0);
+    diag(1, acc.d1);
+    entry(0, 1, acc.z01);
+    entry(0, 2, acc.z02);
+    entry(1, 2, acc.z12);
 }
 
 template <class R>
@@ -426,14 +432,32 @@ __device__ __forceinline__ Herm8<R> h8_axpby(R a, const Herm8<R>& x, R b, const 
     return r;
 }
 
+// A product that the compiler leaves rounded as it stands: contracted into the
+// sums that use it or not, it would make kernels that share this code differ
+// by rounding.
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
 template <class R>
 __device__ __forceinline__ Herm8<R> h8_scale(R a, const Herm8<R>& x) {
     Herm8<R> r;
-    r.d0 = a * x.d0;
-    r.d1 = a * x.d1;
-    r.z01 = cx(a * x.z01.re, a * x.z01.im);
-    r.z02 = cx(a * x.z02.re, a * x.z02.im);
-    r.z12 = cx(a * x.z12.re, a * x.z12.im);
+    r.d0 = mul_rn(a, x.d0);
+    r.d1 = mul_rn(a, x.d1);
+    r.z01 = cx(mul_rn(a, x.z01.re), mul_rn(a, x.z01.im));
+    r.z02 = cx(mul_rn(a, x.z02.re), mul_rn(a, x.z02.im));
+    r.z12 = cx(mul_rn(a, x.z12.re), mul_rn(a, x.z12.im));
+    return r;
+}
+
+// a x + y
+template <class R>
+__device__ __forceinline__ Herm8<R> h8_axpy(R a, const Herm8<R>& x, const Herm8<R>& y) {
+    Herm8<R> r;
+    r.d0 = fma(a, x.d0, y.d0);
+    r.d1 = fma(a, x.d1, y.d1);
+    r.z01 = cx(fma(a, x.z01.re, y.z01.re), fma(a, x.z01.im, y.z01.im));
+    r.z02 = cx(fma(a, x.z02.re, y.z02.re), fma(a, x.z02.im, y.z02.im));
+    r.z12 = cx(fma(a, x.z12.re, y.z12.re), fma(a, x.z12.im, y.z12.im));
     return r;
 }
 
