@@ -29,15 +29,16 @@ struct ymflow_ctx {
     int timed_reunit = 0;             // time_steps / time_kernels: reunitarise every n-th step (0: never)
     double* staging = nullptr;        // .bin-layout device buffer for upload/download
     size_t staging_bytes = 0;
-    double* partials = nullptr;       // observables: 3 doubles per block
-    int partial_cap = 0;
+    double* partials = nullptr;       // observables: block partials
+    int partial_cap = 0;              // in doubles
     double* meas = nullptr;           // measurement rows on the device, 4 doubles each
     int meas_cap = 0;
     double* meas_host = nullptr;      // pinned copy of the rows
     unsigned long long* deviation = nullptr;  // reunitarisation drift (ordered bits)
-    cudaGraphExec_t graph[2] = {nullptr, nullptr};
-    double graph_eps[2] = {0.0, 0.0};
-    int graph_block[2] = {0, 0};
+    // the step from u[k & 1]; k & 2: with its plaquette field ready
+    cudaGraphExec_t graph[4] = {nullptr, nullptr, nullptr, nullptr};
+    double graph_eps[4] = {0.0, 0.0, 0.0, 0.0};
+    int graph_block[4] = {0, 0, 0, 0};
     std::vector<cudaEvent_t> events;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int block = 128;

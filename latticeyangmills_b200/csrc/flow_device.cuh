@@ -185,10 +185,11 @@ __device__ __forceinline__ int plane_index(int a, int b) { return a * (5 - a) / 
 __device__ __forceinline__ int plane_a(int p) { return p < 3 ? 0 : (p < 5 ? 1 : 2); }
 __device__ __forceinline__ int plane_b(int p) { return p < 3 ? p + 1 : (p < 5 ? p - 1 : 3); }
 
-// H_ab(x) = (i/2)[P_ab(x) - P_ab(x)^+]_TL at site s with coordinates c.
+// H_ab(x) = (i/2)[P_ab(x) - P_ab(x)^+]_TL at site s with coordinates c;
+// trace (optional): Re tr P_ab(x).
 template <class F>
 __device__ __forceinline__ Herm8<typename F::Real> plane_generator(const F& u, const Geo& g, int s, const int c[4],
-                                                                   int a, int b) {
+                                                                   int a, int b, typename F::Real* trace = nullptr) {
     using R = typename F::Real;
     const int s_pa = g.hop_rt(s, g.coord(c, a), a, +1);
     const int s_pb = g.hop_rt(s, g.coord(c, b), b, +1);
@@ -216,7 +217,7 @@ __device__ __forceinline__ Herm8<typename F::Real> plane_generator(const F& u, c
         mmul_rows2<false, false>(x, y, t);
         full_from_rows2(t, up);
     }
-    return force_from_b2_cdag(lo, up);
+    return force_from_b2_cdag(lo, up, trace);
 }
 
 // H_p(x) of plane p at site s into hf.

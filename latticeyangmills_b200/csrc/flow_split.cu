@@ -21,6 +21,7 @@
 // read.
 #include "flow_device.cuh"
 #include "kernels.h"
+#include "observables.cuh"
 
 namespace ym {
 
@@ -137,6 +138,69 @@ static cudaError_t launch_split_typed(int stage, const void* uin, void* uout, vo
         default: rk_split_stage_kernel<F, 2><<<grid, 128, 0, st>>>(in, out, zf, hf, g, e); break;
     }
     return cudaGetLastError();
+}
+
+// The plaquette-field kernel of a measurement: the same field, and the sum of
+// Re tr P over the sites [count0, count1) that are the context's own, one
+// FP64 partial per warp (no barrier: a block's warps retire apart, as in
+// plaq_field_kernel; one partial per block after a barrier ran 0.123 / 0.154 ms
+// in FP32-12 / -18 at 32^4 on B200 against 0.112 / 0.123).  FP64 takes 96
+// registers at three resident blocks: 0.255 ms, against 0.291 at
+// plaq_field_kernel's 80.
+template <class F>
+__global__ void __launch_bounds__(192, sizeof(typename F::Real) == 8 ? 3 : PlaqMinBlocks<F>::value)
+    plaq_field_sum_kernel(F u, ForceField<typename F::Real> hf, Geo g, int count0, int count1, double* partials) {
+    using R = typename F::Real;
+    constexpr int kPlanes = PlaqPlanesPerThread<F>::value;
+    const int w = int(threadIdx.x >> 5);
+    const int s = g.site0 + (int(blockIdx.x) * kPlanes + (kPlanes == 1 ? 0 : w / 3)) * 32 + int(threadIdx.x & 31);
+    R t0 = R(0), t1 = R(0);
+    bool counts = false;
+    if (s < g.site1) {
+        int c[4];
+        g.coords(s, c);
+        counts = s >= count0 && s < count1 && g.interior(c);
+        if (kPlanes == 1) {
+            hf.store(w, s, plane_generator(u, g, s, c, plane_a(w), plane_b(w), &t0));
+        } else {
+            const int pr = w % 3;
+            const int p0 = pr == 0 ? 0 : (pr == 1 ? 2 : 3);
+            const int p1 = pr == 0 ? 1 : (pr == 1 ? 4 : 5);
+            const auto h0 = plane_generator(u, g, s, c, plane_a(p0), plane_b(p0), &t0);
+            const auto h1 = plane_generator(u, g, s, c, plane_a(p1), plane_b(p1), &t1);
+            hf.store(p0, s, h0);
+            hf.store(p1, s, h1);
+        }
+    }
+    const double sum = warp_sum(counts ? double(t0) + double(t1) : 0.0);
+    if ((threadIdx.x & 31) == 0) partials[int64_t(blockIdx.x) * 6 + w] = sum;
+}
+
+static int plaq_blocks(int prec, const Geo& g) {
+    const int groups = (g.site1 - g.site0 + 31) / 32;
+    return prec == kFP64 ? groups : (groups + 1) / 2;
+}
+
+int plaq_sum_partials(int prec, const Geo& g) { return 6 * plaq_blocks(prec, g); }
+
+template <class F>
+static cudaError_t launch_plaq_sum_typed(const void* u, void* h, const Geo& g, int count0, int count1,
+                                         double* partials, cudaStream_t st) {
+    F in{const_cast<void*>(u), g.V};
+    ForceField<typename F::Real> hf{h, g.V};
+    plaq_field_sum_kernel<F><<<plaq_blocks(sizeof(typename F::Real) == 8 ? kFP64 : kFP32_18, g), 192, 0, st>>>(in, hf, g, count0, count1, partials);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_plaq_field_sum(int prec, const void* u, void* h, const Geo& g, int count0, int count1,
+                                  double* partials, cudaStream_t st) {
+    if (g.site1 <= g.site0) return cudaErrorInvalidValue;
+    switch (prec) {
+        case kFP64: return launch_plaq_sum_typed<FieldD18>(u, h, g, count0, count1, partials, st);
+        case kFP32_18: return launch_plaq_sum_typed<FieldF18>(u, h, g, count0, count1, partials, st);
+        case kFP32_12: return launch_plaq_sum_typed<FieldF12>(u, h, g, count0, count1, partials, st);
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 cudaError_t launch_plaq_field(int prec, const void* u, void* h, const Geo& g, cudaStream_t st) {

@@ -98,6 +98,20 @@ int obs_blocks(const Geo& g);
 cudaError_t launch_observables(int prec, const void* u, const Geo& g, double* partials, cudaStream_t st);
 cudaError_t launch_obs_finalize(const double* partials, int nblocks, const Geo& g, double* out, cudaStream_t st);
 
+// The same row (out[0..3]) through the plaquette field, in three launches: the
+// field of u over `field`'s sites into h (which then holds u's plaquette field,
+// as after launch_plaq_field) with the plaquette sums, energy and charge from
+// it over `own`'s sites, and the fold.  `partials` holds measure_partials
+// doubles.  The energy and charge kernel's blocks stride over the sites beyond
+// kCloverMaxBlocks.
+constexpr int kCloverMaxBlocks = 148 * 20;
+int plaq_sum_partials(int prec, const Geo& g);
+cudaError_t launch_plaq_field_sum(int prec, const void* u, void* h, const Geo& g, int count0, int count1,
+                                  double* partials, cudaStream_t st);
+int measure_partials(int prec, const Geo& field, const Geo& own);
+cudaError_t launch_measure_from_field(int prec, const void* u, void* h, const Geo& field, const Geo& own,
+                                      double* partials, double* out, cudaStream_t st);
+
 // .bin layout (site-major, mu, 18 doubles) <-> device layout
 // Sites [first, first + n) between a .bin-layout block (aos points at site
 // `first`) and the device links; swap = each double byte-reversed.

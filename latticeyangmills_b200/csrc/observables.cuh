@@ -3,6 +3,7 @@
 // observables.cu and any kernel that needs the same reduction.
 #pragma once
 #include "field.cuh"
+#include "flow_device.cuh"
 #include "su3.cuh"
 
 namespace ym {
@@ -227,6 +228,98 @@ __global__ void __launch_bounds__(kObsThreads, kObsMinBlocks)
     block_sum3(plaq, energy, topc);
     if (threadIdx.x == 0) {
         partials[3 * blockIdx.x + 0] = plaq;
+        partials[3 * blockIdx.x + 1] = energy;
+        partials[3 * blockIdx.x + 2] = topc;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The same observables from a stored plaquette field (the two-kernel stage's
+// H_p = (i/2)[P_p - P_p^+]_TL).  The four leaves of a clover are the plaquettes
+// of x, x - mu, x - nu and x - mu - nu carried to x, and (i/2)[.]_TL commutes
+// with that conjugation, so the clover's traceless anti-Hermitian part is
+// -2i S with
+//   S(x) = H(x) + V^+ H(x-nu) V + W^+ [ H(x-mu) + Y^+ H(x-mu-nu) Y ] W,
+//   V = U_nu(x-nu),  W = U_mu(x-mu),  Y = U_nu(x-mu-nu):
+// three transports of 113 multiply-adds per plane in place of four products
+// of four links (about 1000).  Bound by latency and arithmetic (FP64 pipe at
+// about 53 %), not by HBM.  A measured step at 32^4 on B200 spends, beyond its
+// six stage launches, 0.28 ms in FP64 (observables_kernel: 0.78), 0.15 in
+// FP32-18 (0.41) and 0.15 in FP32-12 (0.45): this kernel 0.245 / 0.137 / 0.139,
+// the sums in the field kernel 0.023 / 0.009 / 0.007 (the field itself is the
+// next stage's), the fold 0.005.
+// ---------------------------------------------------------------------------
+template <class F>
+__device__ __forceinline__ Herm8<typename F::Real> clover_generator(const F& u,
+                                                                    const ForceField<typename F::Real>& hf,
+                                                                    const Geo& g, int s, const int c[4], int mu,
+                                                                    int nu) {
+    using R = typename F::Real;
+    const int p = plane_index(mu, nu);
+    const int s_mm = g.hop_rt(s, g.coord(c, mu), mu, -1);
+    const int s_mn = g.hop_rt(s, g.coord(c, nu), nu, -1);
+    const int s_mm_mn = g.hop_rt(s_mm, g.coord(c, nu), nu, -1);
+    Herm8<R> back = hf.load_ro(p, s_mm);
+    herm_conj_add(u.load(nu, s_mm_mn), hf.load_ro(p, s_mm_mn), back);
+    Herm8<R> sum = hf.load_ro(p, s);
+    herm_conj_add(u.load(nu, s_mn), hf.load_ro(p, s_mn), sum);
+    herm_conj_add(u.load(mu, s_mm), back, sum);
+    return sum;
+}
+
+// tr(a b) of Hermitian traceless a, b.
+template <class R>
+__device__ __forceinline__ R herm_trace_mul(const Herm8<R>& a, const Herm8<R>& b) {
+    const R d = fma(a.d0, b.d0, fma(a.d1, b.d1, (a.d0 + a.d1) * (b.d0 + b.d1)));
+    const R o = fma(a.z01.re, b.z01.re, fma(a.z01.im, b.z01.im, fma(a.z02.re, b.z02.re, fma(a.z02.im, b.z02.im,
+                fma(a.z12.re, b.z12.re, a.z12.im * b.z12.im)))));
+    return fma(R(2), o, d);
+}
+
+// Resident 96-thread blocks: FP64 5 (128 registers, 15 warps per SM; a plane
+// pair with one transport live needs all of them), FP32 10 (64, 30 warps).
+template <class F>
+struct CloverMinBlocks {
+    static constexpr int value = sizeof(typename F::Real) == 8 ? 5 : 10;
+};
+
+// One thread per (site, pair of planes): the pairs (01,23), (02,13), (03,12)
+// that the charge multiplies, so nothing passes between threads; three warps
+// per 32 sites.  Three partials per block, as observables_kernel's: block b's
+// share of the field kernel's nplaq plaquette partials (folded here, so that
+// the last fold reads a bounded number), energy and charge.  A thread's
+// running sums wait in shared memory, not in registers.
+template <class F>
+__global__ void __launch_bounds__(96, CloverMinBlocks<F>::value)
+    clover_field_kernel(F u, ForceField<typename F::Real> hf, Geo g, const double* plaq, int nplaq, double* partials) {
+    __shared__ double sums[2][96];
+    sums[0][threadIdx.x] = sums[1][threadIdx.x] = 0.0;
+    const int k = int(threadIdx.x >> 5);
+    const int mu_b = k == 0 ? 2 : 1;
+    const int nu_b = k == 2 ? 2 : 3;
+    const int items = (g.site1 - g.site0 + 31) / 32;
+    for (int item = blockIdx.x; item < items; item += gridDim.x) {
+        const int s = g.site0 + item * 32 + int(threadIdx.x & 31);
+        if (s >= g.site1) continue;
+        int c[4];
+        g.coords(s, c);
+        if (!g.interior(c)) continue;  // a block's halo sites are its neighbours'
+        const auto a = clover_generator(u, hf, g, s, c, 0, k + 1);
+        const auto b = clover_generator(u, hf, g, s, c, mu_b, nu_b);
+        // Re tr(G_a G_b) = -4 tr(S_a S_b); the pairs' signs as in site_observables
+        sums[0][threadIdx.x] -= 4.0 * (double(herm_trace_mul(a, a)) + double(herm_trace_mul(b, b)));
+        const double t = 4.0 * double(herm_trace_mul(a, b));
+        sums[1][threadIdx.x] += k == 1 ? -t : t;
+    }
+    const int share = (nplaq + int(gridDim.x) - 1) / int(gridDim.x);
+    double p = 0.0, energy = sums[0][threadIdx.x], topc = sums[1][threadIdx.x];
+    for (int i = threadIdx.x; i < share; i += blockDim.x) {
+        const int j = int(blockIdx.x) * share + i;
+        if (j < nplaq) p += plaq[j];
+    }
+    block_sum3(p, energy, topc);
+    if (threadIdx.x == 0) {
+        partials[3 * blockIdx.x + 0] = p;
         partials[3 * blockIdx.x + 1] = energy;
         partials[3 * blockIdx.x + 2] = topc;
     }

@@ -37,6 +37,12 @@ __device__ __forceinline__ Cx<R> cx(R re, R im) {
     return c;
 }
 
+// A product that the compiler leaves rounded as it stands: contracted into the
+// sums that use it or not, it would make kernels that share this code differ
+// by rounding.
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
 // c = op(a) * op(b) with op = identity or dagger (DA / DB).
 template <bool DA, bool DB, class R>
 __device__ __forceinline__ void mmul(const M3<R>& a, const M3<R>& b, M3<R>& c) {
@@ -330,9 +336,10 @@ __device__ __forceinline__ Herm8<R> force_from_b_cdag(const M3<R>& b, const M3<R
 // The same generator of X = B C^+ for X in SU(3), from B's first two rows:
 // rows 0 and 1 of X (six entries), then of row 2 = conj(row0 x row1) only
 // X_20, X_21 and Im X_22.  92 multiply-adds, against 90 plus the 27 that
-// rebuild B's row 2 for the full form.
+// rebuild B's row 2 for the full form.  trace (optional): Re tr X, for four
+// more.
 template <class R>
-__device__ __forceinline__ Herm8<R> force_from_b2_cdag(const Rows2<R>& b, const M3<R>& c) {
+__device__ __forceinline__ Herm8<R> force_from_b2_cdag(const Rows2<R>& b, const M3<R>& c, R* trace = nullptr) {
     Cx<R> x[2][3];
 #pragma unroll
     for (int i = 0; i < 2; i++)
@@ -357,9 +364,10 @@ __device__ __forceinline__ Herm8<R> force_from_b2_cdag(const Rows2<R>& b, const 
     };
     const Cx<R> x20 = cross(1, 2), x21 = cross(2, 0);
     const R i2 = -fma(x[0][0].re, x[1][1].im, fma(x[0][0].im, x[1][1].re, -fma(x[0][1].re, x[1][0].im, x[0][1].im * x[1][0].re)));
+    if (trace) *trace = x[0][0].re + x[1][1].re + cross(0, 1).re;
     Herm8<R> z;
     const R i0 = x[0][0].im, i1 = x[1][1].im;
-    const R mean = (i0 + i1 + i2) * R(1.0 / 3.0);
+    const R mean = mul_rn(i0 + i1 + i2, R(1.0 / 3.0));
     z.d0 = mean - i0;
     z.d1 = mean - i1;
     z.z01 = cx(R(-0.5) * (x[0][1].im + x[1][0].im), R(0.5) * (x[0][1].re - x[1][0].re));
@@ -431,12 +439,6 @@ __device__ __forceinline__ Herm8<R> h8_axpby(R a, const Herm8<R>& x, R b, const 
     r.z12 = cx(a * x.z12.re - b * y.z12.re, a * x.z12.im - b * y.z12.im);
     return r;
 }
-
-// A product that the compiler leaves rounded as it stands: contracted into the
-// sums that use it or not, it would make kernels that share this code differ
-// by rounding.
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 
 template <class R>
 __device__ __forceinline__ Herm8<R> h8_scale(R a, const Herm8<R>& x) {

@@ -64,16 +64,21 @@ int ensure_staging(ymflow_ctx* c, size_t bytes = 0) {
     return r;
 }
 
+// Whether a measurement goes through the plaquette field: where the stages do.
+bool measures_from_field(const ymflow_ctx* c) { return c->stage_form == 1 && c->hfield; }
+
 int ensure_partials(ymflow_ctx* c) {
-    const int nb = obs_blocks(c->geo);
-    if (nb <= c->partial_cap) return YMFLOW_OK;
+    int n = 3 * obs_blocks(c->geo);
+    if (measures_from_field(c)) n = std::max(n, measure_partials(c->prec, plaq_range(c->geo, c->slab), c->geo));
+    if (n <= c->partial_cap) return YMFLOW_OK;
     if (c->partials) {
         cudaFree(c->partials);
-        c->bytes -= int64_t(c->partial_cap) * 3 * sizeof(double);
+        c->bytes -= int64_t(c->partial_cap) * sizeof(double);
         c->partials = nullptr;
+        c->partial_cap = 0;
     }
-    int r = dev_alloc(c, (void**)&c->partials, size_t(nb) * 3 * sizeof(double), "observable partials");
-    if (r == YMFLOW_OK) c->partial_cap = nb;
+    int r = dev_alloc(c, (void**)&c->partials, size_t(n) * sizeof(double), "observable partials");
+    if (r == YMFLOW_OK) c->partial_cap = n;
     return r;
 }
 
@@ -148,17 +153,18 @@ int64_t tile_option(const TileShape& tp) {
 }
 
 void drop_graphs(ymflow_ctx* c) {
-    for (int i = 0; i < 2; i++) {
-        if (c->graph[i]) cudaGraphExecDestroy(c->graph[i]);
-        c->graph[i] = nullptr;
+    for (cudaGraphExec_t& g : c->graph) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
     }
 }
 
 // The launches of one RK3 step starting from u[from]: per stage the fused
 // stage kernel, or the plaquette-field kernel and the stage kernel built on it
-// (stage_form 1).  ev (optional): three events per stage, before the stage,
+// (stage_form 1).  field_ready: the plaquette field already holds u[from]'s
+// (stage 0 needs no field kernel).  ev (optional): three events per stage, before the stage,
 // after its plaquette-field kernel (at once for the fused form) and after it.
-cudaError_t enqueue_step(ymflow_ctx* c, int from, double eps, cudaEvent_t* ev) {
+cudaError_t enqueue_step(ymflow_ctx* c, int from, double eps, cudaEvent_t* ev, bool field_ready) {
     void* a = c->u[from];
     void* b = c->u[1 - from];
     const void* in[3] = {a, b, a};
@@ -167,7 +173,7 @@ cudaError_t enqueue_step(ymflow_ctx* c, int from, double eps, cudaEvent_t* ev) {
         if (ev) cudaEventRecord(ev[3 * s], c->stream);
         cudaError_t e = cudaSuccess;
         if (c->stage_form == 1) {
-            e = launch_plaq_field(c->prec, in[s], c->hfield, c->geo, c->stream);
+            if (s > 0 || !field_ready) e = launch_plaq_field(c->prec, in[s], c->hfield, c->geo, c->stream);
             if (e != cudaSuccess) return e;
             if (ev) cudaEventRecord(ev[3 * s + 1], c->stream);
             e = launch_rk_split_stage(c->prec, s, in[s], out[s], c->z, c->hfield, c->geo, eps, c->stream);
@@ -186,14 +192,15 @@ cudaError_t enqueue_step(ymflow_ctx* c, int from, double eps, cudaEvent_t* ev) {
 
 // One RK3 step of a slab: each stage's new links are followed by the halo
 // exchange of that buffer, which the next stage reads.
-int run_step_slab(ymflow_ctx* c, double eps, cudaEvent_t* ev) {
+int run_step_slab(ymflow_ctx* c, double eps, cudaEvent_t* ev, bool field_ready) {
     const int from = c->cur;
     const int in[3] = {from, 1 - from, from};
     for (int s = 0; s < 3; s++) {
         if (ev) cudaEventRecord(ev[3 * s], c->stream);
         if (c->stage_form == 1) {
-            YM_CK(c, launch_plaq_field(c->prec, c->u[in[s]], c->hfield, plaq_range(c->geo, true), c->stream),
-                  "plaquette-field launch");
+            if (s > 0 || !field_ready)
+                YM_CK(c, launch_plaq_field(c->prec, c->u[in[s]], c->hfield, plaq_range(c->geo, true), c->stream),
+                      "plaquette-field launch");
             if (ev) cudaEventRecord(ev[3 * s + 1], c->stream);
             YM_CK(c, launch_rk_split_stage(c->prec, s, c->u[in[s]], c->u[1 - in[s]], c->z, c->hfield, c->geo, eps,
                                            c->stream),
@@ -212,31 +219,35 @@ int run_step_slab(ymflow_ctx* c, double eps, cudaEvent_t* ev) {
     return YMFLOW_OK;
 }
 
-int run_step(ymflow_ctx* c, double eps, cudaEvent_t* ev) {
-    if (c->slab) return run_step_slab(c, eps, ev);
+// One RK3 step of the current field.  field_ready: the plaquette field holds
+// the current links' (a measurement has just been enqueued, and nothing has
+// changed the links since).
+int run_step(ymflow_ctx* c, double eps, cudaEvent_t* ev, bool field_ready = false) {
+    if (c->slab) return run_step_slab(c, eps, ev, field_ready);
     const int from = c->cur;
     if (c->use_graph && !ev) {
-        if (!c->graph[from] || c->graph_eps[from] != eps || c->graph_block[from] != c->block) {
-            if (c->graph[from]) cudaGraphExecDestroy(c->graph[from]);
-            c->graph[from] = nullptr;
+        const int k = from + (field_ready ? 2 : 0);
+        if (!c->graph[k] || c->graph_eps[k] != eps || c->graph_block[k] != c->block) {
+            if (c->graph[k]) cudaGraphExecDestroy(c->graph[k]);
+            c->graph[k] = nullptr;
             cudaGraph_t g = nullptr;
             YM_CK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal), "begin step capture");
-            cudaError_t le = enqueue_step(c, from, eps, nullptr);
+            cudaError_t le = enqueue_step(c, from, eps, nullptr, field_ready);
             cudaError_t ee = cudaStreamEndCapture(c->stream, &g);
             if (le != cudaSuccess) {
                 if (g) cudaGraphDestroy(g);
                 return cuda_fail(c, le, "stage launch during capture");
             }
             YM_CK(c, ee, "end step capture");
-            cudaError_t ie = cudaGraphInstantiate(&c->graph[from], g, 0);
+            cudaError_t ie = cudaGraphInstantiate(&c->graph[k], g, 0);
             cudaGraphDestroy(g);
             YM_CK(c, ie, "instantiate step graph");
-            c->graph_eps[from] = eps;
-            c->graph_block[from] = c->block;
+            c->graph_eps[k] = eps;
+            c->graph_block[k] = c->block;
         }
-        YM_CK(c, cudaGraphLaunch(c->graph[from], c->stream), "launch step graph");
+        YM_CK(c, cudaGraphLaunch(c->graph[k], c->stream), "launch step graph");
     } else {
-        YM_CK(c, enqueue_step(c, from, eps, ev), "stage launch");
+        YM_CK(c, enqueue_step(c, from, eps, ev, field_ready), "stage launch");
     }
     c->cur = 1 - from;
     return YMFLOW_OK;
@@ -260,10 +271,15 @@ cudaError_t enqueue_stage(ymflow_ctx* c, int stage, const void* in, void* out, d
 int enqueue_measure(ymflow_ctx* c, int row) {
     int r = ensure_partials(c);
     if (r != YMFLOW_OK) return r;
-    YM_CK(c, launch_observables(c->prec, c->u[c->cur], c->geo, c->partials, c->stream),
-          "observables launch");
-    YM_CK(c, launch_obs_finalize(c->partials, obs_blocks(c->geo), c->geo, c->meas + 4 * row, c->stream),
-          "observables fold");
+    if (measures_from_field(c)) {
+        YM_CK(c, launch_measure_from_field(c->prec, c->u[c->cur], c->hfield, plaq_range(c->geo, c->slab), c->geo,
+                                           c->partials, c->meas + 4 * row, c->stream),
+              "observables launch");
+    } else {
+        YM_CK(c, launch_observables(c->prec, c->u[c->cur], c->geo, c->partials, c->stream), "observables launch");
+        YM_CK(c, launch_obs_finalize(c->partials, obs_blocks(c->geo), c->geo, c->meas + 4 * row, c->stream),
+              "observables fold");
+    }
     if (c->slab && c->comm) return slab_reduce_row(c, c->meas + 4 * row);
     return YMFLOW_OK;
 }
@@ -728,8 +744,11 @@ int ymflow_flow(ymflow_ctx* c, double eps, int nsteps, int measure_every, int re
     row_step[row] = c->step;
     row_t[row] = c->t;
     row++;
+    const bool from_field = measures_from_field(c);
+    bool field_ready = from_field;  // a measured row leaves its plaquette field for the next step's stage 0
     for (int s = 1; s <= nsteps; s++) {
-        if ((r = run_step(c, eps, nullptr)) != YMFLOW_OK) return r;
+        if ((r = run_step(c, eps, nullptr, field_ready)) != YMFLOW_OK) return r;
+        field_ready = false;
         c->step++;
         c->t += eps;
         if (reunit && s % reunit_every == 0)
@@ -739,6 +758,7 @@ int ymflow_flow(ymflow_ctx* c, double eps, int nsteps, int measure_every, int re
             row_step[row] = c->step;
             row_t[row] = c->t;
             row++;
+            field_ready = from_field;
         }
     }
     YM_CK(c, cudaMemcpyAsync(c->meas_host, c->meas, size_t(rows) * 4 * sizeof(double), cudaMemcpyDeviceToHost,
