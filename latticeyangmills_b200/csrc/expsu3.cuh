@@ -68,9 +68,9 @@ __device__ __forceinline__ ChCoef<S> ch_series(S c0, S c1) {
 #pragma unroll
     for (int n = 3; n <= N; n++) {
         const S inv = S(1.0 / n);
-        const S na = c0 * c * inv;
-        const S nb = fma(c1, c, a) * inv;
-        const S nc = b * inv;
+        const S na = mul_rn(mul_rn(c0, c), inv);
+        const S nb = mul_rn(fma(c1, c, a), inv);
+        const S nc = mul_rn(b, inv);
         a = na;
         b = nb;
         c = nc;
@@ -156,24 +156,26 @@ struct QSquared {  // Q^2, Hermitian: real diagonal and the upper triangle
     Cx<R> a01, a02, a12;
 };
 
+// (every multiply-add below is written out, so that kernels sharing this code
+// round alike)
 template <class R>
 __device__ __forceinline__ QSquared<R> q_squared(const Herm8<R>& q, R q22) {
     QSquared<R> s;
-    const R n01 = q.z01.re * q.z01.re + q.z01.im * q.z01.im;
-    const R n02 = q.z02.re * q.z02.re + q.z02.im * q.z02.im;
-    const R n12 = q.z12.re * q.z12.re + q.z12.im * q.z12.im;
-    s.a00 = q.d0 * q.d0 + n01 + n02;
-    s.a11 = q.d1 * q.d1 + n01 + n12;
-    s.a22 = q22 * q22 + n02 + n12;
-    // (Q^2)_01 = q00 q01 + q01 q11 + q02 conj(q12)
-    s.a01 = cx((q.d0 + q.d1) * q.z01.re + q.z02.re * q.z12.re + q.z02.im * q.z12.im,
-               (q.d0 + q.d1) * q.z01.im + q.z02.im * q.z12.re - q.z02.re * q.z12.im);
-    // (Q^2)_02 = q00 q02 + q01 q12 + q02 q22
-    s.a02 = cx((q.d0 + q22) * q.z02.re + q.z01.re * q.z12.re - q.z01.im * q.z12.im,
-               (q.d0 + q22) * q.z02.im + q.z01.re * q.z12.im + q.z01.im * q.z12.re);
-    // (Q^2)_12 = conj(q01) q02 + q11 q12 + q12 q22
-    s.a12 = cx((q.d1 + q22) * q.z12.re + q.z01.re * q.z02.re + q.z01.im * q.z02.im,
-               (q.d1 + q22) * q.z12.im + q.z01.re * q.z02.im - q.z01.im * q.z02.re);
+    const R n01 = fma(q.z01.re, q.z01.re, mul_rn(q.z01.im, q.z01.im));
+    const R n02 = fma(q.z02.re, q.z02.re, mul_rn(q.z02.im, q.z02.im));
+    const R n12 = fma(q.z12.re, q.z12.re, mul_rn(q.z12.im, q.z12.im));
+    s.a00 = fma(q.d0, q.d0, n01 + n02);
+    s.a11 = fma(q.d1, q.d1, n01 + n12);
+    s.a22 = fma(q22, q22, n02 + n12);
+    // (Q^2)_01 = q00 q01 + q01 q11 + q02 conj(q12);  q00 + q11 = -q22
+    s.a01 = cx(fma(-q22, q.z01.re, fma(q.z02.re, q.z12.re, mul_rn(q.z02.im, q.z12.im))),
+               fma(-q22, q.z01.im, fma(q.z02.im, q.z12.re, -mul_rn(q.z02.re, q.z12.im))));
+    // (Q^2)_02 = q00 q02 + q01 q12 + q02 q22;  q00 + q22 = -q11
+    s.a02 = cx(fma(-q.d1, q.z02.re, fma(q.z01.re, q.z12.re, -mul_rn(q.z01.im, q.z12.im))),
+               fma(-q.d1, q.z02.im, fma(q.z01.re, q.z12.im, mul_rn(q.z01.im, q.z12.re))));
+    // (Q^2)_12 = conj(q01) q02 + q11 q12 + q12 q22;  q11 + q22 = -q00
+    s.a12 = cx(fma(-q.d0, q.z12.re, fma(q.z01.re, q.z02.re, mul_rn(q.z01.im, q.z02.im))),
+               fma(-q.d0, q.z12.im, fma(q.z01.re, q.z02.im, -mul_rn(q.z01.im, q.z02.re))));
     return s;
 }
 
@@ -183,17 +185,18 @@ __device__ __forceinline__ S herm_det(const Herm8<R>& q, R q22r) {
     const S a = S(q.d0), b = S(q.d1), c = S(q22r);
     const S xr = S(q.z01.re), xi = S(q.z01.im), yr = S(q.z02.re), yi = S(q.z02.im);
     const S zr = S(q.z12.re), zi = S(q.z12.im);
-    const S pr = xr * zr - xi * zi, pi = xr * zi + xi * zr;  // q01 q12
-    const S re3 = pr * yr + pi * yi;                          // Re(q01 q12 conj(q02))
-    return a * b * c + S(2) * re3 - a * (zr * zr + zi * zi) - b * (yr * yr + yi * yi) - c * (xr * xr + xi * xi);
+    const S pr = fma(xr, zr, -mul_rn(xi, zi)), pi = fma(xr, zi, mul_rn(xi, zr));  // q01 q12
+    const S re3 = fma(pr, yr, mul_rn(pi, yi));                                     // Re(q01 q12 conj(q02))
+    const S nz = fma(zr, zr, mul_rn(zi, zi)), ny = fma(yr, yr, mul_rn(yi, yi)), nx = fma(xr, xr, mul_rn(xi, xi));
+    return fma(S(2), re3, fma(a, fma(b, c, -nz), fma(-b, ny, -mul_rn(c, nx))));
 }
 
 template <class S, class R>
 __device__ __forceinline__ S herm_c1(const Herm8<R>& q, R q22r) {
     const S a = S(q.d0), b = S(q.d1), c = S(q22r);
-    const S n = S(q.z01.re) * S(q.z01.re) + S(q.z01.im) * S(q.z01.im) + S(q.z02.re) * S(q.z02.re) +
-                S(q.z02.im) * S(q.z02.im) + S(q.z12.re) * S(q.z12.re) + S(q.z12.im) * S(q.z12.im);
-    return S(0.5) * (a * a + b * b + c * c) + n;
+    const S n = fma(S(q.z01.re), S(q.z01.re), fma(S(q.z01.im), S(q.z01.im), fma(S(q.z02.re), S(q.z02.re),
+                fma(S(q.z02.im), S(q.z02.im), fma(S(q.z12.re), S(q.z12.re), mul_rn(S(q.z12.im), S(q.z12.im)))))));
+    return fma(S(0.5), fma(a, a, fma(b, b, mul_rn(c, c))), n);
 }
 
 // Threshold on c0/c0max above which the mixed path evaluates the coefficients in
@@ -259,17 +262,17 @@ __device__ __forceinline__ void expm1_iq_rows2(const Herm8<R>& q, Rows2<R>& e) {
     const R q22 = -(q.d0 + q.d1);
     const ChCoef<R> f = exp_coefficients<R>(q, q22);
     const QSquared<R> s = q_squared(q, q22);
-    e.e[0][0] = cx(f.f0m1.re + f.f1.re * q.d0 + f.f2.re * s.a00, f.f0m1.im + f.f1.im * q.d0 + f.f2.im * s.a00);
-    e.e[1][1] = cx(f.f0m1.re + f.f1.re * q.d1 + f.f2.re * s.a11, f.f0m1.im + f.f1.im * q.d1 + f.f2.im * s.a11);
+    e.e[0][0] = cx(fma(f.f2.re, s.a00, fma(f.f1.re, q.d0, f.f0m1.re)), fma(f.f2.im, s.a00, fma(f.f1.im, q.d0, f.f0m1.im)));
+    e.e[1][1] = cx(fma(f.f2.re, s.a11, fma(f.f1.re, q.d1, f.f0m1.re)), fma(f.f2.im, s.a11, fma(f.f1.im, q.d1, f.f0m1.im)));
     // upper entries f1 q_ij + f2 (Q^2)_ij; e10 from the conjugates of q01 and (Q^2)_01
-    e.e[0][1] = cx(f.f1.re * q.z01.re - f.f1.im * q.z01.im + f.f2.re * s.a01.re - f.f2.im * s.a01.im,
-                   f.f1.re * q.z01.im + f.f1.im * q.z01.re + f.f2.re * s.a01.im + f.f2.im * s.a01.re);
-    e.e[0][2] = cx(f.f1.re * q.z02.re - f.f1.im * q.z02.im + f.f2.re * s.a02.re - f.f2.im * s.a02.im,
-                   f.f1.re * q.z02.im + f.f1.im * q.z02.re + f.f2.re * s.a02.im + f.f2.im * s.a02.re);
-    e.e[1][2] = cx(f.f1.re * q.z12.re - f.f1.im * q.z12.im + f.f2.re * s.a12.re - f.f2.im * s.a12.im,
-                   f.f1.re * q.z12.im + f.f1.im * q.z12.re + f.f2.re * s.a12.im + f.f2.im * s.a12.re);
-    e.e[1][0] = cx(f.f1.re * q.z01.re + f.f1.im * q.z01.im + f.f2.re * s.a01.re + f.f2.im * s.a01.im,
-                   -f.f1.re * q.z01.im + f.f1.im * q.z01.re - f.f2.re * s.a01.im + f.f2.im * s.a01.re);
+    auto upper = [&](const Cx<R>& z, const Cx<R>& w) {
+        return cx(fma(f.f1.re, z.re, fma(-f.f1.im, z.im, fma(f.f2.re, w.re, -mul_rn(f.f2.im, w.im)))),
+                  fma(f.f1.re, z.im, fma(f.f1.im, z.re, fma(f.f2.re, w.im, mul_rn(f.f2.im, w.re)))));
+    };
+    e.e[0][1] = upper(q.z01, s.a01);
+    e.e[0][2] = upper(q.z02, s.a02);
+    e.e[1][2] = upper(q.z12, s.a12);
+    e.e[1][0] = upper(cx(q.z01.re, -q.z01.im), cx(s.a01.re, -s.a01.im));
 }
 
 }  // namespace ym

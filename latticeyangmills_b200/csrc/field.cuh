@@ -317,6 +317,27 @@ struct LinkField<float, NE> {
 };
 
 using FieldD18 = LinkField<double, 9>;
+
+// An FP64 field between two steps of one flow call, which nobody but the flow's
+// own kernels reads: rows 0 and 1 of its links, in FieldD18's layout.  A stage
+// stores row 2 as row2_entry of the rows it computed, so rebuilding it on load
+// gives the links a FieldD18 would hold, bit for bit, for 96 instead of 144
+// bytes each way.  The FP64 stage kernels were short of HBM bandwidth (65-69 %
+// busy) and of loads in flight; at 32^4 on B200 0.337 -> 0.283-0.312 ms per
+// launch, the field kernel 0.232 -> 0.204, both then at 57-63 % of the FP64 pipe
+// and 40-63 % of HBM.
+struct FieldD18Rows : LinkField<double, 9> {
+    __device__ __forceinline__ M3<double> load(int mu, int s) const {
+        M3<double> a;
+        full_from_rows2(load_rows2(mu, s), a);
+        return a;
+    }
+    __device__ __forceinline__ void store_rows2(int mu, int s, const Rows2<double>& a) const {
+        double2* q = const_cast<double2*>(link(mu, s));
+#pragma unroll
+        for (int e = 0; e < 6; e++) q[32 * e] = make_double2(a.e[e / 3][e % 3].re, a.e[e / 3][e % 3].im);
+    }
+};
 using FieldF18 = LinkField<float, 9>;
 using FieldF12 = LinkField<float, 6>;
 

@@ -75,9 +75,9 @@ __global__ void __launch_bounds__(192, PlaqMinBlocks<F>::value) plaq_field_kerne
 }
 
 // One thread per link: four warps (directions) per 32 sites.
-template <class F, int STAGE>
+template <class F, int STAGE, class FO>
 __global__ void __launch_bounds__(128, SplitMinBlocks<F>::value)
-    rk_split_stage_kernel(F in, F out, ForceField<typename F::Real> zf, ForceField<typename F::Real> hf, Geo g,
+    rk_split_stage_kernel(F in, FO out, ForceField<typename F::Real> zf, ForceField<typename F::Real> hf, Geo g,
                           typename F::Real eps) {
     const int mu = int(threadIdx.x >> 5) & 3;
     const int s = g.site0 + int(blockIdx.x) * 32 + int(threadIdx.x & 31);
@@ -124,18 +124,19 @@ static cudaError_t launch_plaq_typed(const void* u, void* h, const Geo& g, cudaS
     return cudaGetLastError();
 }
 
-template <class F>
+template <class F, class FO = F>
 static cudaError_t launch_split_typed(int stage, const void* uin, void* uout, void* z, const void* h, const Geo& g,
                                       double eps, cudaStream_t st) {
     using R = typename F::Real;
-    F in{const_cast<void*>(uin), g.V}, out{uout, g.V};
+    const F in{const_cast<void*>(uin), g.V};
+    const FO out{uout, g.V};
     ForceField<R> zf{z, g.V}, hf{const_cast<void*>(h), g.V};
     const dim3 grid(unsigned((g.site1 - g.site0 + 31) / 32));
     const R e = R(stage == 0 ? eps * 0.25 : eps);
     switch (stage) {
-        case 0: rk_split_stage_kernel<F, 0><<<grid, 128, 0, st>>>(in, out, zf, hf, g, e); break;
-        case 1: rk_split_stage_kernel<F, 1><<<grid, 128, 0, st>>>(in, out, zf, hf, g, e); break;
-        default: rk_split_stage_kernel<F, 2><<<grid, 128, 0, st>>>(in, out, zf, hf, g, e); break;
+        case 0: rk_split_stage_kernel<F, 0, FO><<<grid, 128, 0, st>>>(in, out, zf, hf, g, e); break;
+        case 1: rk_split_stage_kernel<F, 1, FO><<<grid, 128, 0, st>>>(in, out, zf, hf, g, e); break;
+        default: rk_split_stage_kernel<F, 2, FO><<<grid, 128, 0, st>>>(in, out, zf, hf, g, e); break;
     }
     return cudaGetLastError();
 }
@@ -193,19 +194,23 @@ static cudaError_t launch_plaq_sum_typed(const void* u, void* h, const Geo& g, i
 }
 
 cudaError_t launch_plaq_field_sum(int prec, const void* u, void* h, const Geo& g, int count0, int count1,
-                                  double* partials, cudaStream_t st) {
+                                  double* partials, cudaStream_t st, bool rows_in) {
     if (g.site1 <= g.site0) return cudaErrorInvalidValue;
     switch (prec) {
-        case kFP64: return launch_plaq_sum_typed<FieldD18>(u, h, g, count0, count1, partials, st);
+        case kFP64:
+            if (rows_in) return launch_plaq_sum_typed<FieldD18Rows>(u, h, g, count0, count1, partials, st);
+            return launch_plaq_sum_typed<FieldD18>(u, h, g, count0, count1, partials, st);
         case kFP32_18: return launch_plaq_sum_typed<FieldF18>(u, h, g, count0, count1, partials, st);
         case kFP32_12: return launch_plaq_sum_typed<FieldF12>(u, h, g, count0, count1, partials, st);
         default: return cudaErrorInvalidValue;
     }
 }
 
-cudaError_t launch_plaq_field(int prec, const void* u, void* h, const Geo& g, cudaStream_t st) {
+cudaError_t launch_plaq_field(int prec, const void* u, void* h, const Geo& g, cudaStream_t st, bool rows_in) {
     switch (prec) {
-        case kFP64: return launch_plaq_typed<FieldD18>(u, h, g, st);
+        case kFP64:
+            if (rows_in) return launch_plaq_typed<FieldD18Rows>(u, h, g, st);
+            return launch_plaq_typed<FieldD18>(u, h, g, st);
         case kFP32_18: return launch_plaq_typed<FieldF18>(u, h, g, st);
         case kFP32_12: return launch_plaq_typed<FieldF12>(u, h, g, st);
         default: return cudaErrorInvalidValue;
@@ -231,9 +236,13 @@ cudaError_t launch_rk_split_stage_halo(int prec, int stage, const void* uin, voi
 }
 
 cudaError_t launch_rk_split_stage(int prec, int stage, const void* uin, void* uout, void* z, const void* h,
-                                  const Geo& g, double eps, cudaStream_t st) {
+                                  const Geo& g, double eps, cudaStream_t st, bool rows_in, bool rows_out) {
     switch (prec) {
-        case kFP64: return launch_split_typed<FieldD18>(stage, uin, uout, z, h, g, eps, st);
+        case kFP64:
+            if (rows_in && rows_out) return launch_split_typed<FieldD18Rows>(stage, uin, uout, z, h, g, eps, st);
+            if (rows_in) return launch_split_typed<FieldD18Rows, FieldD18>(stage, uin, uout, z, h, g, eps, st);
+            if (rows_out) return launch_split_typed<FieldD18, FieldD18Rows>(stage, uin, uout, z, h, g, eps, st);
+            return launch_split_typed<FieldD18>(stage, uin, uout, z, h, g, eps, st);
         case kFP32_18: return launch_split_typed<FieldF18>(stage, uin, uout, z, h, g, eps, st);
         case kFP32_12: return launch_split_typed<FieldF12>(stage, uin, uout, z, h, g, eps, st);
         default: return cudaErrorInvalidValue;

@@ -30,10 +30,13 @@ cudaError_t launch_rk_stage(int prec, int stage, const void* uin, void* uout, vo
 
 // The same stage as two kernels (flow_split.cu): the six plaquettes' generators
 // of every site of u into h (plane_field_bytes), then the stage with each
-// link's force built from h (h must hold uin's plaquette field).
-cudaError_t launch_plaq_field(int prec, const void* u, void* h, const Geo& g, cudaStream_t st);
+// link's force built from h (h must hold uin's plaquette field).  rows_in (FP64):
+// read rows 0 and 1 of u's links only (u was written by a stage); rows_out:
+// store rows 0 and 1 only (uout is read with rows_in alone).
+cudaError_t launch_plaq_field(int prec, const void* u, void* h, const Geo& g, cudaStream_t st, bool rows_in = false);
 cudaError_t launch_rk_split_stage(int prec, int stage, const void* uin, void* uout, void* z, const void* h,
-                                  const Geo& g, double eps, cudaStream_t st);
+                                  const Geo& g, double eps, cudaStream_t st, bool rows_in = false,
+                                  bool rows_out = false);
 // Its slab form with the halo stores of launch_rk_stage_halo (h must hold the
 // plane generators of local slices 0..nt, see plaq_range).
 cudaError_t launch_rk_split_stage_halo(int prec, int stage, const void* uin, void* uout, void* z, const void* h,
@@ -107,10 +110,10 @@ cudaError_t launch_obs_finalize(const double* partials, int nblocks, const Geo& 
 constexpr int kCloverMaxBlocks = 148 * 20;
 int plaq_sum_partials(int prec, const Geo& g);
 cudaError_t launch_plaq_field_sum(int prec, const void* u, void* h, const Geo& g, int count0, int count1,
-                                  double* partials, cudaStream_t st);
+                                  double* partials, cudaStream_t st, bool rows_in = false);
 int measure_partials(int prec, const Geo& field, const Geo& own);
 cudaError_t launch_measure_from_field(int prec, const void* u, void* h, const Geo& field, const Geo& own,
-                                      double* partials, double* out, cudaStream_t st);
+                                      double* partials, double* out, cudaStream_t st, bool rows_in = false);
 
 // .bin layout (site-major, mu, 18 doubles) <-> device layout
 // Sites [first, first + n) between a .bin-layout block (aos points at site

@@ -96,14 +96,17 @@ int measure_partials(int prec, const Geo& field, const Geo& own) {
 // 48 0.55 -> 0.39 ms; below, both are a few launches long (8^4 FP64: 9.3 + 2.9
 // us against 4.9 + 6.7 + 2.9, of which the next step saves the first).
 cudaError_t launch_measure_from_field(int prec, const void* u, void* h, const Geo& field, const Geo& own,
-                                      double* partials, double* out, cudaStream_t st) {
+                                      double* partials, double* out, cudaStream_t st, bool rows_in) {
     const int np = plaq_sum_partials(prec, field), nc = clover_blocks(own);
     if (np < 1 || nc < 1) return cudaErrorInvalidValue;
-    cudaError_t e = launch_plaq_field_sum(prec, u, h, field, own.site0, own.site1, partials, st);
+    cudaError_t e = launch_plaq_field_sum(prec, u, h, field, own.site0, own.site1, partials, st, rows_in);
     if (e != cudaSuccess) return e;
     double* const cp = partials + np;
     switch (prec) {
-        case kFP64: e = launch_clover_typed<FieldD18>(u, h, own, nc, partials, np, cp, st); break;
+        case kFP64:
+            e = rows_in ? launch_clover_typed<FieldD18Rows>(u, h, own, nc, partials, np, cp, st)
+                        : launch_clover_typed<FieldD18>(u, h, own, nc, partials, np, cp, st);
+            break;
         case kFP32_18: e = launch_clover_typed<FieldF18>(u, h, own, nc, partials, np, cp, st); break;
         case kFP32_12: e = launch_clover_typed<FieldF12>(u, h, own, nc, partials, np, cp, st); break;
         default: return cudaErrorInvalidValue;

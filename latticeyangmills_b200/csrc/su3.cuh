@@ -432,11 +432,11 @@ __device__ __forceinline__ void herm_conj_add(const M3<R>& v, const Herm8<R>& h,
 template <class R>
 __device__ __forceinline__ Herm8<R> h8_axpby(R a, const Herm8<R>& x, R b, const Herm8<R>& y) {
     Herm8<R> r;
-    r.d0 = a * x.d0 - b * y.d0;
-    r.d1 = a * x.d1 - b * y.d1;
-    r.z01 = cx(a * x.z01.re - b * y.z01.re, a * x.z01.im - b * y.z01.im);
-    r.z02 = cx(a * x.z02.re - b * y.z02.re, a * x.z02.im - b * y.z02.im);
-    r.z12 = cx(a * x.z12.re - b * y.z12.re, a * x.z12.im - b * y.z12.im);
+    r.d0 = fma(a, x.d0, -mul_rn(b, y.d0));
+    r.d1 = fma(a, x.d1, -mul_rn(b, y.d1));
+    r.z01 = cx(fma(a, x.z01.re, -mul_rn(b, y.z01.re)), fma(a, x.z01.im, -mul_rn(b, y.z01.im)));
+    r.z02 = cx(fma(a, x.z02.re, -mul_rn(b, y.z02.re)), fma(a, x.z02.im, -mul_rn(b, y.z02.im)));
+    r.z12 = cx(fma(a, x.z12.re, -mul_rn(b, y.z12.re)), fma(a, x.z12.im, -mul_rn(b, y.z12.im)));
     return r;
 }
 

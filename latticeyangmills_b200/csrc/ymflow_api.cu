@@ -159,12 +159,23 @@ void drop_graphs(ymflow_ctx* c) {
     }
 }
 
+// Whether the steps of a call pass links on as their rows 0 and 1: whole
+// lattices on the two-kernel FP64 stage.
+bool steps_by_rows(const ymflow_ctx* c) {
+    return c->prec == YMFLOW_FP64 && c->stage_form == 1 && !c->slab && !c->is_block;
+}
+
+constexpr int kRowsIn = 1, kRowsOut = 2;
+
 // The launches of one RK3 step starting from u[from]: per stage the fused
 // stage kernel, or the plaquette-field kernel and the stage kernel built on it
 // (stage_form 1).  field_ready: the plaquette field already holds u[from]'s
-// (stage 0 needs no field kernel).  ev (optional): three events per stage, before the stage,
+// (stage 0 needs no field kernel).  rows (FP64, stage_form 1): bit 0, u[from]
+// was written by a stage of the same call; bit 1, another step of the call
+// follows: the links between a call's steps, and between its stages, are
+// stored and read as their rows 0 and 1 (FieldD18Rows).  ev (optional): three events per stage, before the stage,
 // after its plaquette-field kernel (at once for the fused form) and after it.
-cudaError_t enqueue_step(ymflow_ctx* c, int from, double eps, cudaEvent_t* ev, bool field_ready) {
+cudaError_t enqueue_step(ymflow_ctx* c, int from, double eps, cudaEvent_t* ev, bool field_ready, int rows) {
     void* a = c->u[from];
     void* b = c->u[1 - from];
     const void* in[3] = {a, b, a};
@@ -173,10 +184,13 @@ cudaError_t enqueue_step(ymflow_ctx* c, int from, double eps, cudaEvent_t* ev, b
         if (ev) cudaEventRecord(ev[3 * s], c->stream);
         cudaError_t e = cudaSuccess;
         if (c->stage_form == 1) {
-            if (s > 0 || !field_ready) e = launch_plaq_field(c->prec, in[s], c->hfield, c->geo, c->stream);
+            const bool rows_in = s > 0 || (rows & kRowsIn), rows_out = s < 2 || (rows & kRowsOut);
+            if (s > 0 || !field_ready)
+                e = launch_plaq_field(c->prec, in[s], c->hfield, c->geo, c->stream, rows_in);
             if (e != cudaSuccess) return e;
             if (ev) cudaEventRecord(ev[3 * s + 1], c->stream);
-            e = launch_rk_split_stage(c->prec, s, in[s], out[s], c->z, c->hfield, c->geo, eps, c->stream);
+            e = launch_rk_split_stage(c->prec, s, in[s], out[s], c->z, c->hfield, c->geo, eps, c->stream, rows_in,
+                                      rows_out);
         } else if (c->stage_form == 2) {
             if (ev) cudaEventRecord(ev[3 * s + 1], c->stream);
             e = launch_rk_tile_stage(c->prec, s, in[s], out[s], c->z, c->geo, c->tile, eps, c->stream);
@@ -219,20 +233,24 @@ int run_step_slab(ymflow_ctx* c, double eps, cudaEvent_t* ev, bool field_ready) 
     return YMFLOW_OK;
 }
 
-// One RK3 step of the current field.  field_ready: the plaquette field holds
-// the current links' (a measurement has just been enqueued, and nothing has
-// changed the links since).
-int run_step(ymflow_ctx* c, double eps, cudaEvent_t* ev, bool field_ready = false) {
+// One RK3 step of the current field, step `s` of the `nsteps` (from 1) of a
+// call.  field_ready: the plaquette field holds the current links' (a
+// measurement has just been enqueued, and nothing has changed the links
+// since).  The steps that repeat are replayed as graphs; an FP64 call's first
+// and last, which read or leave whole links, are launched as they are.
+int run_step(ymflow_ctx* c, double eps, int s, int nsteps, cudaEvent_t* ev, bool field_ready = false) {
     if (c->slab) return run_step_slab(c, eps, ev, field_ready);
     const int from = c->cur;
-    if (c->use_graph && !ev) {
+    const bool by_rows = steps_by_rows(c);
+    const int rows = by_rows ? (s > 1 ? kRowsIn : 0) | (s < nsteps ? kRowsOut : 0) : 0;
+    if (c->use_graph && !ev && (!by_rows || rows == (kRowsIn | kRowsOut))) {
         const int k = from + (field_ready ? 2 : 0);
         if (!c->graph[k] || c->graph_eps[k] != eps || c->graph_block[k] != c->block) {
             if (c->graph[k]) cudaGraphExecDestroy(c->graph[k]);
             c->graph[k] = nullptr;
             cudaGraph_t g = nullptr;
             YM_CK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal), "begin step capture");
-            cudaError_t le = enqueue_step(c, from, eps, nullptr, field_ready);
+            cudaError_t le = enqueue_step(c, from, eps, nullptr, field_ready, rows);
             cudaError_t ee = cudaStreamEndCapture(c->stream, &g);
             if (le != cudaSuccess) {
                 if (g) cudaGraphDestroy(g);
@@ -247,7 +265,7 @@ int run_step(ymflow_ctx* c, double eps, cudaEvent_t* ev, bool field_ready = fals
         }
         YM_CK(c, cudaGraphLaunch(c->graph[k], c->stream), "launch step graph");
     } else {
-        YM_CK(c, enqueue_step(c, from, eps, ev, field_ready), "stage launch");
+        YM_CK(c, enqueue_step(c, from, eps, ev, field_ready, rows), "stage launch");
     }
     c->cur = 1 - from;
     return YMFLOW_OK;
@@ -268,12 +286,12 @@ cudaError_t enqueue_stage(ymflow_ctx* c, int stage, const void* in, void* out, d
 }
 
 // Observables of the current field into meas row `row` (device).
-int enqueue_measure(ymflow_ctx* c, int row) {
+int enqueue_measure(ymflow_ctx* c, int row, bool rows_in) {
     int r = ensure_partials(c);
     if (r != YMFLOW_OK) return r;
     if (measures_from_field(c)) {
         YM_CK(c, launch_measure_from_field(c->prec, c->u[c->cur], c->hfield, plaq_range(c->geo, c->slab), c->geo,
-                                           c->partials, c->meas + 4 * row, c->stream),
+                                           c->partials, c->meas + 4 * row, c->stream, rows_in),
               "observables launch");
     } else {
         YM_CK(c, launch_observables(c->prec, c->u[c->cur], c->geo, c->partials, c->stream), "observables launch");
@@ -745,16 +763,17 @@ int ymflow_flow(ymflow_ctx* c, double eps, int nsteps, int measure_every, int re
     row_t[row] = c->t;
     row++;
     const bool from_field = measures_from_field(c);
+    const bool by_rows = steps_by_rows(c);
     bool field_ready = from_field;  // a measured row leaves its plaquette field for the next step's stage 0
     for (int s = 1; s <= nsteps; s++) {
-        if ((r = run_step(c, eps, nullptr, field_ready)) != YMFLOW_OK) return r;
+        if ((r = run_step(c, eps, s, nsteps, nullptr, field_ready)) != YMFLOW_OK) return r;
         field_ready = false;
         c->step++;
         c->t += eps;
         if (reunit && s % reunit_every == 0)
             YM_CK(c, launch_reunitarize(c->prec, c->u[c->cur], c->geo, c->deviation, c->stream), "reunitarise");
         if ((measure_every > 0 && s % measure_every == 0) || s == nsteps) {
-            if ((r = enqueue_measure(c, row)) != YMFLOW_OK) return r;
+            if ((r = enqueue_measure(c, row, by_rows)) != YMFLOW_OK) return r;
             row_step[row] = c->step;
             row_t[row] = c->t;
             row++;
@@ -854,7 +873,7 @@ int ymflow_time_kernels(ymflow_ctx* c, double eps, int nsteps, float* elapsed_ms
     const bool reunit = c->prec != YMFLOW_FP64 && c->timed_reunit > 0;
     YM_CK(c, cudaEventRecord(c->ev0, c->stream), "event record");
     for (int s = 0; s < nsteps; s++) {
-        int r = run_step(c, eps, per_kernel ? c->events.data() + 9 * s : nullptr);
+        int r = run_step(c, eps, s + 1, nsteps, per_kernel ? c->events.data() + 9 * s : nullptr);
         if (r != YMFLOW_OK) return r;
         c->step++;
         c->t += eps;
