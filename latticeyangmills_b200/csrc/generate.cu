@@ -21,6 +21,8 @@
 // (link, sweep, hit) come from Philox4x32-10 keyed by the seed with counter
 // (link index, sweep, hit, call), so the chain does not depend on the launch
 // shape; oracle/ymoracle.c runs the same chain on the CPU.
+#include <cmath>
+
 #include "field.cuh"
 #include "kernels.h"
 
@@ -31,43 +33,113 @@ namespace {
 __device__ __forceinline__ uint4 philox_g(uint4 c, uint2 k) {
 #pragma unroll
     for (int r = 0; r < 10; r++) {
-        const uint32_t hi0 = __umulhi(0xD2511F53u, c.x), lo0 = 0xD2511F53u * c.x;
-        const uint32_t hi1 = __umulhi(0xCD9E8D57u, c.z), lo1 = 0xCD9E8D57u * c.z;
-        c = make_uint4(hi1 ^ c.y ^ k.x, lo1, hi0 ^ c.w ^ k.y, lo0);
+        const uint64_t p0 = uint64_t(0xD2511F53u) * c.x, p1 = uint64_t(0xCD9E8D57u) * c.z;
+        c = make_uint4(uint32_t(p1 >> 32) ^ c.y ^ k.x, uint32_t(p1), uint32_t(p0 >> 32) ^ c.w ^ k.y, uint32_t(p0));
         k.x += 0x9E3779B9u;
         k.y += 0xBB67AE85u;
     }
     return c;
 }
 
+// Uniform (w + 1/2) / 2^32 of a random word.
 __device__ __forceinline__ double unit(uint32_t w) { return (double(w) + 0.5) * 2.3283064365386963e-10; }
 
-// one embedded SU(2) element from four uniforms, on rows/columns (p, q)
-template <class R>
-__device__ __forceinline__ void su2_in(const double x[4], double eps, int p, int q, M3<R>& m) {
-    double v1 = x[1] - 0.5, v2 = x[2] - 0.5, v3 = x[3] - 0.5;
-    const double norm = sqrt(v1 * v1 + v2 * v2 + v3 * v3);
-    const double x0 = (x[0] - 0.5 < 0.0 ? -1.0 : 1.0) * sqrt(1.0 - eps * eps);
-    v1 = v1 * eps / norm;
-    v2 = v2 * eps / norm;
-    v3 = v3 * eps / norm;
-    mzero(m);
-    m.e[0][0].re = m.e[1][1].re = m.e[2][2].re = R(1);
-    m.e[p][p] = cx(R(x0), R(v3));
-    m.e[q][q] = cx(R(x0), R(-v3));
-    m.e[p][q] = cx(R(v2), R(v1));
-    m.e[q][p] = cx(R(-v2), R(v1));
+// 2 w + 1 - 2^32, exactly: 2^33 (unit(w) - 1/2), from the word set into a
+// double's low bits (one addition instead of a conversion).
+__device__ __forceinline__ double centred(uint32_t w) {
+    return __hiloint2double(int(0x43300000u | (w >> 31)), int((w << 1) | 1u)) - (4503599627370496.0 + 4294967296.0);
 }
 
+// An embedded SU(2) element [[a, b], [-conj b, conj a]] from four random words:
+// Re a = +-x0 with the first word's sign, the other three components eps long
+// in a uniform direction.
+template <class R>
+struct Su2 {
+    Cx<R> a, b;
+};
+
+// 1 / sqrt(n) by Newton's iteration from the FP32 value (relative error below
+// 2^-22, then 2^-43, then FP64 rounding); n within FP32's range.  No branch, so
+// several proposals' chains can be interleaved.
+__device__ __forceinline__ double rsqrt_newton(double n) {
+    double y = double(rsqrtf(float(n)));
+    const double hn = 0.5 * n;
+#pragma unroll
+    for (int i = 0; i < 2; i++) y = fma(y, fma(-hn * y, y, 0.5), y);
+    return y;
+}
+
+template <class R>
+__device__ __forceinline__ Su2<R> su2_from(const uint4& o, double eps, double x0) {
+    const double v1 = centred(o.y), v2 = centred(o.z), v3 = centred(o.w);
+    const double len = eps * rsqrt_newton(fma(v1, v1, fma(v2, v2, v3 * v3)));
+    Su2<R> m;
+    m.a = cx(R(o.x < 0x80000000u ? -x0 : x0), R(v3 * len));
+    m.b = cx(R(v2 * len), R(v1 * len));
+    return m;
+}
+
+template <class R>
+__device__ __forceinline__ Cx<R> cmul(const Cx<R>& x, const Cx<R>& y) {
+    return cx(fma(x.re, y.re, -x.im * y.im), fma(x.re, y.im, x.im * y.re));
+}
+// x y + z w
+template <class R>
+__device__ __forceinline__ Cx<R> cmul2(const Cx<R>& x, const Cx<R>& y, const Cx<R>& z, const Cx<R>& w) {
+    return cx(fma(x.re, y.re, fma(-x.im, y.im, fma(z.re, w.re, -z.im * w.im))),
+              fma(x.re, y.im, fma(x.im, y.re, fma(z.re, w.im, z.im * w.re))));
+}
+template <class R>
+__device__ __forceinline__ Cx<R> neg_conj(const Cx<R>& x) {
+    return cx(-x.re, x.im);
+}
+template <class R>
+__device__ __forceinline__ Cx<R> conj_of(const Cx<R>& x) {
+    return cx(x.re, -x.im);
+}
+
+// R S T of SU(2) elements in the (0,1), (0,2) and (1,2) blocks: twelve complex
+// products, the zeros of the factors left out.
+template <class R>
+__device__ __forceinline__ void rst_product(const Su2<R>& r, const Su2<R>& s, const Su2<R>& t, M3<R>& x) {
+    const Cx<R> rc = neg_conj(r.b), rd = conj_of(r.a);  // row 1 of R
+    const Cx<R> sc = neg_conj(s.b), sd = conj_of(s.a);  // row 2 of S
+    const Cx<R> tc = neg_conj(t.b), td = conj_of(t.a);  // row 2 of T
+    const Cx<R> p02 = cmul(r.a, s.b), p12 = cmul(rc, s.b);
+    x.e[0][0] = cmul(r.a, s.a);
+    x.e[0][1] = cmul2(r.b, t.a, p02, tc);
+    x.e[0][2] = cmul2(r.b, t.b, p02, td);
+    x.e[1][0] = cmul(rc, s.a);
+    x.e[1][1] = cmul2(rd, t.a, p12, tc);
+    x.e[1][2] = cmul2(rd, t.b, p12, td);
+    x.e[2][0] = sc;
+    x.e[2][1] = cmul(sd, tc);
+    x.e[2][2] = cmul(sd, td);
+}
+
+// exp(x) > r for r = unit(w), in FP32: 1, 0, or -1 where the two are closer
+// than the FP32 evaluation can be off (about one call in 10^5, and NaN).
+__device__ __forceinline__ int exp_exceeds_fp32(double x, uint32_t w) {
+    const float xf = float(x);
+    const float e = expf(xf), r = fmaf(float(w), 2.3283064e-10f, 1.1641532e-10f);
+    // x rounded to FP32: |x| 2^-24; expf: 2 ulp; r: 2 roundings; doubled
+    const float off = fmaf(e, fmaf(fabsf(xf), 1.2e-7f, 5e-7f), r * 3e-7f);
+    return fabsf(e - r) > off ? int(e > r) : -1;
+}
+
+// This lane's part of the staple sum: every `group`-th of the three directions
+// nu != mu, from the `j`-th.
 template <class F>
-__device__ __forceinline__ M3<typename F::Real> staple_sum(const F& u, const Geo& g, int s, const int c[4], int mu) {
+__device__ __forceinline__ M3<typename F::Real> staple_part(const F& u, const Geo& g, int s, const int c[4], int mu,
+                                                            int j, int group) {
     using R = typename F::Real;
     M3<R> omega;
     mzero(omega);
     const int cmu = g.coord(c, mu);
     const int s_pm = g.hop_rt(s, cmu, mu, +1);
-    for (int nu = 0; nu < 4; nu++) {
-        if (nu == mu) continue;
+#pragma unroll 1
+    for (int k = j; k < 3; k += group) {
+        const int nu = k + (k >= mu ? 1 : 0);
         const int cnu = g.coord(c, nu);
         const int s_pn = g.hop_rt(s, cnu, nu, +1);
         const int s_mn = g.hop_rt(s, cnu, nu, -1);
@@ -81,49 +153,99 @@ __device__ __forceinline__ M3<typename F::Real> staple_sum(const F& u, const Geo
     return omega;
 }
 
-template <class F>
-__global__ void __launch_bounds__(128) metropolis_kernel(F u, Geo g, int mu, int parity, double beta, double eps,
-                                                         int hits, uint64_t seed, uint32_t sweep,
-                                                         unsigned long long* accepted) {
-    using R = typename F::Real;
-    const int s = int(blockIdx.x) * blockDim.x + threadIdx.x;
-    unsigned acc = 0;
-    if (s < g.V) {
-        int c[4];
-        g.coords(s, c);
-        if (((c[0] + c[1] + c[2] + c[3]) & 1) == parity) {
-            const M3<R> A = staple_sum(u, g, s, c, mu);
-            M3<R> U = u.load(mu, s);
-            const uint64_t l = uint64_t(s) * 4 + uint64_t(mu);
-            const uint2 key = make_uint2(uint32_t(seed), uint32_t(seed >> 32) ^ 0x4D455452u);
-            for (int h = 0; h < hits; h++) {
-                double r[16];
+constexpr int kMetroThreads = 64;
+
+// Proposal `hit` of link l: X, the acceptance draw's word, and beta/3 Re tr[(U' -
+// U) A] = beta/3 Re tr[(X - 1) W], W = U A.
+template <class R>
+__device__ __forceinline__ double propose(uint32_t l0, uint32_t l1, uint32_t sweep, uint32_t hit, uint2 key,
+                                          double eps, double x0, double beta_3, const M3<R>& W, M3<R>& X,
+                                          uint32_t& draw) {
+    const uint4 oa = philox_g(make_uint4(l0, l1, sweep, hit), key);
+    const uint4 ob = philox_g(make_uint4(l0, l1 ^ (1u << 24), sweep, hit), key);
+    const uint4 oc = philox_g(make_uint4(l0, l1 ^ (2u << 24), sweep, hit), key);
+    const uint4 od = philox_g(make_uint4(l0, l1 ^ (3u << 24), sweep, hit), key);
+    M3<R> m;
+    rst_product(su2_from<R>(oa, eps, x0), su2_from<R>(ob, eps, x0), su2_from<R>(oc, eps, x0), m);
+    const bool inverse = od.y < 0x80000000u;  // X^+ with probability 1/2
 #pragma unroll
-                for (uint32_t call = 0; call < 4; call++) {
-                    const uint4 o = philox_g(make_uint4(uint32_t(l), uint32_t(l >> 32) ^ (call << 24), sweep, uint32_t(h)), key);
-                    r[4 * call + 0] = unit(o.x);
-                    r[4 * call + 1] = unit(o.y);
-                    r[4 * call + 2] = unit(o.z);
-                    r[4 * call + 3] = unit(o.w);
-                }
-                M3<R> a, b, ab, X, Un;
-                su2_in(r + 0, eps, 0, 1, a);
-                su2_in(r + 4, eps, 0, 2, b);
-                mmul<false, false>(a, b, ab);
-                su2_in(r + 8, eps, 1, 2, a);
-                mmul<false, false>(ab, a, X);
-                if (r[13] < 0.5)
-                    mmul<true, false>(X, U, Un);
-                else
-                    mmul<false, false>(X, U, Un);
-                // dS = -(beta/3) Re tr[(U' - U) A]
-                const R dtr = re_trace_mul(Un, A) - re_trace_mul(U, A);
-                const double dS = -beta / 3.0 * double(dtr);
-                if (exp(-dS) > r[12]) {
-                    U = Un;
-                    acc++;
-                }
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++)
+            X.e[i][j] = cx(inverse ? m.e[j][i].re : m.e[i][j].re, inverse ? -m.e[j][i].im : m.e[i][j].im);
+    R dtr = R(0);
+#pragma unroll
+    for (int i = 0; i < 3; i++) {  // one sum per row of X
+        R d = R(0);
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            d = fma(i == j ? X.e[i][j].re - R(1) : X.e[i][j].re, W.e[j][i].re, d);
+            d = fma(-X.e[i][j].im, W.e[j][i].im, d);
+        }
+        dtr += d;
+    }
+    draw = od.x;
+    return beta_3 * double(dtr);
+}
+
+// One thread per link of the (mu, parity) class; link h's site is the one of
+// that parity in the x pair (2h, 2h + 1) (extents are even).  The trace change
+// of a proposal needs W = U A only, so U (kept in shared memory) and W are
+// multiplied by X only when it is accepted.
+//
+// Bound by the chain of a hit (some 600 FP64 and integer instructions, one
+// issued every 3 to 4 cycles per warp; FP64 pipe at 42 %).  16^4, 30 hits, FP64
+// on B200: 53 us per launch, 32^4 0.58 ms, against 153 us and 2.4 ms with one
+// thread per site, half of them idle, and every proposal multiplied out as
+// dense matrices.  Two or three proposals per thread at a time (all but the
+// first accepted one discarded) gained nothing: 52 and 55 us.
+template <class F>
+__global__ void __launch_bounds__(kMetroThreads, 5)
+    metropolis_kernel(F u, Geo g, int mu, int parity, double beta_3, double eps, double x0, int hits, uint64_t seed,
+                      uint32_t sweep, unsigned long long* accepted) {
+    using R = typename F::Real;
+    __shared__ Cx<R> links[9][kMetroThreads];
+    const int h2 = 2 * (int(blockIdx.x) * blockDim.x + threadIdx.x);
+    unsigned acc = 0;
+    if (h2 < g.V) {
+        int c[4];
+        g.coords(h2, c);
+        const int odd = (c[1] + c[2] + c[3] + parity) & 1;
+        const int s = h2 + odd;
+        c[0] += odd;
+        M3<R> W;
+        {
+            const M3<R> A = staple_part(u, g, s, c, mu, 0, 1);
+            const M3<R> U = u.load(mu, s);
+            mmul<false, false>(U, A, W);
+#pragma unroll
+            for (int e = 0; e < 9; e++) links[e][threadIdx.x] = U.e[e / 3][e % 3];
+        }
+        const uint64_t l = uint64_t(s) * 4 + uint64_t(mu);
+        const uint32_t l0 = uint32_t(l), l1 = uint32_t(l >> 32);
+        const uint2 key = make_uint2(uint32_t(seed), uint32_t(seed >> 32) ^ 0x4D455452u);
+        for (int h = 0; h < hits; h++) {
+            M3<R> X;
+            uint32_t draw;
+            const double x = propose(l0, l1, sweep, uint32_t(h), key, eps, x0, beta_3, W, X, draw);
+            int ok = exp_exceeds_fp32(x, draw);
+            if (ok < 0) ok = exp(x) > unit(draw);
+            if (ok) {
+                M3<R> U, t;
+#pragma unroll
+                for (int e = 0; e < 9; e++) U.e[e / 3][e % 3] = links[e][threadIdx.x];
+                mmul<false, false>(X, U, t);
+#pragma unroll
+                for (int e = 0; e < 9; e++) links[e][threadIdx.x] = t.e[e / 3][e % 3];
+                mmul<false, false>(X, W, t);
+                W = t;
+                acc++;
             }
+        }
+        if (acc) {
+            M3<R> U;
+#pragma unroll
+            for (int e = 0; e < 9; e++) U.e[e / 3][e % 3] = links[e][threadIdx.x];
             u.store(mu, s, U);
         }
     }
@@ -133,13 +255,114 @@ __global__ void __launch_bounds__(128) metropolis_kernel(F u, Geo g, int mu, int
     if ((threadIdx.x & 31) == 0 && acc) atomicAdd(accepted, (unsigned long long)acc);
 }
 
+// The same with G lanes per link.  The lanes of a link share its staples, then draw the next G
+// proposals against the same W, one each; the first accepted one is taken and
+// the later ones are drawn again from the new link, so the chain is that of
+// one proposal after another.  X passes through shared memory; the first lane
+// then multiplies W, the others U (one multiplication in the warp).
+//
+// For lattices that leave schedulers without a warp (launch_metro_typed).
+template <class F, int G>
+__global__ void __launch_bounds__(kMetroThreads, 8)
+    metropolis_lanes_kernel(F u, Geo g, int mu, int parity, double beta_3, double eps, double x0, int hits,
+                            uint64_t seed, uint32_t sweep, unsigned long long* accepted) {
+    using R = typename F::Real;
+    __shared__ Cx<R> shared[9][kMetroThreads / G];  // a link's accepted X, then its new W
+    const int lane = int(threadIdx.x & 31), j = lane & (G - 1), slot = int(threadIdx.x) / G;
+    const int h2 = 2 * (int(blockIdx.x) * (kMetroThreads / G) + slot);
+    const bool link = h2 < g.V;
+    unsigned acc = 0;
+    M3<R> W, M;  // M: W in lane 0 of the link, U in the others
+    mzero(W);
+    int s = 0;
+    if (link) {
+        int c[4];
+        g.coords(h2, c);
+        const int odd = (c[1] + c[2] + c[3] + parity) & 1;
+        s = h2 + odd;
+        c[0] += odd;
+        W = staple_part(u, g, s, c, mu, j, G);
+        M = u.load(mu, s);
+    }
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1)
+#pragma unroll
+        for (int e = 0; e < 9; e++) {
+            W.e[e / 3][e % 3].re += __shfl_xor_sync(0xffffffffu, W.e[e / 3][e % 3].re, o);
+            W.e[e / 3][e % 3].im += __shfl_xor_sync(0xffffffffu, W.e[e / 3][e % 3].im, o);
+        }
+    {
+        const M3<R> A = W;
+        mmul<false, false>(M, A, W);
+        if (j == 0) M = W;
+    }
+    const uint64_t l = uint64_t(s) * 4 + uint64_t(mu);
+    const uint32_t l0 = uint32_t(l), l1 = uint32_t(l >> 32);
+    const uint2 key = make_uint2(uint32_t(seed), uint32_t(seed >> 32) ^ 0x4D455452u);
+    int h = link ? 0 : hits;
+    while (__any_sync(0xffffffffu, h < hits)) {
+        M3<R> X;
+        uint32_t draw;
+        const double x = propose(l0, l1, sweep, uint32_t(h + j), key, eps, x0, beta_3, W, X, draw);
+        int ok = exp_exceeds_fp32(x, draw);
+        if (ok < 0) ok = exp(x) > unit(draw);
+        const unsigned all = __ballot_sync(0xffffffffu, ok && h + j < hits);
+        const unsigned mine = (all >> (lane & ~(G - 1))) & ((1u << G) - 1u);
+        const int first = __ffs(int(mine)) - 1;
+        if (j == first) {
+#pragma unroll
+            for (int e = 0; e < 9; e++) shared[e][slot] = X.e[e / 3][e % 3];
+        }
+        __syncwarp();
+        if (mine) {
+#pragma unroll
+            for (int e = 0; e < 9; e++) X.e[e / 3][e % 3] = shared[e][slot];
+            M3<R> t;
+            mmul<false, false>(X, M, t);
+            M = t;
+        }
+        __syncwarp();
+        if (mine && j == 0) {
+            acc++;
+#pragma unroll
+            for (int e = 0; e < 9; e++) shared[e][slot] = M.e[e / 3][e % 3];
+        }
+        __syncwarp();
+        if (mine) {
+#pragma unroll
+            for (int e = 0; e < 9; e++) W.e[e / 3][e % 3] = shared[e][slot];
+        }
+        __syncwarp();  // read before the next accepted X is written
+        h = mine ? h + first + 1 : h + G;
+    }
+    acc = __shfl_sync(0xffffffffu, acc, lane & ~(G - 1));
+    if (link && j == 1 && acc) u.store(mu, s, M);
+    if (j != 0) acc = 0;
+    // warp sum, one atomic per warp
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if (lane == 0 && acc) atomicAdd(accepted, (unsigned long long)acc);
+}
+
 template <class F>
 cudaError_t launch_metro_typed(void* u, const Geo& g, int mu, int parity, double beta, double eps, int hits,
                                uint64_t seed, uint32_t sweep, unsigned long long* accepted, cudaStream_t st) {
-    const int b = 128;
-    metropolis_kernel<F><<<unsigned((g.V + b - 1) / b), b, 0, st>>>(F{u, g.V}, g, mu, parity, beta, eps, hits, seed,
-                                                                     sweep, accepted);
-    return cudaGetLastError();
+    const unsigned links = unsigned(g.V / 2);
+    const double x0 = std::sqrt(std::fma(-eps, eps, 1.0));
+    auto launch = [&](auto kernel, unsigned lanes) {
+        const unsigned per_block = kMetroThreads / lanes;
+        kernel<<<(links + per_block - 1) / per_block, kMetroThreads, 0, st>>>(F{u, g.V}, g, mu, parity, beta / 3.0, eps,
+                                                                              x0, hits, seed, sweep, accepted);
+        return cudaGetLastError();
+    };
+    // One thread per link needs about 15,000 links (three warps on each of the
+    // SM's schedulers, in all 148 SMs) before its work rather than its chain of
+    // hits sets the time; fewer links are given more lanes.  us per launch on
+    // B200 (FP64, 30 hits) at 1 / 4 / 8 lanes: 6^4 30 / 17 / 14, 8^4 31 / 17 /
+    // 15, 12^4 33 / 28 / 34, 16^4 53 / 62 / 77 (2 lanes are never the fastest).
+    if (links <= 4736) return launch(metropolis_lanes_kernel<F, 8>, 8);
+    if (links <= 14208) return launch(metropolis_lanes_kernel<F, 4>, 4);
+    return launch(metropolis_kernel<F>, 1);
 }
 
 }  // namespace

@@ -93,3 +93,21 @@ def test_generate_rejects_bad_arguments():
     with GluonField((4, 4, 4, 5), "fp64") as f:
         with pytest.raises(YmflowError):
             f.generate_metropolis(BETA, EPS, 1, 1, 1, "cold")
+
+
+@pytest.mark.parametrize("n", [(2, 2, 2, 2), (6, 6, 6, 6), (10, 8, 10, 12), (12, 10, 12, 10), (16, 16, 16, 8)], ids=str)
+@pytest.mark.parametrize("hits", [1, 7])
+def test_every_lane_count_runs_the_same_chain(oracle, n, hits):
+    """8, 4 or 1 lanes per link by the number of links, whole and partial warps:
+    the oracle's chain, accept for accept (tolerance as above)."""
+    U = oracle.gen_cold(n)
+    oracle.gen_haar_mix(U, n, 0.3, 13, 0)
+    from latticeyangmills_b200 import GluonField
+
+    with GluonField(n, "fp64") as f:
+        f.upload(U)
+        frac = f.generate_metropolis(BETA, EPS, 1, hits, 21, "current")
+        got = f.download()
+    acc = oracle.gen_metropolis_cb(U, n, BETA, EPS, 1, hits, 21)
+    assert round(frac * hits * 4 * oracle.volume(n)) == acc
+    assert np.abs(got - U).max() < 1e-12
