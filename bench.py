@@ -32,7 +32,7 @@ the single slab exchanges with itself, which prices the exchange on one GPU.
 
 The JSON line carries, besides the contract's keys: `roofline` (HBM: the
 compulsory bytes of a stage, 6 s_U + 4 s_Z per link-update over three
-launches, over the stage kernel's time in the graph-replayed steps, `frac`;
+launches, over the stage kernel's time in the uninstrumented steps, `frac`;
 the whole step's fraction, `step_frac_8d`; the DRAM bytes the ncu captures in
 profiles/ count, over the compulsory ones; `field_kernel` the plaquette-field
 kernel of the two-kernel stage on its own bytes),
@@ -485,11 +485,11 @@ def our_arm(args, dist: Dist):
             print(json.dumps({"profile": True, "precision": prec, "lattice": list(DIMS), "stage_form": form,
                               "ms_per_step": elapsed_ms / args.steps}))
         return
-    # The stage kernels alone, in the same graph-replayed execution without the
+    # The stage kernels alone, in the same execution without the
     # reunitarisation (per launch: a third of a step), and with events around
-    # every launch of a third pass (instrumented: no graph).
+    # every launch of a third pass (instrumented).
     f.set_option(N.OPT_TIMED_REUNIT, 0)
-    graph_ms, _ = f.time_steps(EPS, args.steps)
+    plain_ms, _ = f.time_steps(EPS, args.steps)
     _, field_ms, stage_ms = f.time_kernels(EPS, args.steps)
     f.set_option(N.OPT_TIMED_REUNIT, reunit)
     clocks.stop()
@@ -516,10 +516,10 @@ def our_arm(args, dist: Dist):
     kprefix, kname = STAGE_KERNELS[form]
     split = form == 1
     kernels_per_stage = 2 if split else 1
-    if split:  # the stage kernel's share of the graph-timed stage, from the instrumented pass
-        stage_launch_s = graph_ms / 1e3 / (3 * args.steps) * stage_ms / (field_ms + stage_ms)
+    if split:  # the stage kernel's share of the step, from the instrumented pass
+        stage_launch_s = plain_ms / 1e3 / (3 * args.steps) * stage_ms / (field_ms + stage_ms)
     else:
-        stage_launch_s = graph_ms / 1e3 / (3 * args.steps)
+        stage_launch_s = plain_ms / 1e3 / (3 * args.steps)
     roof = roofline_8d(prec, links, value / dist.world, stage_launch_s, peak)
     alg = roof["algorithmic_bytes_per_launch"]
     traffic = profiled_traffic(prec, DIMS, alg, kprefix)
@@ -540,7 +540,7 @@ def our_arm(args, dist: Dist):
     # time, against the measured CUDA-core FMA peak
     fma_tf = ctypes.c_double(0.0)
     N.check(N.load().ymflow_fma_peak(dev, N.FP64 if prec == "fp64" else N.FP32_18, ctypes.byref(fma_tf)))
-    alu_achieved = links * FLOPS_PER_LINK_STAGE / (graph_ms / 1e3 / (3 * args.steps)) / 1e12
+    alu_achieved = links * FLOPS_PER_LINK_STAGE / (plain_ms / 1e3 / (3 * args.steps)) / 1e12
 
     # accuracy of the mixed form against FP64 at t = 4 (400 steps), same seeded field
     accuracy = None
@@ -605,7 +605,7 @@ def our_arm(args, dist: Dist):
                        "lattice": list(DIMS), "precision": prec,
                        "reductions": "f64", "l2": "inputs larger than L2 (links + generator > 126 MB)",
                        "reunit_every": reunit or None,
-                       "timed_region": "K RK3 steps%s, graph-replayed" % (
+                       "timed_region": "K RK3 steps%s" % (
                            ", with the FP64 reunitarisation after every %d-th (%d launches)" % (reunit, n_reunit)
                            if reunit else ""),
                        "parallelism": "replicas x%d" % dist.world,
@@ -621,7 +621,7 @@ def our_arm(args, dist: Dist):
                          "algorithmic_bytes_per_launch": alg,
                          "avg_launch_ms": stage_launch_s * 1e3,
                          "avg_launch_ms_events": stage_ms / (3 * args.steps),
-                         "launch_time_from": "graph-replayed steps without the reunitarisation, a third of a "
+                         "launch_time_from": "uninstrumented steps without the reunitarisation, a third of a "
                                              "step per stage launch%s" % (
                                                  " times the stage kernel's share of the instrumented pass"
                                                  if split else ""),

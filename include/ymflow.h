@@ -203,8 +203,9 @@ YMFLOW_API int ymflow_time_kernels(ymflow_ctx* ctx, double eps, int nsteps, floa
  * (128: four warps, one per direction, per 32 sites); YMFLOW_OPT_OBS_BLOCK:
  * threads per block of the observables kernel (192: six warps, one per
  * plane, per 32 sites; read-only in effect, other values are rejected);
- * YMFLOW_OPT_GRAPH: 1 = replay each RK3 step as a captured CUDA graph
- * (default), 0 = plain launches; YMFLOW_OPT_STAGE_FORM: the kernels of one RK3
+ * YMFLOW_OPT_GRAPH: 1 = replay each RK3 step of stage form 2 as a captured
+ * CUDA graph (default), 0 = plain launches (forms 0 and 1 launch their kernels
+ * chained, by programmatic dependent launch, either way); YMFLOW_OPT_STAGE_FORM: the kernels of one RK3
  * stage (the reference's computeDerivative + exp + link update for all mu,
  * src/Apps/wilsonflow.cpp:143-171):
  *   0 = one fused kernel, staples summed per link (the FP64 default where

@@ -35,10 +35,9 @@ struct ymflow_ctx {
     int meas_cap = 0;
     double* meas_host = nullptr;      // pinned copy of the rows
     unsigned long long* deviation = nullptr;  // reunitarisation drift (ordered bits)
-    // the step from u[k & 1]; k & 2: with its plaquette field ready
-    cudaGraphExec_t graph[4] = {nullptr, nullptr, nullptr, nullptr};
-    double graph_eps[4] = {0.0, 0.0, 0.0, 0.0};
-    int graph_block[4] = {0, 0, 0, 0};
+    cudaGraphExec_t graph[2] = {nullptr, nullptr};  // stage form 2: the step from u[k]
+    double graph_eps[2] = {0.0, 0.0};
+    int graph_block[2] = {0, 0};
     std::vector<cudaEvent_t> events;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int block = 128;

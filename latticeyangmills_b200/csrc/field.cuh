@@ -177,6 +177,18 @@ inline void set_tiled_order(Geo& g, int target) {
 
 inline int64_t padded_sites(int64_t V) { return (V + 31) & ~int64_t(31); }
 
+// In a kernel that launch_chained may start early: waits for the grid before.
+// Nothing of what another grid writes is read before it, nor is anything
+// written.
+__device__ __forceinline__ void grid_wait() { cudaGridDependencySynchronize(); }
+// Lets the next chained kernel be placed, once every block is here (without
+// effect where the next launch is not chained).  Called before a thread's last
+// stores: earlier, the next kernel's blocks settle on the SMs that happen to
+// have room while most are full, and run unevenly spread (8^3 x 12 FP32-12:
+// 30 us per step with the call at the kernel's start, 16.2 here, 17.4 without
+// it, 20.5 as a graph of unchained launches).
+__device__ __forceinline__ void grid_release() { cudaTriggerProgrammaticLaunchCompletion(); }
+
 // First 16-byte unit of the (mu, group of s) block run, plus the lane of s;
 // `units` = 16-byte units per group (32 x bytes per link / 16).
 __device__ __forceinline__ uint32_t group_lane_unit(int mu, int s, int V, int units) {
@@ -187,6 +199,15 @@ __device__ __forceinline__ uint32_t group_lane_unit(int mu, int s, int V, int un
 template <class R>
 __device__ __forceinline__ void set_elem(M3<R>& a, int e, R re, R im) {
     a.e[e / 3][e % 3] = cx(re, im);
+}
+
+// One vector of a field.  RO: through the read-only path, which the compiler may
+// move ahead of a wait for the grid that wrote the field; kernels launched on
+// that grid's heels (launch_chained) read with RO = false.
+template <bool RO, class V>
+__device__ __forceinline__ V read_vec(const V* p) {
+    if constexpr (RO) return __ldg(p);
+    return *p;
 }
 
 // Link field of NE stored complex elements per link (9: full, 6: two rows).
@@ -205,22 +226,24 @@ struct LinkField<double, NE> {
     __device__ __forceinline__ const double2* link(int mu, int s) const {
         return reinterpret_cast<const double2*>(p) + group_lane_unit(mu, s, V, kUnits);
     }
+    template <bool RO = true>
     __device__ __forceinline__ Rows2<double> load_rows2(int mu, int s) const {
         const double2* b = link(mu, s);
         Rows2<double> a;
 #pragma unroll
         for (int e = 0; e < 6; e++) {
-            const double2 v = __ldg(b + 32 * e);
+            const double2 v = read_vec<RO>(b + 32 * e);
             a.e[e / 3][e % 3] = cx(v.x, v.y);
         }
         return a;
     }
+    template <bool RO = true>
     __device__ __forceinline__ M3<double> load(int mu, int s) const {
         const double2* b = link(mu, s);
         M3<double> a;
 #pragma unroll
         for (int e = 0; e < NE; e++) {
-            const double2 v = __ldg(b + 32 * e);
+            const double2 v = read_vec<RO>(b + 32 * e);
             set_elem(a, e, v.x, v.y);
         }
         if (NE == 6) reconstruct_row2(a);
@@ -266,28 +289,30 @@ struct LinkField<float, NE> {
     __device__ __forceinline__ const float2* tail(const float4* l, int s) const {
         return reinterpret_cast<const float2*>(l - (s & 31) + 32 * kPairs) + (s & 31);
     }
+    template <bool RO = true>
     __device__ __forceinline__ Rows2<float> load_rows2(int mu, int s) const {
         const float4* b = link(mu, s);
         Rows2<float> a;
 #pragma unroll
         for (int k = 0; k < 3; k++) {
-            const float4 v = __ldg(b + 32 * k);
+            const float4 v = read_vec<RO>(b + 32 * k);
             a.e[(2 * k) / 3][(2 * k) % 3] = cx(v.x, v.y);
             a.e[(2 * k + 1) / 3][(2 * k + 1) % 3] = cx(v.z, v.w);
         }
         return a;
     }
+    template <bool RO = true>
     __device__ __forceinline__ M3<float> load(int mu, int s) const {
         const float4* b = link(mu, s);
         M3<float> a;
 #pragma unroll
         for (int k = 0; k < kPairs; k++) {
-            const float4 v = __ldg(b + 32 * k);
+            const float4 v = read_vec<RO>(b + 32 * k);
             set_elem(a, 2 * k, v.x, v.y);
             set_elem(a, 2 * k + 1, v.z, v.w);
         }
         if (NE == 9) {
-            const float2 v = __ldg(tail(b, s));
+            const float2 v = read_vec<RO>(tail(b, s));
             set_elem(a, 8, v.x, v.y);
         } else {
             reconstruct_row2(a);
@@ -327,9 +352,10 @@ using FieldD18 = LinkField<double, 9>;
 // launch, the field kernel 0.232 -> 0.204, both then at 57-63 % of the FP64 pipe
 // and 40-63 % of HBM.
 struct FieldD18Rows : LinkField<double, 9> {
+    template <bool RO = true>
     __device__ __forceinline__ M3<double> load(int mu, int s) const {
         M3<double> a;
-        full_from_rows2(load_rows2(mu, s), a);
+        full_from_rows2(load_rows2<RO>(mu, s), a);
         return a;
     }
     __device__ __forceinline__ void store_rows2(int mu, int s, const Rows2<double>& a) const {

@@ -26,8 +26,9 @@ __global__ void __launch_bounds__(128, StageMinBlocks<F>::value)
     int s;
     int mu;
     link_of_thread<sizeof(typename F::Real) == 8>(g, s, mu);
+    grid_wait();
     if (s >= g.site1) return;
-    rk_link_update<F, STAGE>(in, out, zf, g, eps, s, mu);
+    rk_link_update<F, STAGE, false>(in, out, zf, g, eps, s, mu);
 }
 
 // The same stage for a slab whose boundary links also go straight into its
@@ -63,19 +64,19 @@ static cudaError_t launch_halo_typed(int stage, const void* uin, void* uout, voi
 
 template <class F>
 static cudaError_t launch_typed(int stage, const void* uin, void* uout, void* z, const Geo& g, double eps, int block,
-                                cudaStream_t st) {
+                                bool chained, cudaStream_t st) {
     using R = typename F::Real;
     F in{const_cast<void*>(uin), g.V}, out{uout, g.V};
     ForceField<R> zf{z, g.V};
     const int sites_per_block = block / 4;
-    dim3 grid(unsigned((g.site1 - g.site0 + sites_per_block - 1) / sites_per_block));
+    const unsigned grid = unsigned((g.site1 - g.site0 + sites_per_block - 1) / sites_per_block);
     const R e = R(stage == 0 ? eps * 0.25 : eps);
+    auto launch = [&](auto kernel) { return launch_chained(chained, kernel, grid, unsigned(block), st, in, out, zf, g, e); };
     switch (stage) {
-        case 0: rk_stage_kernel<F, 0><<<grid, block, 0, st>>>(in, out, zf, g, e); break;
-        case 1: rk_stage_kernel<F, 1><<<grid, block, 0, st>>>(in, out, zf, g, e); break;
-        default: rk_stage_kernel<F, 2><<<grid, block, 0, st>>>(in, out, zf, g, e); break;
+        case 0: return launch(rk_stage_kernel<F, 0>);
+        case 1: return launch(rk_stage_kernel<F, 1>);
+        default: return launch(rk_stage_kernel<F, 2>);
     }
-    return cudaGetLastError();
 }
 
 // D_mu of every site as full 3x3 matrices (18 doubles per site, site order):
@@ -147,6 +148,9 @@ cudaError_t launch_rk_stage_halo(int prec, int stage, const void* uin, void* uou
                                  void* lower_out, int lower_v, int lower_t, void* upper_out, int upper_v,
                                  cudaStream_t st) {
     if (g.site0 <= 0 || g.site0 % 32 || (g.site1 - g.site0) % g.site0) return cudaErrorInvalidValue;
+    if (small_lattice(g))
+        return launch_small_stage_halo(prec, stage, uin, uout, z, g, eps, lower_out, lower_v, lower_t, upper_out,
+                                       upper_v, st);
     switch (prec) {
         case kFP64:
             return launch_halo_typed<FieldD18>(stage, uin, uout, z, g, eps, lower_out, lower_v, lower_t, upper_out,
@@ -162,11 +166,12 @@ cudaError_t launch_rk_stage_halo(int prec, int stage, const void* uin, void* uou
 }
 
 cudaError_t launch_rk_stage(int prec, int stage, const void* uin, void* uout, void* z, const Geo& g, double eps,
-                            int block, cudaStream_t st) {
+                            int block, cudaStream_t st, bool chained) {
+    if (small_lattice(g)) return launch_small_stage(prec, stage, uin, uout, z, g, eps, chained, st);
     switch (prec) {
-        case kFP64: return launch_typed<FieldD18>(stage, uin, uout, z, g, eps, block, st);
-        case kFP32_18: return launch_typed<FieldF18>(stage, uin, uout, z, g, eps, block, st);
-        case kFP32_12: return launch_typed<FieldF12>(stage, uin, uout, z, g, eps, block, st);
+        case kFP64: return launch_typed<FieldD18>(stage, uin, uout, z, g, eps, block, chained, st);
+        case kFP32_18: return launch_typed<FieldF18>(stage, uin, uout, z, g, eps, block, chained, st);
+        case kFP32_12: return launch_typed<FieldF12>(stage, uin, uout, z, g, eps, block, chained, st);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -35,7 +35,7 @@ struct StageMinBlocks {
 // the traceless anti-Hermitian part needs are computed.  mu is warp-uniform and the nu loop is kept rolled: one copy of
 // the staple code serves every direction, which keeps the kernel inside the
 // instruction cache.
-template <class F>
+template <bool RO = true, class F>
 __device__ __forceinline__ Herm8<typename F::Real> link_force(const F& in, const Geo& g, int s, const int c[4],
                                                               int mu, M3<typename F::Real>& u) {
     using R = typename F::Real;
@@ -54,22 +54,22 @@ __device__ __forceinline__ Herm8<typename F::Real> link_force(const F& in, const
             {  // upper staple U_nu(x+mu) U_mu(x+nu)^+ U_nu(x)^+
                 Rows2<R> t, st;
                 {
-                    const Rows2<R> a = in.load_rows2(nu, s_pm);
-                    const M3<R> b = in.load(mu, s_pn);
+                    const Rows2<R> a = in.template load_rows2<RO>(nu, s_pm);
+                    const M3<R> b = in.template load<RO>(mu, s_pn);
                     mmul_rows2<false, true>(a, b, t);
                 }
-                const M3<R> d = in.load(nu, s);
+                const M3<R> d = in.template load<RO>(nu, s);
                 mmul_rows2<false, true>(t, d, st);
                 madd_su3_rows2(omega, st);
             }
             {  // lower staple U_nu(x+mu-nu)^+ U_mu(x-nu)^+ U_nu(x-nu)
                 Rows2<R> t, st;
                 {
-                    const M3<R> a = in.load(nu, s_pm_mn);
-                    const M3<R> b = in.load(mu, s_mn);
+                    const M3<R> a = in.template load<RO>(nu, s_pm_mn);
+                    const M3<R> b = in.template load<RO>(mu, s_mn);
                     mmul_rows2<true, true>(a, b, t);
                 }
-                const M3<R> d = in.load(nu, s_mn);
+                const M3<R> d = in.template load<RO>(nu, s_mn);
                 mmul_rows2<false, false>(t, d, st);
                 madd_su3_rows2(omega, st);
             }
@@ -77,26 +77,26 @@ __device__ __forceinline__ Herm8<typename F::Real> link_force(const F& in, const
             {  // upper staple, all three rows
                 M3<R> t;
                 {
-                    const M3<R> a = in.load(nu, s_pm);
-                    const M3<R> b = in.load(mu, s_pn);
+                    const M3<R> a = in.template load<RO>(nu, s_pm);
+                    const M3<R> b = in.template load<RO>(mu, s_pn);
                     mmul<false, true>(a, b, t);
                 }
-                const M3<R> d = in.load(nu, s);
+                const M3<R> d = in.template load<RO>(nu, s);
                 mmul_acc<false, true>(t, d, omega);
             }
             {  // lower staple, all three rows
                 M3<R> t;
                 {
-                    const M3<R> a = in.load(nu, s_pm_mn);
-                    const M3<R> b = in.load(mu, s_mn);
+                    const M3<R> a = in.template load<RO>(nu, s_pm_mn);
+                    const M3<R> b = in.template load<RO>(mu, s_mn);
                     mmul<true, true>(a, b, t);
                 }
-                const M3<R> d = in.load(nu, s_mn);
+                const M3<R> d = in.template load<RO>(nu, s_mn);
                 mmul_acc<false, false>(t, d, omega);
             }
         }
     }
-    u = in.load(mu, s);
+    u = in.template load<RO>(mu, s);
     return force_from_u_omega(u, omega);
 }
 
@@ -119,21 +119,24 @@ struct HaloTargets {
 // The rest of a link's stage once its generator dz = D_mu(x) is known: the RK
 // combination with the stored generator, e^{i eps_s Z} and the new link
 // e^{i eps_s Z} U stored into `out` (returned for the halo stores).
+// prev: the stored generator (stages 1 and 2).
 template <class F, int STAGE, class FO = F>
-__device__ __forceinline__ Rows2<typename F::Real> rk_finish(const FO& out, const ForceField<typename F::Real>& zf,
-                                                            typename F::Real eps, int s, int mu,
-                                                            const Herm8<typename F::Real>& dz,
-                                                            const M3<typename F::Real>& u) {
+__device__ __forceinline__ Rows2<typename F::Real> rk_finish_from(const FO& out,
+                                                                 const ForceField<typename F::Real>& zf,
+                                                                 typename F::Real eps, int s, int mu,
+                                                                 const Herm8<typename F::Real>& dz,
+                                                                 const M3<typename F::Real>& u,
+                                                                 const Herm8<typename F::Real>& prev) {
     using R = typename F::Real;
     Herm8<R> z;
     if (STAGE == 0) {
         z = dz;
         zf.store(mu, s, z);
     } else if (STAGE == 1) {
-        z = h8_axpby(R(8.0 / 9.0), dz, R(17.0 / 36.0), zf.load(mu, s));
+        z = h8_axpby(R(8.0 / 9.0), dz, R(17.0 / 36.0), prev);
         zf.store(mu, s, z);
     } else {
-        z = h8_axpby(R(3.0 / 4.0), dz, R(1.0), zf.load(mu, s));
+        z = h8_axpby(R(3.0 / 4.0), dz, R(1.0), prev);
     }
     const Herm8<R> q = h8_scale(eps, z);
     Rows2<R> d, un;
@@ -146,11 +149,22 @@ __device__ __forceinline__ Rows2<typename F::Real> rk_finish(const FO& out, cons
             un.e[i][j].re += u.e[i][j].re;
             un.e[i][j].im += u.e[i][j].im;
         }
+    grid_release();
     out.store_rows2(mu, s, un);
     return un;
 }
 
-template <class F, int STAGE, bool HALO>
+template <class F, int STAGE, class FO = F>
+__device__ __forceinline__ Rows2<typename F::Real> rk_finish(const FO& out, const ForceField<typename F::Real>& zf,
+                                                            typename F::Real eps, int s, int mu,
+                                                            const Herm8<typename F::Real>& dz,
+                                                            const M3<typename F::Real>& u) {
+    Herm8<typename F::Real> prev = {};
+    if (STAGE != 0) prev = zf.load(mu, s);
+    return rk_finish_from<F, STAGE>(out, zf, eps, s, mu, dz, u, prev);
+}
+
+template <class F, int STAGE, bool HALO, bool RO = true>
 __device__ __forceinline__ void rk_link_update_to(const F& in, const F& out, const ForceField<typename F::Real>& zf,
                                                   const Geo& g, typename F::Real eps, int s, int mu,
                                                   const HaloTargets<F>& h) {
@@ -158,7 +172,7 @@ __device__ __forceinline__ void rk_link_update_to(const F& in, const F& out, con
     int c[4];
     g.coords(s, c);
     M3<R> u;
-    const Herm8<R> dz = link_force(in, g, s, c, mu, u);
+    const Herm8<R> dz = link_force<RO>(in, g, s, c, mu, u);
     const Rows2<R> un = rk_finish<F, STAGE>(out, zf, eps, s, mu, dz, u);
     if constexpr (HALO) {
         if (c[3] == 1) h.lower.store_rows2(mu, h.lower_t * h.slice_sites + (s - h.slice_sites), un);
@@ -166,10 +180,10 @@ __device__ __forceinline__ void rk_link_update_to(const F& in, const F& out, con
     }
 }
 
-template <class F, int STAGE>
+template <class F, int STAGE, bool RO = true>
 __device__ __forceinline__ void rk_link_update(const F& in, const F& out, const ForceField<typename F::Real>& zf,
                                                const Geo& g, typename F::Real eps, int s, int mu) {
-    rk_link_update_to<F, STAGE, false>(in, out, zf, g, eps, s, mu, HaloTargets<F>{});
+    rk_link_update_to<F, STAGE, false, RO>(in, out, zf, g, eps, s, mu, HaloTargets<F>{});
 }
 
 // ---------------------------------------------------------------------------
@@ -187,7 +201,7 @@ __device__ __forceinline__ int plane_b(int p) { return p < 3 ? p + 1 : (p < 5 ? 
 
 // H_ab(x) = (i/2)[P_ab(x) - P_ab(x)^+]_TL at site s with coordinates c;
 // trace (optional): Re tr P_ab(x).
-template <class F>
+template <bool RO = true, class F>
 __device__ __forceinline__ Herm8<typename F::Real> plane_generator(const F& u, const Geo& g, int s, const int c[4],
                                                                    int a, int b, typename F::Real* trace = nullptr) {
     using R = typename F::Real;
@@ -206,14 +220,14 @@ __device__ __forceinline__ Herm8<typename F::Real> plane_generator(const F& u, c
     Rows2<R> lo;
     M3<R> up;
     {
-        const Rows2<R> x = u.load_rows2(a, s);
-        const M3<R> y = u.load(b, s_pa);
+        const Rows2<R> x = u.template load_rows2<RO>(a, s);
+        const M3<R> y = u.template load<RO>(b, s_pa);
         mmul_rows2<false, false>(x, y, lo);
     }
     {
         Rows2<R> t;
-        const Rows2<R> x = u.load_rows2(b, s);
-        const M3<R> y = u.load(a, s_pb);
+        const Rows2<R> x = u.template load_rows2<RO>(b, s);
+        const M3<R> y = u.template load<RO>(a, s_pb);
         mmul_rows2<false, false>(x, y, t);
         full_from_rows2(t, up);
     }
@@ -232,7 +246,7 @@ __device__ __forceinline__ void plaq_plane(const F& u, const ForceField<typename
 // One link through one stage with its generator built from the plane field hf
 // (which holds the plane generators of `in`); HALO: a slab's boundary links
 // also go into its neighbours' halos, as in rk_link_update_to.
-template <class F, int STAGE, bool HALO, class FO = F>
+template <class F, int STAGE, bool HALO, class FO = F, bool RO = true>
 __device__ __forceinline__ void split_link_update_to(const F& in, const FO& out,
                                                      const ForceField<typename F::Real>& zf,
                                                      const ForceField<typename F::Real>& hf, const Geo& g,
@@ -254,11 +268,11 @@ __device__ __forceinline__ void split_link_update_to(const F& in, const FO& out,
         const int p = mu < nu ? plane_index(mu, nu) : plane_index(nu, mu);
         const R sg = mu < nu ? R(1) : R(-1);
         const int y = g.hop_rt(s, g.coord(c, nu), nu, -1);
-        const M3<R> v = in.load(nu, y);
-        d = h8_axpy(sg, hf.load_ro(p, s), d);
-        herm_conj_add(v, h8_scale(-sg, hf.load_ro(p, y)), d);
+        const M3<R> v = in.template load<RO>(nu, y);
+        d = h8_axpy(sg, (RO ? hf.load_ro(p, s) : hf.load(p, s)), d);
+        herm_conj_add(v, h8_scale(-sg, (RO ? hf.load_ro(p, y) : hf.load(p, y))), d);
     }
-    const M3<R> uu = in.load(mu, s);
+    const M3<R> uu = in.template load<RO>(mu, s);
     const Rows2<R> un = rk_finish<F, STAGE>(out, zf, eps, s, mu, d, uu);
     if constexpr (HALO) {
         if (c[3] == 1) h.lower.store_rows2(mu, h.lower_t * h.slice_sites + (s - h.slice_sites), un);
@@ -266,11 +280,11 @@ __device__ __forceinline__ void split_link_update_to(const F& in, const FO& out,
     }
 }
 
-template <class F, int STAGE, class FO = F>
+template <class F, int STAGE, class FO = F, bool RO = true>
 __device__ __forceinline__ void split_link_update(const F& in, const FO& out, const ForceField<typename F::Real>& zf,
                                                   const ForceField<typename F::Real>& hf, const Geo& g,
                                                   typename F::Real eps, int s, int mu) {
-    split_link_update_to<F, STAGE, false>(in, out, zf, hf, g, eps, s, mu, HaloTargets<F>{});
+    split_link_update_to<F, STAGE, false, FO, RO>(in, out, zf, hf, g, eps, s, mu, HaloTargets<F>{});
 }
 
 // Resident blocks of the two-kernel stage kernel: FP32 forms at 8 (64

@@ -58,7 +58,10 @@ __global__ void __launch_bounds__(192, PlaqMinBlocks<F>::value) plaq_field_kerne
         const int s = g.site0 + blk * 32 + int(threadIdx.x & 31);
         if (s >= g.site1) return;
         g.coords(s, c);
-        hf.store(w, s, plane_generator(u, g, s, c, plane_a(w), plane_b(w)));
+        grid_wait();
+        const auto h = plane_generator<false>(u, g, s, c, plane_a(w), plane_b(w));
+        grid_release();
+        hf.store(w, s, h);
         return;
     }
     const int s = g.site0 + (blk * 2 + w / 3) * 32 + int(threadIdx.x & 31);
@@ -67,9 +70,11 @@ __global__ void __launch_bounds__(192, PlaqMinBlocks<F>::value) plaq_field_kerne
     const int p0 = pr == 0 ? 0 : (pr == 1 ? 2 : 3);
     const int p1 = pr == 0 ? 1 : (pr == 1 ? 4 : 5);
     g.coords(s, c);
+    grid_wait();
     // both planes before either store: the link the two share is loaded once
-    const auto h0 = plane_generator(u, g, s, c, plane_a(p0), plane_b(p0));
-    const auto h1 = plane_generator(u, g, s, c, plane_a(p1), plane_b(p1));
+    const auto h0 = plane_generator<false>(u, g, s, c, plane_a(p0), plane_b(p0));
+    const auto h1 = plane_generator<false>(u, g, s, c, plane_a(p1), plane_b(p1));
+    grid_release();
     hf.store(p0, s, h0);
     hf.store(p1, s, h1);
 }
@@ -81,8 +86,9 @@ __global__ void __launch_bounds__(128, SplitMinBlocks<F>::value)
                           typename F::Real eps) {
     const int mu = int(threadIdx.x >> 5) & 3;
     const int s = g.site0 + int(blockIdx.x) * 32 + int(threadIdx.x & 31);
+    grid_wait();
     if (s >= g.site1) return;
-    split_link_update<F, STAGE>(in, out, zf, hf, g, eps, s, mu);
+    split_link_update<F, STAGE, FO, false>(in, out, zf, hf, g, eps, s, mu);
 }
 
 // The same for a time slab, storing its boundary links into its neighbours'
@@ -116,29 +122,29 @@ static cudaError_t launch_split_halo_typed(int stage, const void* uin, void* uou
 }
 
 template <class F>
-static cudaError_t launch_plaq_typed(const void* u, void* h, const Geo& g, cudaStream_t st) {
+static cudaError_t launch_plaq_typed(const void* u, void* h, const Geo& g, bool chained, cudaStream_t st) {
     F in{const_cast<void*>(u), g.V};
     ForceField<typename F::Real> hf{h, g.V};
     const unsigned groups = unsigned((g.site1 - g.site0 + 31) / 32);
-    plaq_field_kernel<F><<<PlaqPlanesPerThread<F>::value == 1 ? groups : (groups + 1) / 2, 192, 0, st>>>(in, hf, g);
-    return cudaGetLastError();
+    return launch_chained(chained, plaq_field_kernel<F>, PlaqPlanesPerThread<F>::value == 1 ? groups : (groups + 1) / 2,
+                          192, st, in, hf, g);
 }
 
 template <class F, class FO = F>
 static cudaError_t launch_split_typed(int stage, const void* uin, void* uout, void* z, const void* h, const Geo& g,
-                                      double eps, cudaStream_t st) {
+                                      double eps, bool chained, cudaStream_t st) {
     using R = typename F::Real;
     const F in{const_cast<void*>(uin), g.V};
     const FO out{uout, g.V};
     ForceField<R> zf{z, g.V}, hf{const_cast<void*>(h), g.V};
-    const dim3 grid(unsigned((g.site1 - g.site0 + 31) / 32));
+    const unsigned grid = unsigned((g.site1 - g.site0 + 31) / 32);
     const R e = R(stage == 0 ? eps * 0.25 : eps);
+    auto launch = [&](auto kernel) { return launch_chained(chained, kernel, grid, 128, st, in, out, zf, hf, g, e); };
     switch (stage) {
-        case 0: rk_split_stage_kernel<F, 0, FO><<<grid, 128, 0, st>>>(in, out, zf, hf, g, e); break;
-        case 1: rk_split_stage_kernel<F, 1, FO><<<grid, 128, 0, st>>>(in, out, zf, hf, g, e); break;
-        default: rk_split_stage_kernel<F, 2, FO><<<grid, 128, 0, st>>>(in, out, zf, hf, g, e); break;
+        case 0: return launch(rk_split_stage_kernel<F, 0, FO>);
+        case 1: return launch(rk_split_stage_kernel<F, 1, FO>);
+        default: return launch(rk_split_stage_kernel<F, 2, FO>);
     }
-    return cudaGetLastError();
 }
 
 // The plaquette-field kernel of a measurement: the same field, and the sum of
@@ -157,18 +163,19 @@ __global__ void __launch_bounds__(192, sizeof(typename F::Real) == 8 ? 3 : PlaqM
     const int s = g.site0 + (int(blockIdx.x) * kPlanes + (kPlanes == 1 ? 0 : w / 3)) * 32 + int(threadIdx.x & 31);
     R t0 = R(0), t1 = R(0);
     bool counts = false;
+    grid_wait();
     if (s < g.site1) {
         int c[4];
         g.coords(s, c);
         counts = s >= count0 && s < count1 && g.interior(c);
         if (kPlanes == 1) {
-            hf.store(w, s, plane_generator(u, g, s, c, plane_a(w), plane_b(w), &t0));
+            hf.store(w, s, plane_generator<false>(u, g, s, c, plane_a(w), plane_b(w), &t0));
         } else {
             const int pr = w % 3;
             const int p0 = pr == 0 ? 0 : (pr == 1 ? 2 : 3);
             const int p1 = pr == 0 ? 1 : (pr == 1 ? 4 : 5);
-            const auto h0 = plane_generator(u, g, s, c, plane_a(p0), plane_b(p0), &t0);
-            const auto h1 = plane_generator(u, g, s, c, plane_a(p1), plane_b(p1), &t1);
+            const auto h0 = plane_generator<false>(u, g, s, c, plane_a(p0), plane_b(p0), &t0);
+            const auto h1 = plane_generator<false>(u, g, s, c, plane_a(p1), plane_b(p1), &t1);
             hf.store(p0, s, h0);
             hf.store(p1, s, h1);
         }
@@ -186,33 +193,34 @@ int plaq_sum_partials(int prec, const Geo& g) { return 6 * plaq_blocks(prec, g);
 
 template <class F>
 static cudaError_t launch_plaq_sum_typed(const void* u, void* h, const Geo& g, int count0, int count1,
-                                         double* partials, cudaStream_t st) {
+                                         double* partials, bool chained, cudaStream_t st) {
     F in{const_cast<void*>(u), g.V};
     ForceField<typename F::Real> hf{h, g.V};
-    plaq_field_sum_kernel<F><<<plaq_blocks(sizeof(typename F::Real) == 8 ? kFP64 : kFP32_18, g), 192, 0, st>>>(in, hf, g, count0, count1, partials);
-    return cudaGetLastError();
+    return launch_chained(chained, plaq_field_sum_kernel<F>, unsigned(plaq_blocks(sizeof(typename F::Real) == 8 ? kFP64 : kFP32_18, g)), 192, st, in, hf, g, count0, count1, partials);
 }
 
 cudaError_t launch_plaq_field_sum(int prec, const void* u, void* h, const Geo& g, int count0, int count1,
-                                  double* partials, cudaStream_t st, bool rows_in) {
+                                  double* partials, cudaStream_t st, bool rows_in, bool chained) {
     if (g.site1 <= g.site0) return cudaErrorInvalidValue;
     switch (prec) {
         case kFP64:
-            if (rows_in) return launch_plaq_sum_typed<FieldD18Rows>(u, h, g, count0, count1, partials, st);
-            return launch_plaq_sum_typed<FieldD18>(u, h, g, count0, count1, partials, st);
-        case kFP32_18: return launch_plaq_sum_typed<FieldF18>(u, h, g, count0, count1, partials, st);
-        case kFP32_12: return launch_plaq_sum_typed<FieldF12>(u, h, g, count0, count1, partials, st);
+            if (rows_in) return launch_plaq_sum_typed<FieldD18Rows>(u, h, g, count0, count1, partials, chained, st);
+            return launch_plaq_sum_typed<FieldD18>(u, h, g, count0, count1, partials, chained, st);
+        case kFP32_18: return launch_plaq_sum_typed<FieldF18>(u, h, g, count0, count1, partials, chained, st);
+        case kFP32_12: return launch_plaq_sum_typed<FieldF12>(u, h, g, count0, count1, partials, chained, st);
         default: return cudaErrorInvalidValue;
     }
 }
 
-cudaError_t launch_plaq_field(int prec, const void* u, void* h, const Geo& g, cudaStream_t st, bool rows_in) {
+cudaError_t launch_plaq_field(int prec, const void* u, void* h, const Geo& g, cudaStream_t st, bool rows_in,
+                              bool chained) {
+    if (small_lattice(g)) return cudaSuccess;  // its stage kernel forms its own plaquettes
     switch (prec) {
         case kFP64:
-            if (rows_in) return launch_plaq_typed<FieldD18Rows>(u, h, g, st);
-            return launch_plaq_typed<FieldD18>(u, h, g, st);
-        case kFP32_18: return launch_plaq_typed<FieldF18>(u, h, g, st);
-        case kFP32_12: return launch_plaq_typed<FieldF12>(u, h, g, st);
+            if (rows_in) return launch_plaq_typed<FieldD18Rows>(u, h, g, chained, st);
+            return launch_plaq_typed<FieldD18>(u, h, g, chained, st);
+        case kFP32_18: return launch_plaq_typed<FieldF18>(u, h, g, chained, st);
+        case kFP32_12: return launch_plaq_typed<FieldF12>(u, h, g, chained, st);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -221,6 +229,9 @@ cudaError_t launch_rk_split_stage_halo(int prec, int stage, const void* uin, voi
                                        const Geo& g, double eps, void* lower_out, int lower_v, int lower_t,
                                        void* upper_out, int upper_v, cudaStream_t st) {
     if (g.site0 <= 0 || g.site0 % 32 || (g.site1 - g.site0) % g.site0) return cudaErrorInvalidValue;
+    if (small_lattice(g))
+        return launch_small_stage_halo(prec, stage, uin, uout, z, g, eps, lower_out, lower_v, lower_t, upper_out,
+                                       upper_v, st);
     switch (prec) {
         case kFP64:
             return launch_split_halo_typed<FieldD18>(stage, uin, uout, z, h, g, eps, lower_out, lower_v, lower_t,
@@ -236,15 +247,16 @@ cudaError_t launch_rk_split_stage_halo(int prec, int stage, const void* uin, voi
 }
 
 cudaError_t launch_rk_split_stage(int prec, int stage, const void* uin, void* uout, void* z, const void* h,
-                                  const Geo& g, double eps, cudaStream_t st, bool rows_in, bool rows_out) {
+                                  const Geo& g, double eps, cudaStream_t st, bool rows_in, bool rows_out, bool chained) {
+    if (small_lattice(g)) return launch_small_stage(prec, stage, uin, uout, z, g, eps, chained, st);
     switch (prec) {
         case kFP64:
-            if (rows_in && rows_out) return launch_split_typed<FieldD18Rows>(stage, uin, uout, z, h, g, eps, st);
-            if (rows_in) return launch_split_typed<FieldD18Rows, FieldD18>(stage, uin, uout, z, h, g, eps, st);
-            if (rows_out) return launch_split_typed<FieldD18, FieldD18Rows>(stage, uin, uout, z, h, g, eps, st);
-            return launch_split_typed<FieldD18>(stage, uin, uout, z, h, g, eps, st);
-        case kFP32_18: return launch_split_typed<FieldF18>(stage, uin, uout, z, h, g, eps, st);
-        case kFP32_12: return launch_split_typed<FieldF12>(stage, uin, uout, z, h, g, eps, st);
+            if (rows_in && rows_out) return launch_split_typed<FieldD18Rows>(stage, uin, uout, z, h, g, eps, chained, st);
+            if (rows_in) return launch_split_typed<FieldD18Rows, FieldD18>(stage, uin, uout, z, h, g, eps, chained, st);
+            if (rows_out) return launch_split_typed<FieldD18, FieldD18Rows>(stage, uin, uout, z, h, g, eps, chained, st);
+            return launch_split_typed<FieldD18>(stage, uin, uout, z, h, g, eps, chained, st);
+        case kFP32_18: return launch_split_typed<FieldF18>(stage, uin, uout, z, h, g, eps, chained, st);
+        case kFP32_12: return launch_split_typed<FieldF12>(stage, uin, uout, z, h, g, eps, chained, st);
         default: return cudaErrorInvalidValue;
     }
 }

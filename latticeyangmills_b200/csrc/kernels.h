@@ -23,20 +23,60 @@ inline size_t plane_field_bytes(int prec, int64_t V) { return size_t(6 * padded_
 // whether field.cuh's 32-bit offsets (16-byte units) reach every link of V sites
 inline bool volume_addressable(int prec, int64_t V) { return link_field_bytes(prec, V) / 16 < (size_t(1) << 32); }
 
+// Launches `kernel` so that it may start while the kernel before it on the
+// stream drains (programmatic dependent launch): its blocks are placed as the
+// other's finish (grid_release) and its index arithmetic runs; it waits
+// (grid_wait) for the other's end before it reads or writes anything.
+// chained = false: an ordinary launch.
+template <class... P, class... A>
+cudaError_t launch_chained(bool chained, void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t st,
+                           A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = st;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
+// Small configurations (flow_small.cu): every stage form and the observables
+// run one kernel each whose threads take one plaquette loop, instead of the
+// kernels below.  By the whole configuration's volume, so that its slabs and
+// blocks take the same.  The line is one block per SM (148 x 32 sites): past it
+// a second wave of the wide blocks costs more than the launches saved, 8^3 x 12
+// on B200 27.7 against 20.8 us per step (FP64), 20.5 against 16.3 (FP32-12).
+constexpr int kSmallSites = 148 * 32;
+inline bool small_lattice(const Geo& g) { return g.vglobal <= kSmallSites; }
+cudaError_t launch_small_stage(int prec, int stage, const void* uin, void* uout, void* z, const Geo& g, double eps,
+                               bool chained, cudaStream_t st);
+cudaError_t launch_small_stage_halo(int prec, int stage, const void* uin, void* uout, void* z, const Geo& g, double eps,
+                                    void* lower_out, int lower_v, int lower_t, void* upper_out, int upper_v,
+                                    cudaStream_t st);
+// `partials`: small_partials(g) doubles, zero before the first call (the last is
+// the launch's count of finished blocks, which it leaves zero).
+inline int small_partials(const Geo& g) { return 3 * ((g.site1 - g.site0 + 31) / 32) + 1; }
+cudaError_t launch_small_observables(int prec, const void* u, const Geo& g, double* partials, double* out,
+                                     bool chained, cudaStream_t st);
+
 // One RK3 stage (0, 1, 2) over every link: staples, generator, RK combination
 // with the stored generator, e^{i eps_stage Z} and the link update uin -> uout.
 cudaError_t launch_rk_stage(int prec, int stage, const void* uin, void* uout, void* z, const Geo& g, double eps,
-                            int block, cudaStream_t st);
+                            int block, cudaStream_t st, bool chained = false);
 
 // The same stage as two kernels (flow_split.cu): the six plaquettes' generators
 // of every site of u into h (plane_field_bytes), then the stage with each
 // link's force built from h (h must hold uin's plaquette field).  rows_in (FP64):
 // read rows 0 and 1 of u's links only (u was written by a stage); rows_out:
 // store rows 0 and 1 only (uout is read with rows_in alone).
-cudaError_t launch_plaq_field(int prec, const void* u, void* h, const Geo& g, cudaStream_t st, bool rows_in = false);
+cudaError_t launch_plaq_field(int prec, const void* u, void* h, const Geo& g, cudaStream_t st, bool rows_in = false,
+                              bool chained = false);
 cudaError_t launch_rk_split_stage(int prec, int stage, const void* uin, void* uout, void* z, const void* h,
                                   const Geo& g, double eps, cudaStream_t st, bool rows_in = false,
-                                  bool rows_out = false);
+                                  bool rows_out = false, bool chained = false);
 // Its slab form with the halo stores of launch_rk_stage_halo (h must hold the
 // plane generators of local slices 0..nt, see plaq_range).
 cudaError_t launch_rk_split_stage_halo(int prec, int stage, const void* uin, void* uout, void* z, const void* h,
@@ -99,7 +139,8 @@ cudaError_t launch_exp(const double* q, double* r, int64_t n, cudaStream_t st);
 // value is not finite.
 int obs_blocks(const Geo& g);
 cudaError_t launch_observables(int prec, const void* u, const Geo& g, double* partials, cudaStream_t st);
-cudaError_t launch_obs_finalize(const double* partials, int nblocks, const Geo& g, double* out, cudaStream_t st);
+cudaError_t launch_obs_finalize(const double* partials, int nblocks, const Geo& g, double* out, cudaStream_t st,
+                                bool chained = false);
 
 // The same row (out[0..3]) through the plaquette field, in three launches: the
 // field of u over `field`'s sites into h (which then holds u's plaquette field,
@@ -110,10 +151,11 @@ cudaError_t launch_obs_finalize(const double* partials, int nblocks, const Geo& 
 constexpr int kCloverMaxBlocks = 148 * 20;
 int plaq_sum_partials(int prec, const Geo& g);
 cudaError_t launch_plaq_field_sum(int prec, const void* u, void* h, const Geo& g, int count0, int count1,
-                                  double* partials, cudaStream_t st, bool rows_in = false);
+                                  double* partials, cudaStream_t st, bool rows_in = false, bool chained = false);
 int measure_partials(int prec, const Geo& field, const Geo& own);
 cudaError_t launch_measure_from_field(int prec, const void* u, void* h, const Geo& field, const Geo& own,
-                                      double* partials, double* out, cudaStream_t st, bool rows_in = false);
+                                      double* partials, double* out, cudaStream_t st, bool rows_in = false,
+                                      bool chained = false);
 
 // .bin layout (site-major, mu, 18 doubles) <-> device layout
 // Sites [first, first + n) between a .bin-layout block (aos points at site

@@ -29,6 +29,7 @@ namespace ym {
 // then the block tree.  Output (plaq, topc, energy, nonfinite flag).
 __global__ void __launch_bounds__(1024) obs_finalize_kernel(const double* partials, int nblocks, double inv_18v,
                                                             double* out) {
+    grid_wait();
     double a = 0.0, b = 0.0, c = 0.0;
 #pragma unroll 4
     for (int i = threadIdx.x; i < nblocks; i += blockDim.x) {
@@ -37,14 +38,7 @@ __global__ void __launch_bounds__(1024) obs_finalize_kernel(const double* partia
         c += partials[3 * i + 2];
     }
     block_sum3(a, b, c);
-    if (threadIdx.x == 0) {
-        const double plaq = a * inv_18v;
-        const double topc = c / (256.0 * 3.14159265358979323846 * 3.14159265358979323846);
-        out[0] = plaq;
-        out[1] = topc;
-        out[2] = b;
-        out[3] = (isfinite(plaq) && isfinite(topc) && isfinite(b)) ? 0.0 : 1.0;
-    }
+    if (threadIdx.x == 0) write_row(a, b, c, inv_18v, out);
 }
 
 int obs_blocks(const Geo& g) {
@@ -70,9 +64,10 @@ cudaError_t launch_observables(int prec, const void* u, const Geo& g, double* pa
     return cudaGetLastError();
 }
 
-cudaError_t launch_obs_finalize(const double* partials, int nblocks, const Geo& g, double* out, cudaStream_t st) {
-    obs_finalize_kernel<<<1, 1024, 0, st>>>(partials, nblocks, 1.0 / (18.0 * double(g.vglobal)), out);
-    return cudaGetLastError();
+cudaError_t launch_obs_finalize(const double* partials, int nblocks, const Geo& g, double* out, cudaStream_t st,
+                                bool chained) {
+    return launch_chained(chained, obs_finalize_kernel, 1, 1024, st, partials, nblocks,
+                          1.0 / (18.0 * double(g.vglobal)), out);
 }
 
 template <class F>
@@ -96,10 +91,10 @@ int measure_partials(int prec, const Geo& field, const Geo& own) {
 // 48 0.55 -> 0.39 ms; below, both are a few launches long (8^4 FP64: 9.3 + 2.9
 // us against 4.9 + 6.7 + 2.9, of which the next step saves the first).
 cudaError_t launch_measure_from_field(int prec, const void* u, void* h, const Geo& field, const Geo& own,
-                                      double* partials, double* out, cudaStream_t st, bool rows_in) {
+                                      double* partials, double* out, cudaStream_t st, bool rows_in, bool chained) {
     const int np = plaq_sum_partials(prec, field), nc = clover_blocks(own);
     if (np < 1 || nc < 1) return cudaErrorInvalidValue;
-    cudaError_t e = launch_plaq_field_sum(prec, u, h, field, own.site0, own.site1, partials, st, rows_in);
+    cudaError_t e = launch_plaq_field_sum(prec, u, h, field, own.site0, own.site1, partials, st, rows_in, chained);
     if (e != cudaSuccess) return e;
     double* const cp = partials + np;
     switch (prec) {
@@ -112,7 +107,7 @@ cudaError_t launch_measure_from_field(int prec, const void* u, void* h, const Ge
         default: return cudaErrorInvalidValue;
     }
     if (e != cudaSuccess) return e;
-    return launch_obs_finalize(cp, nc, own, out, st);
+    return launch_obs_finalize(cp, nc, own, out, st, chained);
 }
 
 }  // namespace ym

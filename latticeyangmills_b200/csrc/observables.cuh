@@ -140,6 +140,18 @@ __device__ __forceinline__ void block_sum3(double& a, double& b, double& c) {
     }
 }
 
+// A measurement row from its sums: (plaq, topc, energy, nonfinite flag) with
+// the reference's normalisations.
+__device__ __forceinline__ void write_row(double plaq_sum, double energy, double topc_sum, double inv_18v,
+                                          double* out) {
+    const double plaq = plaq_sum * inv_18v;
+    const double topc = topc_sum / (256.0 * 3.14159265358979323846 * 3.14159265358979323846);
+    out[0] = plaq;
+    out[1] = topc;
+    out[2] = energy;
+    out[3] = (isfinite(plaq) && isfinite(topc) && isfinite(energy)) ? 0.0 : 1.0;
+}
+
 // One thread per site, the three plane pairs in a loop; block partials, one
 // per block of sites (the allocation-free entry point's form, whose scratch
 // is sized by it).

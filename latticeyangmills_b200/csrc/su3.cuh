@@ -463,4 +463,15 @@ __device__ __forceinline__ Herm8<R> h8_axpy(R a, const Herm8<R>& x, const Herm8<
     return r;
 }
 
+template <class R>
+__device__ __forceinline__ Herm8<R> h8_neg(const Herm8<R>& x) {
+    Herm8<R> r;
+    r.d0 = -x.d0;
+    r.d1 = -x.d1;
+    r.z01 = cx(-x.z01.re, -x.z01.im);
+    r.z02 = cx(-x.z02.re, -x.z02.im);
+    r.z12 = cx(-x.z12.re, -x.z12.im);
+    return r;
+}
+
 }  // namespace ym

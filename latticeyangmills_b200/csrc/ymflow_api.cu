@@ -65,10 +65,12 @@ int ensure_staging(ymflow_ctx* c, size_t bytes = 0) {
 }
 
 // Whether a measurement goes through the plaquette field: where the stages do.
-bool measures_from_field(const ymflow_ctx* c) { return c->stage_form == 1 && c->hfield; }
+bool measures_from_field(const ymflow_ctx* c) {
+    return c->stage_form == 1 && c->hfield && !small_lattice(c->geo);
+}
 
 int ensure_partials(ymflow_ctx* c) {
-    int n = 3 * obs_blocks(c->geo);
+    int n = small_lattice(c->geo) ? small_partials(c->geo) : 3 * obs_blocks(c->geo);
     if (measures_from_field(c)) n = std::max(n, measure_partials(c->prec, plaq_range(c->geo, c->slab), c->geo));
     if (n <= c->partial_cap) return YMFLOW_OK;
     if (c->partials) {
@@ -78,7 +80,9 @@ int ensure_partials(ymflow_ctx* c) {
         c->partial_cap = 0;
     }
     int r = dev_alloc(c, (void**)&c->partials, size_t(n) * sizeof(double), "observable partials");
-    if (r == YMFLOW_OK) c->partial_cap = n;
+    if (r != YMFLOW_OK) return r;
+    YM_CK(c, cudaMemsetAsync(c->partials, 0, size_t(n) * sizeof(double), c->stream), "clear partials");
+    c->partial_cap = n;
     return r;
 }
 
@@ -162,7 +166,7 @@ void drop_graphs(ymflow_ctx* c) {
 // Whether the steps of a call pass links on as their rows 0 and 1: whole
 // lattices on the two-kernel FP64 stage.
 bool steps_by_rows(const ymflow_ctx* c) {
-    return c->prec == YMFLOW_FP64 && c->stage_form == 1 && !c->slab && !c->is_block;
+    return c->prec == YMFLOW_FP64 && c->stage_form == 1 && !c->slab && !c->is_block && !small_lattice(c->geo);
 }
 
 constexpr int kRowsIn = 1, kRowsOut = 2;
@@ -186,17 +190,17 @@ cudaError_t enqueue_step(ymflow_ctx* c, int from, double eps, cudaEvent_t* ev, b
         if (c->stage_form == 1) {
             const bool rows_in = s > 0 || (rows & kRowsIn), rows_out = s < 2 || (rows & kRowsOut);
             if (s > 0 || !field_ready)
-                e = launch_plaq_field(c->prec, in[s], c->hfield, c->geo, c->stream, rows_in);
+                e = launch_plaq_field(c->prec, in[s], c->hfield, c->geo, c->stream, rows_in, true);
             if (e != cudaSuccess) return e;
             if (ev) cudaEventRecord(ev[3 * s + 1], c->stream);
             e = launch_rk_split_stage(c->prec, s, in[s], out[s], c->z, c->hfield, c->geo, eps, c->stream, rows_in,
-                                      rows_out);
+                                      rows_out, true);
         } else if (c->stage_form == 2) {
             if (ev) cudaEventRecord(ev[3 * s + 1], c->stream);
             e = launch_rk_tile_stage(c->prec, s, in[s], out[s], c->z, c->geo, c->tile, eps, c->stream);
         } else {
             if (ev) cudaEventRecord(ev[3 * s + 1], c->stream);
-            e = launch_rk_stage(c->prec, s, in[s], out[s], c->z, c->geo, eps, c->block, c->stream);
+            e = launch_rk_stage(c->prec, s, in[s], out[s], c->z, c->geo, eps, c->block, c->stream, true);
         }
         if (e != cudaSuccess) return e;
         if (ev) cudaEventRecord(ev[3 * s + 2], c->stream);
@@ -236,35 +240,39 @@ int run_step_slab(ymflow_ctx* c, double eps, cudaEvent_t* ev, bool field_ready) 
 // One RK3 step of the current field, step `s` of the `nsteps` (from 1) of a
 // call.  field_ready: the plaquette field holds the current links' (a
 // measurement has just been enqueued, and nothing has changed the links
-// since).  The steps that repeat are replayed as graphs; an FP64 call's first
-// and last, which read or leave whole links, are launched as they are.
+// since).  Forms 0 and 1 launch their kernels chained (launch_chained), which
+// is faster than a replayed graph at every size, most of all between a step and
+// a measurement: us per step / per measured step on B200, graphs of unchained
+// launches against chained launches of the same kernels, 12^4 FP64 41.9 / 60
+// against 38.1 / 52, 16^4 FP32-12 57.5 / 78 against 53.9 / 71, 16^3 x 32
+// FP32-12 102.9 / 133 against 97.5 / 124 (graphs of chained launches lie
+// between); and a context's first steps build no graph.  The tile form's one
+// kernel per stage is replayed.
 int run_step(ymflow_ctx* c, double eps, int s, int nsteps, cudaEvent_t* ev, bool field_ready = false) {
     if (c->slab) return run_step_slab(c, eps, ev, field_ready);
     const int from = c->cur;
-    const bool by_rows = steps_by_rows(c);
-    const int rows = by_rows ? (s > 1 ? kRowsIn : 0) | (s < nsteps ? kRowsOut : 0) : 0;
-    if (c->use_graph && !ev && (!by_rows || rows == (kRowsIn | kRowsOut))) {
-        const int k = from + (field_ready ? 2 : 0);
-        if (!c->graph[k] || c->graph_eps[k] != eps || c->graph_block[k] != c->block) {
-            if (c->graph[k]) cudaGraphExecDestroy(c->graph[k]);
-            c->graph[k] = nullptr;
+    if (c->use_graph && c->stage_form == 2 && !ev) {
+        if (!c->graph[from] || c->graph_eps[from] != eps || c->graph_block[from] != c->block) {
+            if (c->graph[from]) cudaGraphExecDestroy(c->graph[from]);
+            c->graph[from] = nullptr;
             cudaGraph_t g = nullptr;
             YM_CK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal), "begin step capture");
-            cudaError_t le = enqueue_step(c, from, eps, nullptr, field_ready, rows);
+            cudaError_t le = enqueue_step(c, from, eps, nullptr, false, 0);
             cudaError_t ee = cudaStreamEndCapture(c->stream, &g);
             if (le != cudaSuccess) {
                 if (g) cudaGraphDestroy(g);
                 return cuda_fail(c, le, "stage launch during capture");
             }
             YM_CK(c, ee, "end step capture");
-            cudaError_t ie = cudaGraphInstantiate(&c->graph[k], g, 0);
+            cudaError_t ie = cudaGraphInstantiate(&c->graph[from], g, 0);
             cudaGraphDestroy(g);
             YM_CK(c, ie, "instantiate step graph");
-            c->graph_eps[k] = eps;
-            c->graph_block[k] = c->block;
+            c->graph_eps[from] = eps;
+            c->graph_block[from] = c->block;
         }
-        YM_CK(c, cudaGraphLaunch(c->graph[k], c->stream), "launch step graph");
+        YM_CK(c, cudaGraphLaunch(c->graph[from], c->stream), "launch step graph");
     } else {
+        const int rows = steps_by_rows(c) ? (s > 1 ? kRowsIn : 0) | (s < nsteps ? kRowsOut : 0) : 0;
         YM_CK(c, enqueue_step(c, from, eps, ev, field_ready, rows), "stage launch");
     }
     c->cur = 1 - from;
@@ -289,9 +297,17 @@ cudaError_t enqueue_stage(ymflow_ctx* c, int stage, const void* in, void* out, d
 int enqueue_measure(ymflow_ctx* c, int row, bool rows_in) {
     int r = ensure_partials(c);
     if (r != YMFLOW_OK) return r;
-    if (measures_from_field(c)) {
+    // Kernels of a whole lattice follow one another on its stream alone, so they
+    // may be launched on each other's heels; slabs and blocks also wait for
+    // their neighbours' streams.
+    const bool chained = !c->slab && !c->is_block;
+    if (small_lattice(c->geo)) {
+        YM_CK(c, launch_small_observables(c->prec, c->u[c->cur], c->geo, c->partials, c->meas + 4 * row, chained,
+                                          c->stream),
+              "observables launch");
+    } else if (measures_from_field(c)) {
         YM_CK(c, launch_measure_from_field(c->prec, c->u[c->cur], c->hfield, plaq_range(c->geo, c->slab), c->geo,
-                                           c->partials, c->meas + 4 * row, c->stream, rows_in),
+                                           c->partials, c->meas + 4 * row, c->stream, rows_in, chained),
               "observables launch");
     } else {
         YM_CK(c, launch_observables(c->prec, c->u[c->cur], c->geo, c->partials, c->stream), "observables launch");
