@@ -387,8 +387,9 @@ YMFLOW_API int ymflow_ensemble_time_steps(ymflow_ens* ens, double eps, int nstep
  * ensemble in each form it can take and keeps the fastest, cached for every
  * ensemble of the same sizes and precision in the process:
  *   - the per-link kernel (FP64) over persistent grids {one CTA per work
- *     item, 1x and 2x the resident CTAs}, or the two-kernel stage (FP32), one
- *     block per 32-site item;
+ *     item, 1x and 2x the resident CTAs};
+ *   - the two-kernel stage, one block per 32-site item (FP64 ensembles where
+ *     their plane-generator pool fits);
  *   - the two-kernel stage launched once per run of consecutive
  *     configurations with equal extents, each run's geometry a launch
  *     parameter (two launches per run and stage; FP64 ensembles where their
@@ -404,7 +405,8 @@ YMFLOW_API int ymflow_ensemble_time_steps(ymflow_ens* ens, double eps, int nstep
 YMFLOW_API int ymflow_ensemble_autotune(ymflow_ens* ens, double eps, int* block, int* grid);
 /* The ensemble's current stage form (0 per-link kernel, 1 two-kernel stage,
  * 2 tiles in shared memory, 3 two-kernel stage per run of equal extents),
- * block size and grid. */
+ * block size and grid.  An ensemble that was neither tuned nor given a form
+ * settles on 1 or 3 at its first flow where it has a plane-generator pool. */
 YMFLOW_API int ymflow_ensemble_tuning(const ymflow_ens* ens, int* stage_form, int* block, int* grid);
 /* Sets the form by hand: 0 with block 128 and a grid (0: one block per item),
  * 1 or 3 with block 128 (ensembles with a plane-generator pool: every FP32

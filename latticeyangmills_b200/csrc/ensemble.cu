@@ -22,6 +22,7 @@
 
 #include "api_util.h"
 #include "flow_tile.cuh"
+#include "observables.cuh"
 #include "ymflow.h"
 
 namespace ym {
@@ -121,22 +122,69 @@ static cudaError_t launch_ens_typed(int stage, void* uin, void* uout, void* z, c
     return cudaGetLastError();
 }
 
-// The two-kernel stage over the work list (FP32 ensembles): one 192-thread block
-// per 32-site item forms that item's six plane generators, then one 128-thread
-// block per item runs the stage from them.  One block per item, as the flat kernel.
+// The two-kernel stage over the work list: a 192-thread block per 32-site item
+// (FP64, a plane per warp) or per two items (FP32, two planes per warp, as
+// plaq_field_kernel) forms the plane generators, then one 128-thread block per
+// item runs the stage from them.  One block per item, as the flat kernel.
+//
+// The plane generators of this thread's site by warp `w` of its block: FP64
+// plane w; FP32 the pair w % 3 of the block's item w / 3.  TRACE: also this
+// thread's part of the plaquette sum.
 template <class F>
-__global__ void __launch_bounds__(192) ens_plaq_kernel(char* u, char* h, const EnsConf* __restrict__ confs, int nconf) {
-    const int item = blockIdx.x;
+struct EnsItemsPerBlock {
+    static constexpr int value = sizeof(typename F::Real) == 8 ? 1 : 2;
+};
+
+template <bool TRACE, class F>
+__device__ __forceinline__ double item_planes(const F& u, const ForceField<typename F::Real>& hf, const Geo& g, int s,
+                                              int w) {
+    using R = typename F::Real;
+    R t0 = R(0), t1 = R(0);
+    int c[4];
+    g.coords(s, c);
+    if constexpr (EnsItemsPerBlock<F>::value == 1) {
+        const auto h = plane_generator<false>(u, g, s, c, plane_a(w), plane_b(w), TRACE ? &t0 : nullptr);
+        grid_release();
+        hf.store(w, s, h);
+    } else {
+        const int pr = w % 3;
+        const int p0 = pr == 0 ? 0 : (pr == 1 ? 2 : 3);
+        const int p1 = pr == 0 ? 1 : (pr == 1 ? 4 : 5);
+        // both planes before either store: the link the two share is loaded once
+        const auto h0 = plane_generator<false>(u, g, s, c, plane_a(p0), plane_b(p0), TRACE ? &t0 : nullptr);
+        const auto h1 = plane_generator<false>(u, g, s, c, plane_a(p1), plane_b(p1), TRACE ? &t1 : nullptr);
+        grid_release();
+        hf.store(p0, s, h0);
+        hf.store(p1, s, h1);
+    }
+    return double(t0) + double(t1);
+}
+
+template <class F>
+__device__ __forceinline__ int block_item(int w) {
+    return int(blockIdx.x) * EnsItemsPerBlock<F>::value + (EnsItemsPerBlock<F>::value == 1 ? 0 : w / 3);
+}
+
+template <class F>
+unsigned plaq_item_blocks(int nitems) {
+    return unsigned((nitems + EnsItemsPerBlock<F>::value - 1) / EnsItemsPerBlock<F>::value);
+}
+
+template <class F>
+__global__ void __launch_bounds__(192, PlaqMinBlocks<F>::value)
+    ens_plaq_kernel(char* u, char* h, const EnsConf* __restrict__ confs, int nconf, int nitems) {
+    const int w = int(threadIdx.x >> 5);
+    const int item = block_item<F>(w);
+    if (item >= nitems) return;
     const EnsConf& C = confs[find_conf(confs, nconf, item)];
     const Geo& g = C.g;
     const int s = (item - C.blk0) * 32 + int(threadIdx.x & 31);
+    grid_wait();
     if (s >= g.V) return;
-    const F uf{u + C.uoff, g.V};
-    const ForceField<typename F::Real> hf{h + C.hoff, g.V};
-    plaq_plane(uf, hf, g, s, int(threadIdx.x >> 5));
+    item_planes<false>(F{u + C.uoff, g.V}, ForceField<typename F::Real>{h + C.hoff, g.V}, g, s, w);
 }
 
-template <class F, int STAGE>
+template <class F, int STAGE, class FO>
 __global__ void __launch_bounds__(128, SplitMinBlocks<F>::value)
     ens_split_kernel(char* uin, char* uout, char* z, char* h, const EnsConf* __restrict__ confs, int nconf,
                      typename F::Real eps) {
@@ -146,10 +194,104 @@ __global__ void __launch_bounds__(128, SplitMinBlocks<F>::value)
     const EnsConf& C = confs[find_conf(confs, nconf, item)];
     const Geo& g = C.g;
     const int s = (item - C.blk0) * 32 + int(threadIdx.x & 31);
+    grid_wait();
     if (s >= g.V) return;
-    const F in{uin + C.uoff, g.V}, out{uout + C.uoff, g.V};
+    const F in{uin + C.uoff, g.V};
+    const FO out{uout + C.uoff, g.V};
     const ForceField<R> zf{z + C.zoff, g.V}, hf{h + C.hoff, g.V};
-    split_link_update<F, STAGE>(in, out, zf, hf, g, eps, s, mu);
+    split_link_update<F, STAGE, FO, false>(in, out, zf, hf, g, eps, s, mu);
+}
+
+// Every configuration's measurement in three launches over the work list: the
+// plane generators with one plaquette partial per warp (3 or 6 per item), the
+// energy and charge from them (clover_pair, observables.cuh) with three
+// partials per item, and one folding block per configuration.  The two launches
+// per configuration before it cost more than their kernels on small fields:
+// 6 x 8^4 + 4 x (6 x 10 x 12 x 14) + 2 x (12^3 x 24) in FP64 on B200, 120-125 us
+// less per measurement beyond what its step saves (the field is the next
+// stage 0's).
+template <class F>
+__global__ void __launch_bounds__(192, sizeof(typename F::Real) == 8 ? 3 : PlaqMinBlocks<F>::value)
+    ens_plaq_sum_kernel(char* u, char* h, const EnsConf* __restrict__ confs, int nconf, int nitems, double* partials) {
+    const int w = int(threadIdx.x >> 5);
+    const int item = block_item<F>(w);
+    if (item >= nitems) return;
+    const EnsConf& C = confs[find_conf(confs, nconf, item)];
+    const Geo& g = C.g;
+    const int s = (item - C.blk0) * 32 + int(threadIdx.x & 31);
+    double sum = 0.0;
+    if (s < g.V) sum = item_planes<true>(F{u + C.uoff, g.V}, ForceField<typename F::Real>{h + C.hoff, g.V}, g, s, w);
+    sum = warp_sum(sum);
+    constexpr int kPer = EnsItemsPerBlock<F>::value == 1 ? 6 : 3;
+    if ((threadIdx.x & 31) == 0) partials[int64_t(item) * kPer + w % kPer] = sum;
+}
+
+template <class F>
+__global__ void __launch_bounds__(96, CloverMinBlocks<F>::value)
+    ens_clover_kernel(char* u, char* h, const EnsConf* __restrict__ confs, int nconf, const double* plaq,
+                      double* partials) {
+    const int k = int(threadIdx.x >> 5), item = int(blockIdx.x);
+    const EnsConf& C = confs[find_conf(confs, nconf, item)];
+    const Geo& g = C.g;
+    const int s = (item - C.blk0) * 32 + int(threadIdx.x & 31);
+    double p = 0.0, energy = 0.0, topc = 0.0;
+    if (s < g.V) {
+        int c[4];
+        g.coords(s, c);
+        clover_pair(F{u + C.uoff, g.V}, ForceField<typename F::Real>{h + C.hoff, g.V}, g, s, c, k, energy, topc);
+    }
+    constexpr int kPer = EnsItemsPerBlock<F>::value == 1 ? 6 : 3;
+    if (threadIdx.x < kPer) p = plaq[int64_t(item) * kPer + threadIdx.x];
+    block_sum3(p, energy, topc);
+    if (threadIdx.x == 0) {
+        partials[3 * int64_t(item) + 0] = p;
+        partials[3 * int64_t(item) + 1] = energy;
+        partials[3 * int64_t(item) + 2] = topc;
+    }
+}
+
+// Block c folds configuration c's items in order: out + 4 c is its row.
+__global__ void __launch_bounds__(256) ens_fold_kernel(const EnsConf* __restrict__ confs, const double* partials,
+                                                       double* out) {
+    const EnsConf& C = confs[blockIdx.x];
+    const double* q = partials + 3 * int64_t(C.blk0);
+    double p = 0.0, energy = 0.0, topc = 0.0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < C.nblk; i += blockDim.x) {
+        p += q[3 * i + 0];
+        energy += q[3 * i + 1];
+        topc += q[3 * i + 2];
+    }
+    block_sum3(p, energy, topc);
+    if (threadIdx.x == 0) write_row(p, energy, topc, 1.0 / (18.0 * double(C.g.vglobal)), out + 4 * int64_t(blockIdx.x));
+}
+
+int64_t ens_measure_partials(int nitems) { return 9 * int64_t(nitems); }
+
+template <class F>
+static cudaError_t launch_ens_measure_typed(void* u, void* h, const EnsConf* confs, int nconf, int nitems,
+                                            double* partials, double* out, cudaStream_t st) {
+    char *a = (char*)u, *hh = (char*)h;
+    double* items = partials + 6 * int64_t(nitems);
+    ens_plaq_sum_kernel<F><<<plaq_item_blocks<F>(nitems), 192, 0, st>>>(a, hh, confs, nconf, nitems, partials);
+    ens_clover_kernel<F><<<nitems, 96, 0, st>>>(a, hh, confs, nconf, partials, items);
+    ens_fold_kernel<<<nconf, 256, 0, st>>>(confs, items, out);
+    return cudaGetLastError();
+}
+
+// Every configuration's row (out + 4 c) through the plane-generator pool h,
+// which then holds u's.  rows_in (FP64): rows 0 and 1 of the links only.
+cudaError_t launch_ens_measure(int prec, void* u, void* h, const EnsConf* confs, int nconf, int nitems, bool rows_in,
+                               double* partials, double* out, cudaStream_t st) {
+    switch (prec) {
+        case kFP64:
+            if (rows_in)
+                return launch_ens_measure_typed<FieldD18Rows>(u, h, confs, nconf, nitems, partials, out, st);
+            return launch_ens_measure_typed<FieldD18>(u, h, confs, nconf, nitems, partials, out, st);
+        case kFP32_18: return launch_ens_measure_typed<FieldF18>(u, h, confs, nconf, nitems, partials, out, st);
+        case kFP32_12: return launch_ens_measure_typed<FieldF12>(u, h, confs, nconf, nitems, partials, out, st);
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 // The same two kernels with the work list as a launch parameter (up to
@@ -174,29 +316,20 @@ __device__ __forceinline__ int find_conf_param(const EnsTable& t, int item) {
 }
 
 template <class F>
-__global__ void __launch_bounds__(192, PlaqMinBlocks<F>::value) ens_plaq_param_kernel(char* u, char* h, const __grid_constant__ EnsTable tab) {
+__global__ void __launch_bounds__(192, PlaqMinBlocks<F>::value)
+    ens_plaq_param_kernel(char* u, char* h, const __grid_constant__ EnsTable tab) {
     const int w = int(threadIdx.x >> 5);
-    const int item = int(blockIdx.x) * 2 + w / 3;
+    const int item = block_item<F>(w);
     if (item >= tab.c[tab.n - 1].blk0 + tab.c[tab.n - 1].nblk) return;
     const EnsConf& C = tab.c[find_conf_param(tab, item)];
     const Geo& g = C.g;
     const int s = (item - C.blk0) * 32 + int(threadIdx.x & 31);
+    grid_wait();
     if (s >= g.V) return;
-    const F uf{u + C.uoff, g.V};
-    const ForceField<typename F::Real> hf{h + C.hoff, g.V};
-    const int pr = w % 3;
-    const int p0 = pr == 0 ? 0 : (pr == 1 ? 2 : 3);
-    const int p1 = pr == 0 ? 1 : (pr == 1 ? 4 : 5);
-    int c[4];
-    g.coords(s, c);
-    // both planes before either store: the link the two share is loaded once
-    const auto h0 = plane_generator(uf, g, s, c, plane_a(p0), plane_b(p0));
-    const auto h1 = plane_generator(uf, g, s, c, plane_a(p1), plane_b(p1));
-    hf.store(p0, s, h0);
-    hf.store(p1, s, h1);
+    item_planes<false>(F{u + C.uoff, g.V}, ForceField<typename F::Real>{h + C.hoff, g.V}, g, s, w);
 }
 
-template <class F, int STAGE>
+template <class F, int STAGE, class FO>
 __global__ void __launch_bounds__(128, SplitMinBlocks<F>::value)
     ens_split_param_kernel(char* uin, char* uout, char* z, char* h, const __grid_constant__ EnsTable tab,
                            typename F::Real eps) {
@@ -206,38 +339,45 @@ __global__ void __launch_bounds__(128, SplitMinBlocks<F>::value)
     const EnsConf& C = tab.c[find_conf_param(tab, item)];
     const Geo& g = C.g;
     const int s = (item - C.blk0) * 32 + int(threadIdx.x & 31);
+    grid_wait();
     if (s >= g.V) return;
-    const F in{uin + C.uoff, g.V}, out{uout + C.uoff, g.V};
+    const F in{uin + C.uoff, g.V};
+    const FO out{uout + C.uoff, g.V};
     const ForceField<R> zf{z + C.zoff, g.V}, hf{h + C.hoff, g.V};
-    split_link_update<F, STAGE>(in, out, zf, hf, g, eps, s, mu);
+    split_link_update<F, STAGE, FO, false>(in, out, zf, hf, g, eps, s, mu);
 }
 
-template <class F>
+// field: the plane-generator launch (not where the pool holds uin's already).
+template <class F, class FO = F>
 static cudaError_t launch_ens_split_typed(int stage, void* uin, void* uout, void* z, void* h, const EnsConf* confs,
-                                          int nconf, int nitems, double eps, cudaStream_t st,
+                                          int nconf, int nitems, bool field, double eps, cudaStream_t st,
                                           const EnsConf* host_confs) {
     using R = typename F::Real;
     const R e = R(stage == 0 ? eps * 0.25 : eps);
     char *a = (char*)uin, *b = (char*)uout, *zz = (char*)z, *hh = (char*)h;
+    const unsigned pb = plaq_item_blocks<F>(nitems), sb = unsigned(nitems);
+    cudaError_t r = cudaSuccess;
     if (host_confs && nconf <= kParamConfs) {
         EnsTable tab;
         std::memcpy(tab.c, host_confs, sizeof(EnsConf) * size_t(nconf));
         tab.n = nconf;
-        ens_plaq_param_kernel<F><<<(nitems + 1) / 2, 192, 0, st>>>(a, hh, tab);
+        if (field) r = launch_chained(true, ens_plaq_param_kernel<F>, pb, 192, st, a, hh, tab);
+        if (r != cudaSuccess) return r;
+        auto launch = [&](auto kernel) { return launch_chained(true, kernel, sb, 128, st, a, b, zz, hh, tab, e); };
         switch (stage) {
-            case 0: ens_split_param_kernel<F, 0><<<nitems, 128, 0, st>>>(a, b, zz, hh, tab, e); break;
-            case 1: ens_split_param_kernel<F, 1><<<nitems, 128, 0, st>>>(a, b, zz, hh, tab, e); break;
-            default: ens_split_param_kernel<F, 2><<<nitems, 128, 0, st>>>(a, b, zz, hh, tab, e); break;
+            case 0: return launch(ens_split_param_kernel<F, 0, FO>);
+            case 1: return launch(ens_split_param_kernel<F, 1, FO>);
+            default: return launch(ens_split_param_kernel<F, 2, FO>);
         }
-        return cudaGetLastError();
     }
-    ens_plaq_kernel<F><<<nitems, 192, 0, st>>>(a, hh, confs, nconf);
+    if (field) r = launch_chained(true, ens_plaq_kernel<F>, pb, 192, st, a, hh, confs, nconf, nitems);
+    if (r != cudaSuccess) return r;
+    auto launch = [&](auto kernel) { return launch_chained(true, kernel, sb, 128, st, a, b, zz, hh, confs, nconf, e); };
     switch (stage) {
-        case 0: ens_split_kernel<F, 0><<<nitems, 128, 0, st>>>(a, b, zz, hh, confs, nconf, e); break;
-        case 1: ens_split_kernel<F, 1><<<nitems, 128, 0, st>>>(a, b, zz, hh, confs, nconf, e); break;
-        default: ens_split_kernel<F, 2><<<nitems, 128, 0, st>>>(a, b, zz, hh, confs, nconf, e); break;
+        case 0: return launch(ens_split_kernel<F, 0, FO>);
+        case 1: return launch(ens_split_kernel<F, 1, FO>);
+        default: return launch(ens_split_kernel<F, 2, FO>);
     }
-    return cudaGetLastError();
 }
 
 // The same two kernels per run of consecutive configurations of one geometry
@@ -254,46 +394,23 @@ struct EnsRun {
 };
 
 template <class F>
-__global__ void __launch_bounds__(192, PlaqMinBlocks<F>::value) ens_run_plaq_kernel(char* u, char* h, const __grid_constant__ EnsRun r) {
+__global__ void __launch_bounds__(192, PlaqMinBlocks<F>::value)
+    ens_run_plaq_kernel(char* u, char* h, const __grid_constant__ EnsRun r) {
     const int w = int(threadIdx.x >> 5);
-    if constexpr (sizeof(typename F::Real) == 8) {  // FP64: one plane per thread, warp w plane w of one item
-        const int item = int(blockIdx.x);
-        const int conf = item / r.nblk;
-        if (conf >= r.nconf) return;
-        const Geo& g = r.g;
-        const int s = (item - conf * r.nblk) * 32 + int(threadIdx.x & 31);
-        if (s >= g.V) return;
-        const F uf{u + conf * r.ustride, g.V};
-        const ForceField<typename F::Real> hf{h + conf * r.hstride, g.V};
-        int c[4];
-        g.coords(s, c);
-        hf.store(w, s, plane_generator(uf, g, s, c, plane_a(w), plane_b(w)));
-        return;
-    }
     // FP32: from the run's end, as plaq_field_kernel (its stage kernel starts
     // on the L2-resident items)
-    const int blk = int(gridDim.x - 1 - blockIdx.x);
-    const int item = blk * 2 + w / 3;
+    const int item = EnsItemsPerBlock<F>::value == 1 ? int(blockIdx.x)
+                                                     : int(gridDim.x - 1 - blockIdx.x) * 2 + w / 3;
     const int conf = item / r.nblk;
     if (conf >= r.nconf) return;
     const Geo& g = r.g;
     const int s = (item - conf * r.nblk) * 32 + int(threadIdx.x & 31);
+    grid_wait();
     if (s >= g.V) return;
-    const F uf{u + conf * r.ustride, g.V};
-    const ForceField<typename F::Real> hf{h + conf * r.hstride, g.V};
-    const int pr = w % 3;
-    const int p0 = pr == 0 ? 0 : (pr == 1 ? 2 : 3);
-    const int p1 = pr == 0 ? 1 : (pr == 1 ? 4 : 5);
-    int c[4];
-    g.coords(s, c);
-    // both planes before either store: the link the two share is loaded once
-    const auto h0 = plane_generator(uf, g, s, c, plane_a(p0), plane_b(p0));
-    const auto h1 = plane_generator(uf, g, s, c, plane_a(p1), plane_b(p1));
-    hf.store(p0, s, h0);
-    hf.store(p1, s, h1);
+    item_planes<false>(F{u + conf * r.ustride, g.V}, ForceField<typename F::Real>{h + conf * r.hstride, g.V}, g, s, w);
 }
 
-template <class F, int STAGE>
+template <class F, int STAGE, class FO>
 __global__ void __launch_bounds__(128, SplitMinBlocks<F>::value)
     ens_run_split_kernel(char* uin, char* uout, char* z, char* h, const __grid_constant__ EnsRun r,
                          typename F::Real eps) {
@@ -303,10 +420,12 @@ __global__ void __launch_bounds__(128, SplitMinBlocks<F>::value)
     const int conf = item / r.nblk;
     const Geo& g = r.g;
     const int s = (item - conf * r.nblk) * 32 + int(threadIdx.x & 31);
+    grid_wait();
     if (s >= g.V) return;
-    const F in{uin + conf * r.ustride, g.V}, out{uout + conf * r.ustride, g.V};
+    const F in{uin + conf * r.ustride, g.V};
+    const FO out{uout + conf * r.ustride, g.V};
     const ForceField<R> zf{z + conf * r.zstride, g.V}, hf{h + conf * r.hstride, g.V};
-    split_link_update<F, STAGE>(in, out, zf, hf, g, eps, s, mu);
+    split_link_update<F, STAGE, FO, false>(in, out, zf, hf, g, eps, s, mu);
 }
 
 // A run and where its first configuration starts in each pool.
@@ -315,29 +434,43 @@ struct EnsRunLaunch {
     int64_t uoff, zoff, hoff;
 };
 
-// One stage of one run: its plaquette-field launch, then its stage launch.
-template <class F>
+// One stage of one run: its plaquette-field launch (field: not where the pool
+// holds uin's already), then its stage launch, chained to it.
+template <class F, class FO = F>
 static cudaError_t launch_ens_run_typed(int stage, void* uin, void* uout, void* z, void* h, const EnsRunLaunch& L,
-                                        double eps, cudaStream_t st) {
+                                        bool field, double eps, cudaStream_t st) {
     using R = typename F::Real;
     const R e = R(stage == 0 ? eps * 0.25 : eps);
     const int items = L.r.nconf * L.r.nblk;
     char *a = (char*)uin + L.uoff, *b = (char*)uout + L.uoff, *zz = (char*)z + L.zoff, *hh = (char*)h + L.hoff;
-    ens_run_plaq_kernel<F><<<sizeof(R) == 8 ? items : (items + 1) / 2, 192, 0, st>>>(a, hh, L.r);
+    if (field) ens_run_plaq_kernel<F><<<plaq_item_blocks<F>(items), 192, 0, st>>>(a, hh, L.r);
     switch (stage) {
-        case 0: ens_run_split_kernel<F, 0><<<items, 128, 0, st>>>(a, b, zz, hh, L.r, e); break;
-        case 1: ens_run_split_kernel<F, 1><<<items, 128, 0, st>>>(a, b, zz, hh, L.r, e); break;
-        default: ens_run_split_kernel<F, 2><<<items, 128, 0, st>>>(a, b, zz, hh, L.r, e); break;
+        case 0: ens_run_split_kernel<F, 0, FO><<<items, 128, 0, st>>>(a, b, zz, hh, L.r, e); break;
+        case 1: ens_run_split_kernel<F, 1, FO><<<items, 128, 0, st>>>(a, b, zz, hh, L.r, e); break;
+        default: ens_run_split_kernel<F, 2, FO><<<items, 128, 0, st>>>(a, b, zz, hh, L.r, e); break;
     }
     return cudaGetLastError();
 }
 
+// What a two-kernel stage of an ensemble reads and leaves: field, as above;
+// rows_in / rows_out (FP64), as launch_rk_split_stage.
+struct EnsStageIo {
+    bool field = true, rows_in = false, rows_out = false;
+};
+
 cudaError_t launch_ens_run_stage(int prec, int stage, void* uin, void* uout, void* z, void* h, const EnsRunLaunch& L,
-                                 double eps, cudaStream_t st) {
+                                 const EnsStageIo& io, double eps, cudaStream_t st) {
     switch (prec) {
-        case kFP64: return launch_ens_run_typed<FieldD18>(stage, uin, uout, z, h, L, eps, st);
-        case kFP32_18: return launch_ens_run_typed<FieldF18>(stage, uin, uout, z, h, L, eps, st);
-        case kFP32_12: return launch_ens_run_typed<FieldF12>(stage, uin, uout, z, h, L, eps, st);
+        case kFP64:
+            if (io.rows_in && io.rows_out)
+                return launch_ens_run_typed<FieldD18Rows>(stage, uin, uout, z, h, L, io.field, eps, st);
+            if (io.rows_in)
+                return launch_ens_run_typed<FieldD18Rows, FieldD18>(stage, uin, uout, z, h, L, io.field, eps, st);
+            if (io.rows_out)
+                return launch_ens_run_typed<FieldD18, FieldD18Rows>(stage, uin, uout, z, h, L, io.field, eps, st);
+            return launch_ens_run_typed<FieldD18>(stage, uin, uout, z, h, L, io.field, eps, st);
+        case kFP32_18: return launch_ens_run_typed<FieldF18>(stage, uin, uout, z, h, L, io.field, eps, st);
+        case kFP32_12: return launch_ens_run_typed<FieldF12>(stage, uin, uout, z, h, L, io.field, eps, st);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -452,12 +585,27 @@ cudaError_t launch_ens_tile_stage(int prec, int stage, void* uin, void* uout, vo
 
 // Work items must be 32-site groups (block 128).
 cudaError_t launch_ens_split_stage(int prec, int stage, void* uin, void* uout, void* z, void* h, const EnsConf* confs,
-                                   int nconf, int nitems, double eps, cudaStream_t st,
-                                   const EnsConf* host_confs = nullptr) {
+                                   int nconf, int nitems, const EnsStageIo& io, double eps, cudaStream_t st,
+                                   const EnsConf* host) {
     switch (prec) {
-        case kFP64: return launch_ens_split_typed<FieldD18>(stage, uin, uout, z, h, confs, nconf, nitems, eps, st, host_confs);
-        case kFP32_18: return launch_ens_split_typed<FieldF18>(stage, uin, uout, z, h, confs, nconf, nitems, eps, st, host_confs);
-        case kFP32_12: return launch_ens_split_typed<FieldF12>(stage, uin, uout, z, h, confs, nconf, nitems, eps, st, host_confs);
+        case kFP64:
+            if (io.rows_in && io.rows_out)
+                return launch_ens_split_typed<FieldD18Rows>(stage, uin, uout, z, h, confs, nconf, nitems, io.field, eps,
+                                                            st, host);
+            if (io.rows_in)
+                return launch_ens_split_typed<FieldD18Rows, FieldD18>(stage, uin, uout, z, h, confs, nconf, nitems,
+                                                                      io.field, eps, st, host);
+            if (io.rows_out)
+                return launch_ens_split_typed<FieldD18, FieldD18Rows>(stage, uin, uout, z, h, confs, nconf, nitems,
+                                                                      io.field, eps, st, host);
+            return launch_ens_split_typed<FieldD18>(stage, uin, uout, z, h, confs, nconf, nitems, io.field, eps, st,
+                                                    host);
+        case kFP32_18:
+            return launch_ens_split_typed<FieldF18>(stage, uin, uout, z, h, confs, nconf, nitems, io.field, eps, st,
+                                                    host);
+        case kFP32_12:
+            return launch_ens_split_typed<FieldF12>(stage, uin, uout, z, h, confs, nconf, nitems, io.field, eps, st,
+                                                    host);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -498,6 +646,13 @@ std::map<std::string, EnsTuning> g_tune_cache;
 
 using namespace ym;
 
+// A captured step and what it was captured for.
+struct EnsGraph {
+    cudaGraphExec_t exec = nullptr;
+    double eps = 0.0;
+    int block = 0, grid = 0, io = 0;
+};
+
 struct ymflow_ens {
     int nconf = 0;
     int prec = 0;
@@ -508,8 +663,8 @@ struct ymflow_ens {
     void* u[2] = {nullptr, nullptr};
     int cur = 0;
     void* z = nullptr;
-    void* h = nullptr;       // plane generators of the two-kernel stage (FP32 ensembles)
-    bool split = false;      // FP32: the two-kernel stage, one block per work item
+    void* h = nullptr;       // plane generators of the two-kernel stage (FP64: where they fit)
+    bool split = false;      // the two-kernel stage, one block per work item
     bool by_runs = false;    // ... launched per run of equal-geometry configurations
     std::vector<EnsRunLaunch> runs;
     // the runs' launch streams (run i on side[i % side.size()]): each run's
@@ -528,18 +683,16 @@ struct ymflow_ens {
     double* staging = nullptr;  // .bin-layout buffer sized for the largest configuration
     int64_t max_v = 0;
     double* partials = nullptr;
-    int partial_cap = 0;
     double* meas = nullptr;
     int meas_cap = 0;
     double* meas_host = nullptr;
     unsigned long long* deviation = nullptr;
-    cudaGraphExec_t graph[2] = {nullptr, nullptr};
-    double graph_eps[2] = {0.0, 0.0};
-    int graph_cfg[2][2] = {{0, 0}, {0, 0}};
+    EnsGraph graphs[4];      // the step from u[k & 1]; k & 2: after a measurement
     int block = 128;
     int grid = 0;  // persistent CTAs (0: one per work item)
     bool use_graph = true;
     bool tuned = false;
+    bool form_chosen = false;  // set_tuning was called, or the first flow has settled the form
     std::vector<char> loaded;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int64_t step = 0;
@@ -656,12 +809,13 @@ int apply_tuning(ymflow_ens* e, const EnsTuning& tn) {
 // stream onto the side streams and joined back (parallel branches when
 // captured into the step graph).  With one side stream, everything stays on
 // the ensemble's stream.
-cudaError_t enqueue_runs(ymflow_ens* e, int nst, void* const* in, void* const* out, double eps) {
+cudaError_t enqueue_runs(ymflow_ens* e, int nst, void* const* in, void* const* out, const EnsStageIo* io, double eps) {
     const int ns = int(e->side.size());
     if (ns == 0) {
         for (int s = 0; s < nst; s++)
             for (const EnsRunLaunch& L : e->runs) {
-                const cudaError_t r = launch_ens_run_stage(e->prec, s, in[s], out[s], e->z, e->h, L, eps, e->stream);
+                const cudaError_t r =
+                    launch_ens_run_stage(e->prec, s, in[s], out[s], e->z, e->h, L, io[s], eps, e->stream);
                 if (r != cudaSuccess) return r;
             }
         return cudaSuccess;
@@ -670,7 +824,7 @@ cudaError_t enqueue_runs(ymflow_ens* e, int nst, void* const* in, void* const* o
     for (int k = 0; k < ns && r == cudaSuccess; k++) r = cudaStreamWaitEvent(e->side[k], e->fork, 0);
     for (int s = 0; s < nst && r == cudaSuccess; s++)
         for (size_t i = 0; i < e->runs.size() && r == cudaSuccess; i++)
-            r = launch_ens_run_stage(e->prec, s, in[s], out[s], e->z, e->h, e->runs[i], eps, e->side[i % ns]);
+            r = launch_ens_run_stage(e->prec, s, in[s], out[s], e->z, e->h, e->runs[i], io[s], eps, e->side[i % ns]);
     for (int k = 0; k < ns; k++) {  // join every branch, also after a failed launch
         const cudaError_t j = cudaEventRecord(e->side_done[k], e->side[k]);
         const cudaError_t w = j == cudaSuccess ? cudaStreamWaitEvent(e->stream, e->side_done[k], 0) : j;
@@ -679,20 +833,37 @@ cudaError_t enqueue_runs(ymflow_ens* e, int nst, void* const* in, void* const* o
     return r;
 }
 
-cudaError_t enqueue_ens_step(ymflow_ens* e, int from, double eps) {
+// How a step meets its neighbours in a call: its plane generators are in the
+// pool already (a measurement has just formed them), its links were written,
+// and will be read, by a stage of the same call (FP64: as rows 0 and 1).
+struct EnsStepIo {
+    bool field_ready = false, rows_in = false, rows_out = false;
+    int key() const { return (field_ready ? 1 : 0) | (rows_in ? 2 : 0) | (rows_out ? 4 : 0); }
+};
+
+bool two_kernel_form(const ymflow_ens* e) { return !e->tile && e->split; }
+
+cudaError_t enqueue_ens_step(ymflow_ens* e, int from, const EnsStepIo& step, double eps) {
     void* a = e->u[from];
     void* b = e->u[1 - from];
     void* in[3] = {a, b, a};
     void* out[3] = {b, a, b};
     const int ni = nitems(e);
     const int grid = e->grid > 0 ? std::min(e->grid, ni) : ni;
-    if (!e->tile && e->split && e->by_runs) return enqueue_runs(e, 3, in, out, eps);
+    const bool rows = e->prec == YMFLOW_FP64;
+    EnsStageIo io[3];
+    for (int s = 0; s < 3; s++) {
+        io[s].field = s > 0 || !step.field_ready;
+        io[s].rows_in = rows && (s > 0 || step.rows_in);
+        io[s].rows_out = rows && (s < 2 || step.rows_out);
+    }
+    if (two_kernel_form(e) && e->by_runs) return enqueue_runs(e, 3, in, out, io, eps);
     for (int s = 0; s < 3; s++) {
         cudaError_t r = e->tile ? launch_ens_tile_stage(e->prec, s, in[s], out[s], e->z, e->confs_dev, e->nconf,
                                                         e->nunits, e->tile_grid, e->tile_threads, e->tile_smem, eps,
                                                         e->stream)
                         : e->split ? launch_ens_split_stage(e->prec, s, in[s], out[s], e->z, e->h, e->confs_dev,
-                                                            e->nconf, ni, eps, e->stream, e->confs.data())
+                                                            e->nconf, ni, io[s], eps, e->stream, e->confs.data())
                                    : launch_ens_stage(e->prec, s, in[s], out[s], e->z, e->confs_dev, e->nconf, ni,
                                                       grid, e->block, eps, e->stream);
         if (r != cudaSuccess) return r;
@@ -701,38 +872,50 @@ cudaError_t enqueue_ens_step(ymflow_ens* e, int from, double eps) {
 }
 
 void drop_graphs(ymflow_ens* e) {
-    for (int i = 0; i < 2; i++) {
-        if (e->graph[i]) cudaGraphExecDestroy(e->graph[i]);
-        e->graph[i] = nullptr;
+    for (auto& g : e->graphs) {
+        if (g.exec) cudaGraphExecDestroy(g.exec);
+        g.exec = nullptr;
     }
 }
 
-int run_ens_step(ymflow_ens* e, double eps) {
+// The steps that repeat within a call are replayed as graphs (one per buffer
+// and with or without a measurement before); its first and last are launched
+// as they are.
+int run_ens_step(ymflow_ens* e, double eps, int s, int nsteps, bool field_ready = false) {
     const int from = e->cur;
-    if (e->use_graph) {
-        if (!e->graph[from] || e->graph_eps[from] != eps || e->graph_cfg[from][0] != e->block ||
-            e->graph_cfg[from][1] != e->grid) {
-            if (e->graph[from]) cudaGraphExecDestroy(e->graph[from]);
-            e->graph[from] = nullptr;
+    EnsStepIo step;
+    if (two_kernel_form(e)) {
+        step.field_ready = field_ready;
+        if (e->prec == YMFLOW_FP64) {
+            step.rows_in = s > 1;
+            step.rows_out = s < nsteps;
+        }
+    }
+    if (e->use_graph && s > 1 && s < nsteps) {
+        EnsGraph& G = e->graphs[from + (step.field_ready ? 2 : 0)];
+        if (!G.exec || G.eps != eps || G.block != e->block || G.grid != e->grid || G.io != step.key()) {
+            if (G.exec) cudaGraphExecDestroy(G.exec);
+            G.exec = nullptr;
             cudaGraph_t g = nullptr;
             YE_CK(e, cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
-            cudaError_t le = enqueue_ens_step(e, from, eps);
+            cudaError_t le = enqueue_ens_step(e, from, step, eps);
             cudaError_t ce = cudaStreamEndCapture(e->stream, &g);
             if (le != cudaSuccess) {
                 if (g) cudaGraphDestroy(g);
                 return ecuda(e, le, "stage launch during capture");
             }
             YE_CK(e, ce, "end capture");
-            cudaError_t ie = cudaGraphInstantiate(&e->graph[from], g, 0);
+            cudaError_t ie = cudaGraphInstantiate(&G.exec, g, 0);
             cudaGraphDestroy(g);
             YE_CK(e, ie, "instantiate step graph");
-            e->graph_eps[from] = eps;
-            e->graph_cfg[from][0] = e->block;
-            e->graph_cfg[from][1] = e->grid;
+            G.eps = eps;
+            G.block = e->block;
+            G.grid = e->grid;
+            G.io = step.key();
         }
-        YE_CK(e, cudaGraphLaunch(e->graph[from], e->stream), "launch step graph");
+        YE_CK(e, cudaGraphLaunch(G.exec, e->stream), "launch step graph");
     } else {
-        YE_CK(e, enqueue_ens_step(e, from, eps), "stage launch");
+        YE_CK(e, enqueue_ens_step(e, from, step, eps), "stage launch");
     }
     e->cur = 1 - from;
     return YMFLOW_OK;
@@ -763,17 +946,45 @@ int ensure_ens_meas(ymflow_ens* e, int rows) {
     return YMFLOW_OK;
 }
 
-// Observables of every configuration into rows [row*nconf, row*nconf + nconf).
-int enqueue_ens_measure(ymflow_ens* e, int row) {
+// Observables of every configuration into rows [row*nconf, row*nconf + nconf),
+// through the plane-generator pool where there is one (it then holds the
+// current links').
+int enqueue_ens_measure(ymflow_ens* e, int row, bool rows_in) {
+    double* out = e->meas + 4 * size_t(row) * e->nconf;
+    if (e->h) {
+        YE_CK(e, launch_ens_measure(e->prec, e->u[e->cur], e->h, e->confs_dev, e->nconf, nitems(e), rows_in, e->partials,
+                                    out, e->stream),
+              "observables launch");
+        return YMFLOW_OK;
+    }
     for (int c = 0; c < e->nconf; c++) {
         const EnsConf& C = e->confs[c];
         const void* u = (const char*)e->u[e->cur] + C.uoff;
         YE_CK(e, launch_observables(e->prec, u, C.g, e->partials, e->stream), "observables launch");
-        YE_CK(e, launch_obs_finalize(e->partials, obs_blocks(C.g), C.g,
-                                     e->meas + 4 * (size_t(row) * e->nconf + c), e->stream),
+        YE_CK(e, launch_obs_finalize(e->partials, obs_blocks(C.g), C.g, out + 4 * size_t(c), e->stream),
               "observables fold");
     }
     return YMFLOW_OK;
+}
+
+// The form of an ensemble that nobody has tuned, settled at its first flow: the
+// two-kernel stage where there is a plane-generator pool, per run (form 3)
+// where the runs are large enough on average to be launched apart, else over
+// the work list (form 1), whose blocks look their geometry up.  us per step on
+// B200 at forms 1 / 3: runs of 5,184 sites FP64 32 / 31, FP32-12 25 / 26; 8 runs
+// of 8,000 FP32-12 58 / 64; 3 runs of 12,288 FP64 67 / 57, FP32-12 45 / 38; 8
+// runs of 16,000 FP64 208 / 185, FP32-12 106 / 96; 6 x 8^4 + 4 x (6 x 10 x 12 x
+// 14) + 2 x (12^3 x 24) FP64 245 / 235 (309 with the fused kernel), FP32-12 126 /
+// 106.
+constexpr int64_t kSitesPerRun = 10240;
+void settle_form(ymflow_ens* e) {
+    if (e->tuned || e->form_chosen) return;
+    e->form_chosen = true;
+    if (!e->h) return;
+    int64_t sites = 0;
+    for (const EnsConf& C : e->confs) sites += C.g.V;
+    e->split = true;
+    e->by_runs = sites >= kSitesPerRun * int64_t(e->runs.size());
 }
 
 void* conf_links(const ymflow_ens* e, int c) { return (char*)e->u[e->cur] + e->confs[c].uoff; }
@@ -789,9 +1000,10 @@ float time_stage0(ymflow_ens* e, double eps, int reps) {
         if (e->tile)
             return launch_ens_tile_stage(e->prec, 0, a, b, e->z, e->confs_dev, e->nconf, e->nunits, e->tile_grid,
                                          e->tile_threads, e->tile_smem, eps, e->stream);
-        if (e->split && e->by_runs) return enqueue_runs(e, 1, &a, &b, eps);
+        const EnsStageIo io;
+        if (e->split && e->by_runs) return enqueue_runs(e, 1, &a, &b, &io, eps);
         if (e->split)
-            return launch_ens_split_stage(e->prec, 0, a, b, e->z, e->h, e->confs_dev, e->nconf, ni, eps, e->stream,
+            return launch_ens_split_stage(e->prec, 0, a, b, e->z, e->h, e->confs_dev, e->nconf, ni, io, eps, e->stream,
                                           e->confs.data());
         return launch_ens_stage(e->prec, 0, a, b, e->z, e->confs_dev, e->nconf, ni, grid, e->block, eps, e->stream);
     };
@@ -876,11 +1088,8 @@ ymflow_ens* ymflow_ensemble_create(int nconf, const int* dims, int precision, in
     if (r == YMFLOW_OK) r = ens_alloc(e, &e->u[0], size_t(uo), "link pool 0");
     if (r == YMFLOW_OK) r = ens_alloc(e, &e->u[1], size_t(uo), "link pool 1");
     if (r == YMFLOW_OK) r = ens_alloc(e, &e->z, size_t(zo), "generator pool");
-    // FP32 ensembles flow with the two-kernel stage, as FP32 single contexts do
-    // FP32 ensembles flow with the two-kernel stage, FP64 ones with the fused
-    // kernel until the autotuner or ymflow_ensemble_set_tuning picks the
-    // per-run two-kernel form; an FP64 ensemble without room for the plane
-    // generators keeps the fused kernel only
+    // the two-kernel stage (FP64: from the first flow on, settle_form); an FP64
+    // ensemble without room for the plane generators keeps the fused kernel
     e->split = precision != YMFLOW_FP64;
     if (r == YMFLOW_OK) {
         r = ens_alloc(e, &e->h, size_t(ho), "plane-generator pool");
@@ -929,11 +1138,14 @@ ymflow_ens* ymflow_ensemble_create(int nconf, const int* dims, int precision, in
     if (r == YMFLOW_OK) r = ens_alloc(e, (void**)&e->confs_dev, sizeof(EnsConf) * nconf, "work list");
     if (r == YMFLOW_OK) r = ens_alloc(e, (void**)&e->deviation, sizeof(unsigned long long), "drift flag");
     if (r == YMFLOW_OK) {
-        // most observable blocks of any configuration (the kernel's grid is capped)
-        int cap = 1;
-        for (const EnsConf& C : e->confs) cap = std::max(cap, obs_blocks(C.g));
-        e->partial_cap = cap;
-        r = ens_alloc(e, (void**)&e->partials, size_t(e->partial_cap) * 3 * sizeof(double), "partials");
+        // all configurations' work items at once, or (without the
+        // plane-generator pool) one configuration's observable blocks
+        int64_t cap = 3;
+        if (e->h)
+            for (const EnsConf& C : e->confs) cap += ens_measure_partials((C.g.V + 31) / 32);
+        else
+            for (const EnsConf& C : e->confs) cap = std::max<int64_t>(cap, 3 * int64_t(obs_blocks(C.g)));
+        r = ens_alloc(e, (void**)&e->partials, size_t(cap) * sizeof(double), "partials");
     }
     if (r == YMFLOW_OK && (cudaEventCreate(&e->ev0) != cudaSuccess || cudaEventCreate(&e->ev1) != cudaSuccess))
         r = YMFLOW_ERR_CUDA;
@@ -1049,12 +1261,16 @@ int ymflow_ensemble_flow(ymflow_ens* e, double eps, int nsteps, int measure_ever
     const bool reunit = e->prec != YMFLOW_FP64 && reunit_every > 0;
     if (reunit) YE_CK(e, cudaMemsetAsync(e->deviation, 0, sizeof(unsigned long long), e->stream), "reset drift");
     int row = 0;
-    if ((r = enqueue_ens_measure(e, row)) != YMFLOW_OK) return r;
+    settle_form(e);
+    if ((r = enqueue_ens_measure(e, row, false)) != YMFLOW_OK) return r;
     rs[row] = e->step;
     rt[row] = e->t;
     row++;
+    const bool by_rows = e->prec == YMFLOW_FP64 && two_kernel_form(e);
+    bool field_ready = e->h != nullptr;  // a measurement leaves its plane generators for the next stage 0
     for (int s = 1; s <= nsteps; s++) {
-        if ((r = run_ens_step(e, eps)) != YMFLOW_OK) return r;
+        if ((r = run_ens_step(e, eps, s, nsteps, field_ready)) != YMFLOW_OK) return r;
+        field_ready = false;
         e->step++;
         e->t += eps;
         if (reunit && s % reunit_every == 0)
@@ -1062,10 +1278,11 @@ int ymflow_ensemble_flow(ymflow_ens* e, double eps, int nsteps, int measure_ever
                 YE_CK(e, launch_reunitarize(e->prec, conf_links(e, c), e->confs[c].g, e->deviation, e->stream),
                       "reunitarise");
         if ((measure_every > 0 && s % measure_every == 0) || s == nsteps) {
-            if ((r = enqueue_ens_measure(e, row)) != YMFLOW_OK) return r;
+            if ((r = enqueue_ens_measure(e, row, by_rows && s < nsteps)) != YMFLOW_OK) return r;
             rs[row] = e->step;
             rt[row] = e->t;
             row++;
+            field_ready = e->h != nullptr;
         }
     }
     YE_CK(e, cudaMemcpyAsync(e->meas_host, e->meas, size_t(rows) * e->nconf * 4 * sizeof(double),
@@ -1108,8 +1325,9 @@ int ymflow_ensemble_time_steps(ymflow_ens* e, double eps, int nsteps, float* ela
         if (!e->loaded[c]) return efail(e, YMFLOW_ERR_STATE, "configuration not loaded");
     DeviceGuard guard(e->device);
     YE_CK(e, cudaEventRecord(e->ev0, e->stream), "event");
+    settle_form(e);
     for (int s = 0; s < nsteps; s++) {
-        int r = run_ens_step(e, eps);
+        int r = run_ens_step(e, eps, s + 1, nsteps);
         if (r != YMFLOW_OK) return r;
         e->step++;
         e->t += eps;
@@ -1159,7 +1377,8 @@ int ymflow_ensemble_autotune(ymflow_ens* e, double eps, int* block_out, int* gri
     } else {
         const int resident = ens_max_resident(e->prec, 128);
         for (int grid : {0, resident * sms, 2 * resident * sms}) cands.push_back({0, 128, grid});
-        if (e->h) cands.push_back({3, 128, 0});
+        if (e->h)
+            for (int form : {1, 3}) cands.push_back({form, 128, 0});
     }
     for (int threads : {128, 256, 384, 512}) cands.push_back({2, threads, 0});
     const bool was_split = e->split;
@@ -1220,6 +1439,7 @@ int ymflow_ensemble_set_tuning(ymflow_ens* e, int stage_form, int block, int gri
         return efail(e, YMFLOW_ERR_ARG, "stage form is 0, 1, 2 or 3 (1 and 3 need the plane-generator pool)");
     }
     YE_CK(e, cudaStreamSynchronize(e->stream), "set tuning");
+    e->form_chosen = true;
     drop_graphs(e);
     return YMFLOW_OK;
 }

@@ -288,6 +288,18 @@ __device__ __forceinline__ R herm_trace_mul(const Herm8<R>& a, const Herm8<R>& b
     return fma(R(2), o, d);
 }
 
+// Energy and charge of the plane pair k of site s, (01,23), (02,13) or (03,12).
+template <class F>
+__device__ __forceinline__ void clover_pair(const F& u, const ForceField<typename F::Real>& hf, const Geo& g, int s,
+                                            const int c[4], int k, double& energy, double& topc) {
+    const auto a = clover_generator(u, hf, g, s, c, 0, k + 1);
+    const auto b = clover_generator(u, hf, g, s, c, k == 0 ? 2 : 1, k == 2 ? 2 : 3);
+    // Re tr(G_a G_b) = -4 tr(S_a S_b); the pairs' signs as in site_observables
+    energy = -4.0 * (double(herm_trace_mul(a, a)) + double(herm_trace_mul(b, b)));
+    const double t = 4.0 * double(herm_trace_mul(a, b));
+    topc = k == 1 ? -t : t;
+}
+
 // Resident 96-thread blocks: FP64 5 (128 registers, 15 warps per SM; a plane
 // pair with one transport live needs all of them), FP32 10 (64, 30 warps).
 template <class F>
@@ -307,8 +319,6 @@ __global__ void __launch_bounds__(96, CloverMinBlocks<F>::value)
     __shared__ double sums[2][96];
     sums[0][threadIdx.x] = sums[1][threadIdx.x] = 0.0;
     const int k = int(threadIdx.x >> 5);
-    const int mu_b = k == 0 ? 2 : 1;
-    const int nu_b = k == 2 ? 2 : 3;
     const int items = (g.site1 - g.site0 + 31) / 32;
     for (int item = blockIdx.x; item < items; item += gridDim.x) {
         const int s = g.site0 + item * 32 + int(threadIdx.x & 31);
@@ -316,12 +326,10 @@ __global__ void __launch_bounds__(96, CloverMinBlocks<F>::value)
         int c[4];
         g.coords(s, c);
         if (!g.interior(c)) continue;  // a block's halo sites are its neighbours'
-        const auto a = clover_generator(u, hf, g, s, c, 0, k + 1);
-        const auto b = clover_generator(u, hf, g, s, c, mu_b, nu_b);
-        // Re tr(G_a G_b) = -4 tr(S_a S_b); the pairs' signs as in site_observables
-        sums[0][threadIdx.x] -= 4.0 * (double(herm_trace_mul(a, a)) + double(herm_trace_mul(b, b)));
-        const double t = 4.0 * double(herm_trace_mul(a, b));
-        sums[1][threadIdx.x] += k == 1 ? -t : t;
+        double e, t;
+        clover_pair(u, hf, g, s, c, k, e, t);
+        sums[0][threadIdx.x] += e;
+        sums[1][threadIdx.x] += t;
     }
     const int share = (nplaq + int(gridDim.x) - 1) / int(gridDim.x);
     double p = 0.0, energy = sums[0][threadIdx.x], topc = sums[1][threadIdx.x];
