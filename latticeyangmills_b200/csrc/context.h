@@ -8,11 +8,13 @@
 
 #include "api_util.h"
 #include "kernels.h"
+#include "transfer.h"
 #include "ymflow.h"
 
 using ym::Geo;
 
 struct ymflow_ctx {
+    ym::TransferUser transfers;
     int dims[4] = {0, 0, 0, 0};
     int prec = 0;
     int device = 0;

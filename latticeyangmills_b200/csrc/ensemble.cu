@@ -23,6 +23,7 @@
 #include "api_util.h"
 #include "flow_tile.cuh"
 #include "observables.cuh"
+#include "transfer.h"
 #include "ymflow.h"
 
 namespace ym {
@@ -654,6 +655,7 @@ struct EnsGraph {
 };
 
 struct ymflow_ens {
+    TransferUser transfers;
     int nconf = 0;
     int prec = 0;
     int device = 0;
@@ -1199,8 +1201,7 @@ int ymflow_ensemble_upload(ymflow_ens* e, int conf, const double* links) {
         if (r != YMFLOW_OK) return r;
     }
     const EnsConf& C = e->confs[conf];
-    YE_CK(e, cudaMemcpyAsync(e->staging, links, size_t(C.g.V) * 72 * sizeof(double), cudaMemcpyHostToDevice,
-                             e->stream),
+    YE_CK(e, transfer_upload(e->device, e->staging, links, size_t(C.g.V) * 72 * sizeof(double), e->stream),
           "upload copy");
     YE_CK(e, launch_pack(e->prec, e->staging, conf_links(e, conf), C.g, e->stream), "pack");
     YE_CK(e, cudaStreamSynchronize(e->stream), "upload");
@@ -1218,8 +1219,7 @@ int ymflow_ensemble_download(ymflow_ens* e, int conf, double* links) {
     }
     const EnsConf& C = e->confs[conf];
     YE_CK(e, launch_unpack(e->prec, conf_links(e, conf), e->staging, C.g, e->stream), "unpack");
-    YE_CK(e, cudaMemcpyAsync(links, e->staging, size_t(C.g.V) * 72 * sizeof(double), cudaMemcpyDeviceToHost,
-                             e->stream),
+    YE_CK(e, transfer_download(e->device, links, e->staging, size_t(C.g.V) * 72 * sizeof(double), e->stream),
           "download copy");
     YE_CK(e, cudaStreamSynchronize(e->stream), "download");
     return YMFLOW_OK;

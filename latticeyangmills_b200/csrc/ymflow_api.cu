@@ -644,7 +644,7 @@ int ymflow_upload_sites(ymflow_ctx* c, const double* links, int64_t first_site, 
     const size_t bytes = size_t(nsites) * 4 * 18 * sizeof(double);
     r = ensure_staging(c, bytes);
     if (r != YMFLOW_OK) return r;
-    YM_CK(c, cudaMemcpyAsync(c->staging, links, bytes, cudaMemcpyHostToDevice, c->stream), "upload copy");
+    YM_CK(c, transfer_upload(c->device, c->staging, links, bytes, c->stream), "upload copy");
     YM_CK(c, launch_pack_range(c->prec, c->staging, c->u[c->cur], c->geo, c->geo.site0 + int(first_site), int(nsites),
                                (flags & YMFLOW_IO_BIG_ENDIAN) != 0, c->stream),
           "pack launch");
@@ -669,7 +669,7 @@ int ymflow_download_sites(ymflow_ctx* c, double* links, int64_t first_site, int6
                                  int(nsites),
                                  (flags & YMFLOW_IO_BIG_ENDIAN) != 0, c->stream),
           "unpack launch");
-    YM_CK(c, cudaMemcpyAsync(links, c->staging, bytes, cudaMemcpyDeviceToHost, c->stream), "download copy");
+    YM_CK(c, transfer_download(c->device, links, c->staging, bytes, c->stream), "download copy");
     YM_CK(c, cudaStreamSynchronize(c->stream), "download");
     return YMFLOW_OK;
 }
@@ -829,8 +829,7 @@ int ymflow_derivative(ymflow_ctx* c, int mu, double* z_host) {
     int r = ensure_staging(c);
     if (r != YMFLOW_OK) return r;
     YM_CK(c, launch_force(c->prec, mu, c->u[c->cur], c->geo, c->staging, c->stream), "force launch");
-    YM_CK(c, cudaMemcpyAsync(z_host, c->staging, size_t(c->geo.V) * 18 * sizeof(double), cudaMemcpyDeviceToHost,
-                             c->stream),
+    YM_CK(c, transfer_download(c->device, z_host, c->staging, size_t(c->geo.V) * 18 * sizeof(double), c->stream),
           "force copy");
     YM_CK(c, cudaStreamSynchronize(c->stream), "derivative");
     return YMFLOW_OK;
