@@ -51,55 +51,47 @@ __device__ __forceinline__ float ch_small_c1<float>() { return 1e-20f; }
 
 // The same coefficients from the power series of e^{iQ}, for small Q.  By the
 // Cayley-Hamilton theorem Q^3 = c1 Q + c0, so every power reduces to
-// Q^n = A_n + B_n Q + C_n Q^2 with the real recursion
-//   A_{n+1} = c0 C_n,   B_{n+1} = A_n + c1 C_n,   C_{n+1} = B_n,
+// Q^n = A_n + B_n Q + C_n Q^2 with A_n = c0 C_{n-1}, B_n = C_{n+1} and
+//   C_2 = 1, C_3 = 0, C_4 = c1, C_5 = c0, C_6 = c1^2, C_7 = 2 c0 c1,
+//   C_8 = c1^3 + c0^2, C_9 = 3 c0 c1^2, C_10 = c1^4 + 3 c0^2 c1,
+//   C_11 = 4 c0 c1^3 + c0^3, C_12 = c1^5 + 6 c0^2 c1^2,
 // and f_j = sum_n i^n {A,B,C}_n / n!.  Truncating after Q^N is truncating
 // the series of e^{iQ} itself: the error is below rho^{N+1}/(N+1)! e^rho with
 // rho the largest |eigenvalue| of Q, rho^2 <= 4 c1 / 3.  No transcendental
 // function, no division and no cancellation: every term is a small correction
-// to (1, i, -1/2), and f0 - 1 is the sum of the terms alone.
-template <class S, int N>
-__device__ __forceinline__ ChCoef<S> ch_series(S c0, S c1) {
-    ChCoef<S> f;
-    f.f0m1 = cx(S(0), S(0));
-    f.f1 = cx(S(0), S(1));
-    f.f2 = cx(S(-0.5), S(0));
-    S a = S(0), b = S(0), c = S(0.5);  // A_2/2!, B_2/2!, C_2/2!
-#pragma unroll
-    for (int n = 3; n <= N; n++) {
-        const S inv = S(1.0 / n);
-        const S na = mul_rn(mul_rn(c0, c), inv);
-        const S nb = mul_rn(fma(c1, c, a), inv);
-        const S nc = mul_rn(b, inv);
-        a = na;
-        b = nb;
-        c = nc;
-        switch (n & 3) {  // i^n
-            case 0: f.f0m1.re += a; f.f1.re += b; f.f2.re += c; break;
-            case 1: f.f0m1.im += a; f.f1.im += b; f.f2.im += c; break;
-            case 2: f.f0m1.re -= a; f.f1.re -= b; f.f2.re -= c; break;
-            default: f.f0m1.im -= a; f.f1.im -= b; f.f2.im -= c; break;
-        }
-    }
-    return f;
-}
-
+// to (1, i, -1/2), and f0 - 1 is the sum of the terms alone.  Collected by
+// coefficient: 11 operations in FP32 and 34 in FP64, against 32 and 72 for the
+// recursion term by term.
+//
 // Where the series replaces the closed form: c1 <= YM_SERIES_C1, i.e. every
 // eigenvalue of Q within rho <= sqrt(4 YM_SERIES_C1 / 3) = 0.163 of zero.  The
 // flow stays far inside it (eps Z at eps = 0.02 has c1 <= 0.011 on the
 // benchmark fields, Haar-mixed included).  Terms: FP64 up to Q^11 (truncation
 // below 0.163^12/12! = 7e-19), FP32 up to Q^6 (below 0.163^7/7! = 2e-9).
 #define YM_SERIES_C1 0.02
-template <class S>
-struct SeriesTerms;
-template <>
-struct SeriesTerms<double> {
-    static constexpr int value = 11;
-};
-template <>
-struct SeriesTerms<float> {
-    static constexpr int value = 6;
-};
+
+__device__ __forceinline__ ChCoef<float> ch_series(float c0, float c1) {
+    ChCoef<float> f;
+    f.f0m1 = cx(mul_rn(mul_rn(c0, c0), -1.f / 720.f), mul_rn(c0, fmaf(c1, 1.f / 120.f, -1.f / 6.f)));
+    f.f1 = cx(mul_rn(c0, fmaf(c1, -1.f / 360.f, 1.f / 24.f)), fmaf(c1, fmaf(c1, 1.f / 120.f, -1.f / 6.f), 1.f));
+    f.f2 = cx(fmaf(c1, fmaf(c1, -1.f / 720.f, 1.f / 24.f), -0.5f), mul_rn(c0, 1.f / 120.f));
+    return f;
+}
+
+__device__ __forceinline__ ChCoef<double> ch_series(double c0, double c1) {
+    constexpr double k4 = 1.0 / 24, k5 = 1.0 / 120, k6 = 1.0 / 720, k7 = 1.0 / 5040, k8 = 1.0 / 40320,
+                     k9 = 1.0 / 362880, k10 = 1.0 / 3628800, k11 = 1.0 / 39916800;
+    const double q = mul_rn(c0, c0), p = mul_rn(c1, c1), c3 = mul_rn(c1, p);
+    const double s8 = c3 + q, s10 = mul_rn(c1, fma(3.0, q, c3)), s11 = fma(4.0, c3, q), s12 = mul_rn(p, fma(6.0, q, c3));
+    ChCoef<double> f;
+    f.f0m1 = cx(mul_rn(q, fma(-3.0 * k10, p, fma(2.0 * k8, c1, -k6))),
+                mul_rn(c0, fma(-k11, s10, fma(k9, s8, fma(-k7, p, fma(k5, c1, -1.0 / 6))))));
+    f.f1 = cx(mul_rn(c0, fma(-k10, s11, fma(3.0 * k8, p, fma(-2.0 * k6, c1, k4)))),
+              fma(-k11, s12, fma(k9, s10, fma(-k7, s8, fma(k5, p, fma(-1.0 / 6, c1, 1.0))))));
+    f.f2 = cx(fma(-k10, s10, fma(k8, s8, fma(-k6, p, fma(k4, c1, -0.5)))),
+              mul_rn(c0, fma(-k11, s11, fma(3.0 * k9, p, fma(-2.0 * k7, c1, k5)))));
+    return f;
+}
 
 // Cayley-Hamilton coefficients from c0 = det Q and c1 = tr(Q^2)/2, in type S.
 template <class S>
@@ -158,15 +150,27 @@ struct QSquared {  // Q^2, Hermitian: real diagonal and the upper triangle
 
 // (every multiply-add below is written out, so that kernels sharing this code
 // round alike)
+//
+// |q01|^2, |q02|^2, |q12|^2: shared by Q^2, c0 and c1.
 template <class R>
-__device__ __forceinline__ QSquared<R> q_squared(const Herm8<R>& q, R q22) {
+struct OffNorms {
+    R n01, n02, n12;
+};
+template <class R>
+__device__ __forceinline__ OffNorms<R> off_norms(const Herm8<R>& q) {
+    OffNorms<R> n;
+    n.n01 = fma(q.z01.re, q.z01.re, mul_rn(q.z01.im, q.z01.im));
+    n.n02 = fma(q.z02.re, q.z02.re, mul_rn(q.z02.im, q.z02.im));
+    n.n12 = fma(q.z12.re, q.z12.re, mul_rn(q.z12.im, q.z12.im));
+    return n;
+}
+
+template <class R>
+__device__ __forceinline__ QSquared<R> q_squared(const Herm8<R>& q, R q22, const OffNorms<R>& n) {
     QSquared<R> s;
-    const R n01 = fma(q.z01.re, q.z01.re, mul_rn(q.z01.im, q.z01.im));
-    const R n02 = fma(q.z02.re, q.z02.re, mul_rn(q.z02.im, q.z02.im));
-    const R n12 = fma(q.z12.re, q.z12.re, mul_rn(q.z12.im, q.z12.im));
-    s.a00 = fma(q.d0, q.d0, n01 + n02);
-    s.a11 = fma(q.d1, q.d1, n01 + n12);
-    s.a22 = fma(q22, q22, n02 + n12);
+    s.a00 = fma(q.d0, q.d0, n.n01 + n.n02);
+    s.a11 = fma(q.d1, q.d1, n.n01 + n.n12);
+    s.a22 = fma(q22, q22, n.n02 + n.n12);
     // (Q^2)_01 = q00 q01 + q01 q11 + q02 conj(q12);  q00 + q11 = -q22
     s.a01 = cx(fma(-q22, q.z01.re, fma(q.z02.re, q.z12.re, mul_rn(q.z02.im, q.z12.im))),
                fma(-q22, q.z01.im, fma(q.z02.im, q.z12.re, -mul_rn(q.z02.re, q.z12.im))));
@@ -177,6 +181,20 @@ __device__ __forceinline__ QSquared<R> q_squared(const Herm8<R>& q, R q22) {
     s.a12 = cx(fma(-q.d0, q.z12.re, fma(q.z01.re, q.z02.re, mul_rn(q.z01.im, q.z02.im))),
                fma(-q.d0, q.z12.im, fma(q.z01.re, q.z02.im, -mul_rn(q.z01.im, q.z02.re))));
     return s;
+}
+
+// c1 = tr(Q^2)/2 = q00^2 + q00 q11 + q11^2 + |q01|^2 + |q02|^2 + |q12|^2 and c0 =
+// det Q, in Q's own type.
+template <class R>
+__device__ __forceinline__ R c1_of(const Herm8<R>& q, R q22, const OffNorms<R>& n) {
+    return fma(-q.d0, q22, fma(q.d1, q.d1, (n.n01 + n.n02) + n.n12));
+}
+template <class R>
+__device__ __forceinline__ R c0_of(const Herm8<R>& q, R q22, const OffNorms<R>& n) {
+    const R pr = fma(q.z01.re, q.z12.re, -mul_rn(q.z01.im, q.z12.im));  // q01 q12
+    const R pi = fma(q.z01.re, q.z12.im, mul_rn(q.z01.im, q.z12.re));
+    const R re3 = fma(pr, q.z02.re, mul_rn(pi, q.z02.im));  // Re(q01 q12 conj(q02))
+    return fma(R(2), re3, fma(q.d0, fma(q.d1, q22, -n.n12), fma(-q.d1, n.n02, -mul_rn(q22, n.n01))));
 }
 
 // det Q for Hermitian Q: q00 q11 q22 + 2 Re(q01 q12 conj(q02)) - q00|q12|^2 - q11|q02|^2 - q22|q01|^2
@@ -203,24 +221,20 @@ __device__ __forceinline__ S herm_c1(const Herm8<R>& q, R q22r) {
 // FP64: near a doubly degenerate spectrum acos loses about half the significand.
 #define YM_DEGENERATE_X 0.98
 
-template <class R>
-__device__ __forceinline__ ChCoef<R> exp_coefficients(const Herm8<R>& q, R q22);
-
-template <>
-__device__ __forceinline__ ChCoef<double> exp_coefficients<double>(const Herm8<double>& q, double q22) {
-    const double c0 = herm_det<double>(q, q22), c1 = herm_c1<double>(q, q22);
-    if (c1 <= YM_SERIES_C1) return ch_series<double, SeriesTerms<double>::value>(c0, c1);
+__device__ __forceinline__ ChCoef<double> exp_coefficients(const Herm8<double>& q, double q22,
+                                                           const OffNorms<double>& n) {
+    const double c0 = c0_of(q, q22, n), c1 = c1_of(q, q22, n);
+    if (c1 <= YM_SERIES_C1) return ch_series(c0, c1);
     return ch_coefficients<double>(c0, c1);
 }
 
 // Mixed path: the FP32 series for small Q; otherwise the FP32 closed form
 // unless the spectrum is nearly degenerate (or tiny), then the closed form in
 // FP64 from the FP32 entries.
-template <>
-__device__ __forceinline__ ChCoef<float> exp_coefficients<float>(const Herm8<float>& q, float q22) {
-    const float c0 = herm_det<float>(q, q22);
-    const float c1 = herm_c1<float>(q, q22);
-    if (c1 <= float(YM_SERIES_C1)) return ch_series<float, SeriesTerms<float>::value>(c0, c1);
+__device__ __forceinline__ ChCoef<float> exp_coefficients(const Herm8<float>& q, float q22, const OffNorms<float>& n) {
+    const float c0 = c0_of(q, q22, n);
+    const float c1 = c1_of(q, q22, n);
+    if (c1 <= float(YM_SERIES_C1)) return ch_series(c0, c1);
     const float c1s = sqrtf(c1);
     const float c0max = c1 * c1s * 0.38490017945975050f;  // 2/(3 sqrt 3)
     const float x = fabsf(c0) / c0max;
@@ -237,8 +251,9 @@ __device__ __forceinline__ ChCoef<float> exp_coefficients<float>(const Herm8<flo
 template <class R>
 __device__ __forceinline__ void exp_iq(const Herm8<R>& q, M3<R>& e) {
     const R q22 = -(q.d0 + q.d1);
-    const ChCoef<R> f = exp_coefficients<R>(q, q22);
-    const QSquared<R> s = q_squared(q, q22);
+    const OffNorms<R> n = off_norms(q);
+    const ChCoef<R> f = exp_coefficients(q, q22, n);
+    const QSquared<R> s = q_squared(q, q22, n);
     // diagonal: 1 + f0m1 + f1 q_ii + f2 (Q^2)_ii  (q_ii and (Q^2)_ii real)
     e.e[0][0] = cx(R(1) + (f.f0m1.re + f.f1.re * q.d0 + f.f2.re * s.a00), f.f0m1.im + f.f1.im * q.d0 + f.f2.im * s.a00);
     e.e[1][1] = cx(R(1) + (f.f0m1.re + f.f1.re * q.d1 + f.f2.re * s.a11), f.f0m1.im + f.f1.im * q.d1 + f.f2.im * s.a11);
@@ -260,8 +275,9 @@ __device__ __forceinline__ void exp_iq(const Herm8<R>& q, M3<R>& e) {
 template <class R>
 __device__ __forceinline__ void expm1_iq_rows2(const Herm8<R>& q, Rows2<R>& e) {
     const R q22 = -(q.d0 + q.d1);
-    const ChCoef<R> f = exp_coefficients<R>(q, q22);
-    const QSquared<R> s = q_squared(q, q22);
+    const OffNorms<R> n = off_norms(q);
+    const ChCoef<R> f = exp_coefficients(q, q22, n);
+    const QSquared<R> s = q_squared(q, q22, n);
     e.e[0][0] = cx(fma(f.f2.re, s.a00, fma(f.f1.re, q.d0, f.f0m1.re)), fma(f.f2.im, s.a00, fma(f.f1.im, q.d0, f.f0m1.im)));
     e.e[1][1] = cx(fma(f.f2.re, s.a11, fma(f.f1.re, q.d1, f.f0m1.re)), fma(f.f2.im, s.a11, fma(f.f1.im, q.d1, f.f0m1.im)));
     // upper entries f1 q_ij + f2 (Q^2)_ij; e10 from the conjugates of q01 and (Q^2)_01
