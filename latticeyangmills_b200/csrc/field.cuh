@@ -122,6 +122,17 @@ struct Geo {
         if (dir > 0) return c[d] == n[d] - 1 ? s - (n[d] - 1) * stride[d] : s + stride[d];
         return c[d] == 0 ? s + (n[d] - 1) * stride[d] : s - stride[d];
     }
+    // what hop adds to a site's index, for every direction
+    __device__ __forceinline__ void steps(const int c[4], int dir, int d[4]) const {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int far = (n[i] - 1) * stride[i];
+            d[i] = dir > 0 ? (c[i] == n[i] - 1 ? -far : stride[i]) : (c[i] == 0 ? far : -stride[i]);
+        }
+    }
+    __device__ __forceinline__ static int pick(const int d[4], int i) {
+        return i == 0 ? d[0] : (i == 1 ? d[1] : (i == 2 ? d[2] : d[3]));
+    }
     // the same with a direction known only at run time (warp-uniform): the
     // coordinate, extent and stride are picked by selects (no dynamic register
     // or parameter indexing, which would go through local memory)

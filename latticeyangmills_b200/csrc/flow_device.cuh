@@ -205,8 +205,10 @@ template <bool RO = true, class F>
 __device__ __forceinline__ Herm8<typename F::Real> plane_generator(const F& u, const Geo& g, int s, const int c[4],
                                                                    int a, int b, typename F::Real* trace = nullptr) {
     using R = typename F::Real;
-    const int s_pa = g.hop_rt(s, g.coord(c, a), a, +1);
-    const int s_pb = g.hop_rt(s, g.coord(c, b), b, +1);
+    int up_step[4];
+    g.steps(c, +1, up_step);
+    const int s_pa = s + g.pick(up_step, a);
+    const int s_pb = s + g.pick(up_step, b);
     // lo = U_a(x) U_b(x+a) and up = U_b(x) U_a(x+b) (P = lo up^+), each
     // through its first two rows: rows 0 and 1 of the left link times the
     // right link; up's row 2 = conj(row0 x row1), and of P only rows 0 and 1
@@ -254,6 +256,8 @@ __device__ __forceinline__ void split_link_update_to(const F& in, const FO& out,
     using R = typename F::Real;
     int c[4];
     g.coords(s, c);
+    int down[4];
+    g.steps(c, -1, down);
     Herm8<R> d;
     d.d0 = d.d1 = R(0);
     d.z01 = d.z02 = d.z12 = cx(R(0), R(0));
@@ -267,7 +271,7 @@ __device__ __forceinline__ void split_link_update_to(const F& in, const FO& out,
         const int nu = k + (k >= mu ? 1 : 0);
         const int p = mu < nu ? plane_index(mu, nu) : plane_index(nu, mu);
         const R sg = mu < nu ? R(1) : R(-1);
-        const int y = g.hop_rt(s, g.coord(c, nu), nu, -1);
+        const int y = s + g.pick(down, nu);
         const M3<R> v = in.template load<RO>(nu, y);
         d = h8_axpy(sg, (RO ? hf.load_ro(p, s) : hf.load(p, s)), d);
         herm_conj_add(v, h8_scale(-sg, (RO ? hf.load_ro(p, y) : hf.load(p, y))), d);
