@@ -145,10 +145,10 @@ __device__ __forceinline__ M3<typename F::Real> staple_part(const F& u, const Ge
         const int s_mn = g.hop_rt(s, cnu, nu, -1);
         const int s_pm_mn = g.hop_rt(s_mn, cmu, mu, +1);
         M3<R> t;
-        mmul<false, true>(u.load(nu, s_pm), u.load(mu, s_pn), t);
-        mmul_acc<false, true>(t, u.load(nu, s), omega);
-        mmul<true, true>(u.load(nu, s_pm_mn), u.load(mu, s_mn), t);
-        mmul_acc<false, false>(t, u.load(nu, s_mn), omega);
+        mmul<false, true>(u.template load<false>(nu, s_pm), u.template load<false>(mu, s_pn), t);
+        mmul_acc<false, true>(t, u.template load<false>(nu, s), omega);
+        mmul<true, true>(u.template load<false>(nu, s_pm_mn), u.template load<false>(mu, s_mn), t);
+        mmul_acc<false, false>(t, u.template load<false>(nu, s_mn), omega);
     }
     return omega;
 }
@@ -206,6 +206,7 @@ __global__ void __launch_bounds__(kMetroThreads, 5)
     using R = typename F::Real;
     __shared__ Cx<R> links[9][kMetroThreads];
     const int h2 = 2 * (int(blockIdx.x) * blockDim.x + threadIdx.x);
+    grid_wait();
     unsigned acc = 0;
     if (h2 < g.V) {
         int c[4];
@@ -216,7 +217,7 @@ __global__ void __launch_bounds__(kMetroThreads, 5)
         M3<R> W;
         {
             const M3<R> A = staple_part(u, g, s, c, mu, 0, 1);
-            const M3<R> U = u.load(mu, s);
+            const M3<R> U = u.template load<false>(mu, s);
             mmul<false, false>(U, A, W);
 #pragma unroll
             for (int e = 0; e < 9; e++) links[e][threadIdx.x] = U.e[e / 3][e % 3];
@@ -242,6 +243,7 @@ __global__ void __launch_bounds__(kMetroThreads, 5)
                 acc++;
             }
         }
+        grid_release();
         if (acc) {
             M3<R> U;
 #pragma unroll
@@ -263,7 +265,7 @@ __global__ void __launch_bounds__(kMetroThreads, 5)
 //
 // For lattices that leave schedulers without a warp (launch_metro_typed).
 template <class F, int G>
-__global__ void __launch_bounds__(kMetroThreads, 8)
+__global__ void __launch_bounds__(kMetroThreads, 6)
     metropolis_lanes_kernel(F u, Geo g, int mu, int parity, double beta_3, double eps, double x0, int hits,
                             uint64_t seed, uint32_t sweep, unsigned long long* accepted) {
     using R = typename F::Real;
@@ -271,6 +273,7 @@ __global__ void __launch_bounds__(kMetroThreads, 8)
     const int lane = int(threadIdx.x & 31), j = lane & (G - 1), slot = int(threadIdx.x) / G;
     const int h2 = 2 * (int(blockIdx.x) * (kMetroThreads / G) + slot);
     const bool link = h2 < g.V;
+    grid_wait();
     unsigned acc = 0;
     M3<R> W, M;  // M: W in lane 0 of the link, U in the others
     mzero(W);
@@ -282,7 +285,7 @@ __global__ void __launch_bounds__(kMetroThreads, 8)
         s = h2 + odd;
         c[0] += odd;
         W = staple_part(u, g, s, c, mu, j, G);
-        M = u.load(mu, s);
+        M = u.template load<false>(mu, s);
     }
 #pragma unroll
     for (int o = 1; o < G; o <<= 1)
@@ -336,6 +339,7 @@ __global__ void __launch_bounds__(kMetroThreads, 8)
         h = mine ? h + first + 1 : h + G;
     }
     acc = __shfl_sync(0xffffffffu, acc, lane & ~(G - 1));
+    grid_release();
     if (link && j == 1 && acc) u.store(mu, s, M);
     if (j != 0) acc = 0;
     // warp sum, one atomic per warp
@@ -351,15 +355,14 @@ cudaError_t launch_metro_typed(void* u, const Geo& g, int mu, int parity, double
     const double x0 = std::sqrt(std::fma(-eps, eps, 1.0));
     auto launch = [&](auto kernel, unsigned lanes) {
         const unsigned per_block = kMetroThreads / lanes;
-        kernel<<<(links + per_block - 1) / per_block, kMetroThreads, 0, st>>>(F{u, g.V}, g, mu, parity, beta / 3.0, eps,
-                                                                              x0, hits, seed, sweep, accepted);
-        return cudaGetLastError();
+        return launch_chained(true, kernel, (links + per_block - 1) / per_block, kMetroThreads, st, F{u, g.V}, g, mu,
+                              parity, beta / 3.0, eps, x0, hits, seed, sweep, accepted);
     };
     // One thread per link needs about 15,000 links (three warps on each of the
     // SM's schedulers, in all 148 SMs) before its work rather than its chain of
     // hits sets the time; fewer links are given more lanes.  us per launch on
-    // B200 (FP64, 30 hits) at 1 / 4 / 8 lanes: 6^4 30 / 17 / 14, 8^4 31 / 17 /
-    // 15, 12^4 33 / 28 / 34, 16^4 53 / 62 / 77 (2 lanes are never the fastest).
+    // B200 (FP64, 30 hits) at 1 / 4 / 8 lanes: 6^4 30 / 16 / 12, 8^4 31 / 16 /
+    // 14, 12^4 33 / 27 / 32, 16^4 53 / 60 / 75 (2 lanes are never the fastest).
     if (links <= 4736) return launch(metropolis_lanes_kernel<F, 8>, 8);
     if (links <= 14208) return launch(metropolis_lanes_kernel<F, 4>, 4);
     return launch(metropolis_kernel<F>, 1);
