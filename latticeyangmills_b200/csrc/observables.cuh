@@ -257,20 +257,20 @@ __global__ void __launch_bounds__(kObsThreads, kObsMinBlocks)
 // of four links (about 1000).  Bound by latency and arithmetic (FP64 pipe at
 // about 53 %), not by HBM.  A measured step at 32^4 on B200 spends, beyond its
 // six stage launches, 0.28 ms in FP64 (observables_kernel: 0.78), 0.15 in
-// FP32-18 (0.41) and 0.15 in FP32-12 (0.45): this kernel 0.245 / 0.137 / 0.139,
+// FP32-18 (0.41) and 0.15 in FP32-12 (0.45): this kernel 0.250 / 0.135 / 0.135,
 // the sums in the field kernel 0.023 / 0.009 / 0.007 (the field itself is the
 // next stage's), the fold 0.005.
 // ---------------------------------------------------------------------------
+// (down: Geo::steps of the site in the negative directions)
 template <class F>
 __device__ __forceinline__ Herm8<typename F::Real> clover_generator(const F& u,
                                                                     const ForceField<typename F::Real>& hf,
-                                                                    const Geo& g, int s, const int c[4], int mu,
+                                                                    const Geo& g, int s, const int down[4], int mu,
                                                                     int nu) {
     using R = typename F::Real;
     const int p = plane_index(mu, nu);
-    const int s_mm = g.hop_rt(s, g.coord(c, mu), mu, -1);
-    const int s_mn = g.hop_rt(s, g.coord(c, nu), nu, -1);
-    const int s_mm_mn = g.hop_rt(s_mm, g.coord(c, nu), nu, -1);
+    const int d_mu = g.pick(down, mu), d_nu = g.pick(down, nu);
+    const int s_mm = s + d_mu, s_mn = s + d_nu, s_mm_mn = s_mm + d_nu;
     Herm8<R> back = hf.load_ro(p, s_mm);
     herm_conj_add(u.load(nu, s_mm_mn), hf.load_ro(p, s_mm_mn), back);
     Herm8<R> sum = hf.load_ro(p, s);
@@ -292,8 +292,10 @@ __device__ __forceinline__ R herm_trace_mul(const Herm8<R>& a, const Herm8<R>& b
 template <class F>
 __device__ __forceinline__ void clover_pair(const F& u, const ForceField<typename F::Real>& hf, const Geo& g, int s,
                                             const int c[4], int k, double& energy, double& topc) {
-    const auto a = clover_generator(u, hf, g, s, c, 0, k + 1);
-    const auto b = clover_generator(u, hf, g, s, c, k == 0 ? 2 : 1, k == 2 ? 2 : 3);
+    int down[4];
+    g.steps(c, -1, down);
+    const auto a = clover_generator(u, hf, g, s, down, 0, k + 1);
+    const auto b = clover_generator(u, hf, g, s, down, k == 0 ? 2 : 1, k == 2 ? 2 : 3);
     // Re tr(G_a G_b) = -4 tr(S_a S_b); the pairs' signs as in site_observables
     energy = -4.0 * (double(herm_trace_mul(a, a)) + double(herm_trace_mul(b, b)));
     const double t = 4.0 * double(herm_trace_mul(a, b));
@@ -301,10 +303,12 @@ __device__ __forceinline__ void clover_pair(const F& u, const ForceField<typenam
 }
 
 // Resident 96-thread blocks: FP64 5 (128 registers, 15 warps per SM; a plane
-// pair with one transport live needs all of them), FP32 10 (64, 30 warps).
+// pair with one transport live needs all of them; 6 and 7 spill: 0.30 and 0.52
+// ms), FP32 8 (80, 24 warps: 0.135 ms at 32^4, against 0.139-0.141 at 10 and
+// 0.16 at 12).
 template <class F>
 struct CloverMinBlocks {
-    static constexpr int value = sizeof(typename F::Real) == 8 ? 5 : 10;
+    static constexpr int value = sizeof(typename F::Real) == 8 ? 5 : 8;
 };
 
 // One thread per (site, pair of planes): the pairs (01,23), (02,13), (03,12)
