@@ -260,10 +260,6 @@ struct LinkField<double, NE> {
         if (NE == 6) reconstruct_row2(a);
         return a;
     }
-    __device__ __forceinline__ void put(int mu, int e, int s, Cx<double> v) const {
-        double2* q = const_cast<double2*>(link(mu, s)) + 32 * e;
-        *q = make_double2(v.re, v.im);
-    }
     __device__ __forceinline__ void store(int mu, int s, const M3<double>& a) const {
         double2* q = const_cast<double2*>(link(mu, s));
 #pragma unroll

@@ -236,15 +236,6 @@ __device__ __forceinline__ Herm8<typename F::Real> plane_generator(const F& u, c
     return force_from_b2_cdag(lo, up, trace);
 }
 
-// H_p(x) of plane p at site s into hf.
-template <class F>
-__device__ __forceinline__ void plaq_plane(const F& u, const ForceField<typename F::Real>& hf, const Geo& g, int s,
-                                           int p) {
-    int c[4];
-    g.coords(s, c);
-    hf.store(p, s, plane_generator(u, g, s, c, plane_a(p), plane_b(p)));
-}
-
 // One link through one stage with its generator built from the plane field hf
 // (which holds the plane generators of `in`); HALO: a slab's boundary links
 // also go into its neighbours' halos, as in rk_link_update_to.

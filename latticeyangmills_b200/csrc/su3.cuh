@@ -100,33 +100,8 @@ __device__ __forceinline__ void mzero(M3<R>& a) {
 }
 
 template <class R>
-__device__ __forceinline__ void madd(M3<R>& a, const M3<R>& b) {
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            a.e[i][j].re += b.e[i][j].re;
-            a.e[i][j].im += b.e[i][j].im;
-        }
-}
-
-template <class R>
 __device__ __forceinline__ R re_trace(const M3<R>& a) {
     return a.e[0][0].re + a.e[1][1].re + a.e[2][2].re;
-}
-
-// Re tr(a * b) and Re tr(a * b^+) without forming the product.
-template <class R>
-__device__ __forceinline__ R re_trace_mul(const M3<R>& a, const M3<R>& b) {
-    R s = R(0);
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            s = fma(a.e[i][k].re, b.e[k][i].re, s);
-            s = fma(-a.e[i][k].im, b.e[k][i].im, s);
-        }
-    return s;
 }
 
 // Entry k of row 2 of the SU(3) matrix whose rows 0 and 1 are those of a
@@ -259,26 +234,12 @@ __device__ __forceinline__ R mul_diag_im(const M3<R>& u, const M3<R>& w, int i) 
     return im;
 }
 
-// Flow generator from X = U * Omega (Omega the staple sum):
+// Flow generator of X = U Omega (Omega the staple sum):
 //   Z = (i/2) [X - X^+]_traceless   (Hermitian, traceless),
 // the quantity the reference returns from PureGauge::computeDerivative
-// (src/Actions/puregauge.cpp:62-79, where X is formed as (Omega^+ U^+)^+).
-template <class R>
-__device__ __forceinline__ Herm8<R> force_from_x(const M3<R>& x) {
-    Herm8<R> z;
-    const R i0 = x.e[0][0].im, i1 = x.e[1][1].im, i2 = x.e[2][2].im;
-    const R mean = (i0 + i1 + i2) * R(1.0 / 3.0);
-    z.d0 = mean - i0;
-    z.d1 = mean - i1;
-    // (i/2)(a + ib) = (-b/2, a/2) with a + ib = X_ij - conj(X_ji)
-    z.z01 = cx(R(-0.5) * (x.e[0][1].im + x.e[1][0].im), R(0.5) * (x.e[0][1].re - x.e[1][0].re));
-    z.z02 = cx(R(-0.5) * (x.e[0][2].im + x.e[2][0].im), R(0.5) * (x.e[0][2].re - x.e[2][0].re));
-    z.z12 = cx(R(-0.5) * (x.e[1][2].im + x.e[2][1].im), R(0.5) * (x.e[1][2].re - x.e[2][1].re));
-    return z;
-}
-
-// The same generator from U and Omega without forming X: only the six
-// off-diagonal entries and the imaginary diagonal of U * Omega are computed.
+// (src/Actions/puregauge.cpp:62-79, where X is formed as (Omega^+ U^+)^+).  Only
+// the six off-diagonal entries and the imaginary diagonal of X are computed:
+// (i/2)(a + ib) = (-b/2, a/2) with a + ib = X_ij - conj(X_ji).
 template <class R>
 __device__ __forceinline__ Herm8<R> force_from_u_omega(const M3<R>& u, const M3<R>& w) {
     Herm8<R> z;
@@ -295,46 +256,8 @@ __device__ __forceinline__ Herm8<R> force_from_u_omega(const M3<R>& u, const M3<
     return z;
 }
 
-// The generator (i/2)[X - X^+]_traceless of X = B C^+ without forming X: the
-// six off-diagonal entries and the imaginary diagonal of B C^+.
-template <class R>
-__device__ __forceinline__ Herm8<R> force_from_b_cdag(const M3<R>& b, const M3<R>& c) {
-    auto entry = [&](int i, int j) {  // (B C^+)_ij = sum_k b_ik conj(c_jk)
-        R re = R(0), im = R(0);
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            re = fma(b.e[i][k].re, c.e[j][k].re, re);
-            re = fma(b.e[i][k].im, c.e[j][k].im, re);
-            im = fma(b.e[i][k].im, c.e[j][k].re, im);
-            im = fma(-b.e[i][k].re, c.e[j][k].im, im);
-        }
-        return cx(re, im);
-    };
-    auto diag_im = [&](int i) {
-        R im = R(0);
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            im = fma(b.e[i][k].im, c.e[i][k].re, im);
-            im = fma(-b.e[i][k].re, c.e[i][k].im, im);
-        }
-        return im;
-    };
-    Herm8<R> z;
-    const R i0 = diag_im(0), i1 = diag_im(1), i2 = diag_im(2);
-    const R mean = (i0 + i1 + i2) * R(1.0 / 3.0);
-    z.d0 = mean - i0;
-    z.d1 = mean - i1;
-    const Cx<R> x01 = entry(0, 1), x10 = entry(1, 0);
-    const Cx<R> x02 = entry(0, 2), x20 = entry(2, 0);
-    const Cx<R> x12 = entry(1, 2), x21 = entry(2, 1);
-    z.z01 = cx(R(-0.5) * (x01.im + x10.im), R(0.5) * (x01.re - x10.re));
-    z.z02 = cx(R(-0.5) * (x02.im + x20.im), R(0.5) * (x02.re - x20.re));
-    z.z12 = cx(R(-0.5) * (x12.im + x21.im), R(0.5) * (x12.re - x21.re));
-    return z;
-}
-
-// The same generator of X = B C^+ for X in SU(3), from B's first two rows:
-// rows 0 and 1 of X (six entries), then of row 2 = conj(row0 x row1) only
+// The generator (i/2)[X - X^+]_traceless of X = B C^+ for X in SU(3), from B's
+// first two rows: rows 0 and 1 of X (six entries), then of row 2 = conj(row0 x row1) only
 // X_20, X_21 and Im X_22.  92 multiply-adds, against 90 plus the 27 that
 // rebuild B's row 2 for the full form.  trace (optional): Re tr X, for four
 // more.
