@@ -188,160 +188,130 @@ __device__ __forceinline__ double propose(uint32_t l0, uint32_t l1, uint32_t swe
     return beta_3 * double(dtr);
 }
 
-// One thread per link of the (mu, parity) class; link h's site is the one of
-// that parity in the x pair (2h, 2h + 1) (extents are even).  The trace change
-// of a proposal needs W = U A only, so U (kept in shared memory) and W are
-// multiplied by X only when it is accepted.
+// G lanes per link of the (mu, parity) class (1, 4 or 8); link h's site is the
+// one of that parity in the x pair (2h, 2h + 1) (extents are even).  The lanes
+// of a link share its staples, then draw the next G proposals against the same
+// link, one each; the first accepted one is taken and the later ones are drawn
+// again from the new link, so the chain is that of one proposal after another.
+// The trace change of a proposal needs W = U A only, so U and W are multiplied
+// by X only when it is accepted.
 //
-// Bound by the chain of a hit (some 600 FP64 and integer instructions, one
-// issued every 3 to 4 cycles per warp; FP64 pipe at 42 %).  16^4, 30 hits, FP64
-// on B200: 53 us per launch, 32^4 0.58 ms, against 153 us and 2.4 ms with one
-// thread per site, half of them idle, and every proposal multiplied out as
-// dense matrices.  Two or three proposals per thread at a time (all but the
-// first accepted one discarded) gained nothing: 52 and 55 us.
-template <class F>
-__global__ void __launch_bounds__(kMetroThreads, 5)
+// One proposal in nine is accepted (eps = 0.24), so nearly every hit some links
+// of a warp have two 3x3 products to do and most have none.  U, W and the
+// accepted X stand in shared memory and the warp does the products together:
+// six lanes per accepted link, each a column of X U or X W, five links at a
+// time.
+//
+// Bound by the chain of a hit and the few warps that 168 registers (FP64) and
+// a small lattice's links leave.  FP64, 30 hits, per launch on B200, before
+// (each thread multiplying its own link) and now: 12^4 (4 lanes) 27.0 -> 24.1
+// us, 16^4 53.0 -> 47.6, 24^4 206 -> 184, 32^4 600 -> 525; FP32-12 16^4 37.9 ->
+// 37.1, 32^4 458 -> 386.  (One thread per site, half of them idle, and dense
+// products for every proposal: 16^4 153 us, 32^4 2.4 ms.)  Two or three
+// proposals per thread at a time gained nothing, nor did drawing the next hit's
+// X during this one's test (16^4 47.9 us, 24^4 225), reading W's triangle
+// instead of forming X^+ (48.1, 184) or 7 blocks per SM (53, 210).
+template <class F, int G>
+__global__ void __launch_bounds__(kMetroThreads, G == 1 ? 5 : 6)
     metropolis_kernel(F u, Geo g, int mu, int parity, double beta_3, double eps, double x0, int hits, uint64_t seed,
                       uint32_t sweep, unsigned long long* accepted) {
     using R = typename F::Real;
-    __shared__ Cx<R> links[9][kMetroThreads];
-    const int h2 = 2 * (int(blockIdx.x) * blockDim.x + threadIdx.x);
-    grid_wait();
-    unsigned acc = 0;
-    if (h2 < g.V) {
-        int c[4];
-        g.coords(h2, c);
-        const int odd = (c[1] + c[2] + c[3] + parity) & 1;
-        const int s = h2 + odd;
-        c[0] += odd;
-        M3<R> W;
-        {
-            const M3<R> A = staple_part(u, g, s, c, mu, 0, 1);
-            const M3<R> U = u.template load<false>(mu, s);
-            mmul<false, false>(U, A, W);
-#pragma unroll
-            for (int e = 0; e < 9; e++) links[e][threadIdx.x] = U.e[e / 3][e % 3];
-        }
-        const uint64_t l = uint64_t(s) * 4 + uint64_t(mu);
-        const uint32_t l0 = uint32_t(l), l1 = uint32_t(l >> 32);
-        const uint2 key = make_uint2(uint32_t(seed), uint32_t(seed >> 32) ^ 0x4D455452u);
-        for (int h = 0; h < hits; h++) {
-            M3<R> X;
-            uint32_t draw;
-            const double x = propose(l0, l1, sweep, uint32_t(h), key, eps, x0, beta_3, W, X, draw);
-            int ok = exp_exceeds_fp32(x, draw);
-            if (ok < 0) ok = exp(x) > unit(draw);
-            if (ok) {
-                M3<R> U, t;
-#pragma unroll
-                for (int e = 0; e < 9; e++) U.e[e / 3][e % 3] = links[e][threadIdx.x];
-                mmul<false, false>(X, U, t);
-#pragma unroll
-                for (int e = 0; e < 9; e++) links[e][threadIdx.x] = t.e[e / 3][e % 3];
-                mmul<false, false>(X, W, t);
-                W = t;
-                acc++;
-            }
-        }
-        grid_release();
-        if (acc) {
-            M3<R> U;
-#pragma unroll
-            for (int e = 0; e < 9; e++) U.e[e / 3][e % 3] = links[e][threadIdx.x];
-            u.store(mu, s, U);
-        }
-    }
-    // warp sum, one atomic per warp
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0 && acc) atomicAdd(accepted, (unsigned long long)acc);
-}
-
-// The same with G lanes per link.  The lanes of a link share its staples, then draw the next G
-// proposals against the same W, one each; the first accepted one is taken and
-// the later ones are drawn again from the new link, so the chain is that of
-// one proposal after another.  X passes through shared memory; the first lane
-// then multiplies W, the others U (one multiplication in the warp).
-//
-// For lattices that leave schedulers without a warp (launch_metro_typed).
-template <class F, int G>
-__global__ void __launch_bounds__(kMetroThreads, 6)
-    metropolis_lanes_kernel(F u, Geo g, int mu, int parity, double beta_3, double eps, double x0, int hits,
-                            uint64_t seed, uint32_t sweep, unsigned long long* accepted) {
-    using R = typename F::Real;
-    __shared__ Cx<R> shared[9][kMetroThreads / G];  // a link's accepted X, then its new W
+    constexpr int kLinks = kMetroThreads / G, kWarpLinks = 32 / G;
+    __shared__ Cx<R> uw[18][kLinks];  // U, then W
+    __shared__ Cx<R> xs[9][kLinks];
+    __shared__ int takers[kLinks];  // the links of a warp that accepted, in order
     const int lane = int(threadIdx.x & 31), j = lane & (G - 1), slot = int(threadIdx.x) / G;
-    const int h2 = 2 * (int(blockIdx.x) * (kMetroThreads / G) + slot);
+    int* const warp_takers = takers + slot / kWarpLinks * kWarpLinks;
+    const int col = (lane % 6) % 3 + ((lane % 6) / 3) * 9;  // this lane's column in uw: entries col, col + 3, col + 6
+    const int h2 = 2 * (int(blockIdx.x) * kLinks + slot);
     const bool link = h2 < g.V;
     grid_wait();
-    unsigned acc = 0;
-    M3<R> W, M;  // M: W in lane 0 of the link, U in the others
-    mzero(W);
     int s = 0;
-    if (link) {
-        int c[4];
-        g.coords(h2, c);
-        const int odd = (c[1] + c[2] + c[3] + parity) & 1;
-        s = h2 + odd;
-        c[0] += odd;
-        W = staple_part(u, g, s, c, mu, j, G);
-        M = u.template load<false>(mu, s);
-    }
-#pragma unroll
-    for (int o = 1; o < G; o <<= 1)
-#pragma unroll
-        for (int e = 0; e < 9; e++) {
-            W.e[e / 3][e % 3].re += __shfl_xor_sync(0xffffffffu, W.e[e / 3][e % 3].re, o);
-            W.e[e / 3][e % 3].im += __shfl_xor_sync(0xffffffffu, W.e[e / 3][e % 3].im, o);
-        }
     {
-        const M3<R> A = W;
-        mmul<false, false>(M, A, W);
-        if (j == 0) M = W;
+        M3<R> U, A, W;
+        mzero(U);
+        mzero(A);
+        if (link) {
+            int c[4];
+            g.coords(h2, c);
+            const int odd = (c[1] + c[2] + c[3] + parity) & 1;
+            s = h2 + odd;
+            c[0] += odd;
+            A = staple_part(u, g, s, c, mu, j, G);
+            U = u.template load<false>(mu, s);
+        }
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1)
+#pragma unroll
+            for (int e = 0; e < 9; e++) {
+                A.e[e / 3][e % 3].re += __shfl_xor_sync(0xffffffffu, A.e[e / 3][e % 3].re, o);
+                A.e[e / 3][e % 3].im += __shfl_xor_sync(0xffffffffu, A.e[e / 3][e % 3].im, o);
+            }
+        mmul<false, false>(U, A, W);
+        if (j == 0) {
+#pragma unroll
+            for (int e = 0; e < 9; e++) {
+                uw[e][slot] = U.e[e / 3][e % 3];
+                uw[9 + e][slot] = W.e[e / 3][e % 3];
+            }
+        }
+        __syncwarp();
     }
     const uint64_t l = uint64_t(s) * 4 + uint64_t(mu);
     const uint32_t l0 = uint32_t(l), l1 = uint32_t(l >> 32);
     const uint2 key = make_uint2(uint32_t(seed), uint32_t(seed >> 32) ^ 0x4D455452u);
+    unsigned acc = 0;  // of this lane's proposals
     int h = link ? 0 : hits;
     while (__any_sync(0xffffffffu, h < hits)) {
-        M3<R> X;
+        M3<R> X, W;
+#pragma unroll
+        for (int e = 0; e < 9; e++) W.e[e / 3][e % 3] = uw[9 + e][slot];
         uint32_t draw;
         const double x = propose(l0, l1, sweep, uint32_t(h + j), key, eps, x0, beta_3, W, X, draw);
         int ok = exp_exceeds_fp32(x, draw);
         if (ok < 0) ok = exp(x) > unit(draw);
-        const unsigned all = __ballot_sync(0xffffffffu, ok && h + j < hits);
-        const unsigned mine = (all >> (lane & ~(G - 1))) & ((1u << G) - 1u);
-        const int first = __ffs(int(mine)) - 1;
-        if (j == first) {
-#pragma unroll
-            for (int e = 0; e < 9; e++) shared[e][slot] = X.e[e / 3][e % 3];
+        unsigned taken = __ballot_sync(0xffffffffu, ok && h + j < hits);  // one lane per link that accepts, its first
+        int first = 0;
+        if (G > 1) {
+            const unsigned mine = (taken >> (lane & ~(G - 1))) & ((1u << G) - 1u);
+            first = mine ? __ffs(int(mine)) - 1 : G - 1;
+            taken = __ballot_sync(0xffffffffu, mine && j == first);
         }
-        __syncwarp();
-        if (mine) {
+        if (taken >> lane & 1u) {
 #pragma unroll
-            for (int e = 0; e < 9; e++) X.e[e / 3][e % 3] = shared[e][slot];
-            M3<R> t;
-            mmul<false, false>(X, M, t);
-            M = t;
-        }
-        __syncwarp();
-        if (mine && j == 0) {
+            for (int e = 0; e < 9; e++) xs[e][slot] = X.e[e / 3][e % 3];
+            warp_takers[__popc(taken & ((1u << lane) - 1u))] = slot;
             acc++;
-#pragma unroll
-            for (int e = 0; e < 9; e++) shared[e][slot] = M.e[e / 3][e % 3];
         }
         __syncwarp();
-        if (mine) {
+        for (int r = lane < 30 ? lane / 6 : kWarpLinks; r < __popc(taken); r += 5) {
+            const int o = warp_takers[r];
+            const Cx<R> y[3] = {uw[col][o], uw[col + 3][o], uw[col + 6][o]};
 #pragma unroll
-            for (int e = 0; e < 9; e++) W.e[e / 3][e % 3] = shared[e][slot];
+            for (int i = 0; i < 3; i++) {  // the sums of mmul
+                R re = R(0), im = R(0);
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    const Cx<R> a = xs[3 * i + k][o];
+                    re = fma(a.re, y[k].re, re);
+                    re = fma(-a.im, y[k].im, re);
+                    im = fma(a.re, y[k].im, im);
+                    im = fma(a.im, y[k].re, im);
+                }
+                uw[col + 3 * i][o] = cx(re, im);
+            }
         }
-        __syncwarp();  // read before the next accepted X is written
-        h = mine ? h + first + 1 : h + G;
+        __syncwarp();
+        h += first + 1;
     }
-    acc = __shfl_sync(0xffffffffu, acc, lane & ~(G - 1));
+    const unsigned changed = __ballot_sync(0xffffffffu, acc != 0) >> (lane & ~(G - 1)) & ((1u << G) - 1u);
     grid_release();
-    if (link && j == 1 && acc) u.store(mu, s, M);
-    if (j != 0) acc = 0;
+    if (changed && j == 0) {
+        M3<R> U;
+#pragma unroll
+        for (int e = 0; e < 9; e++) U.e[e / 3][e % 3] = uw[e][slot];
+        u.store(mu, s, U);
+    }
     // warp sum, one atomic per warp
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
@@ -361,11 +331,12 @@ cudaError_t launch_metro_typed(void* u, const Geo& g, int mu, int parity, double
     // One thread per link needs about 15,000 links (three warps on each of the
     // SM's schedulers, in all 148 SMs) before its work rather than its chain of
     // hits sets the time; fewer links are given more lanes.  us per launch on
-    // B200 (FP64, 30 hits) at 1 / 4 / 8 lanes: 6^4 30 / 16 / 12, 8^4 31 / 16 /
-    // 14, 12^4 33 / 27 / 32, 16^4 53 / 60 / 75 (2 lanes are never the fastest).
-    if (links <= 4736) return launch(metropolis_lanes_kernel<F, 8>, 8);
-    if (links <= 14208) return launch(metropolis_lanes_kernel<F, 4>, 4);
-    return launch(metropolis_kernel<F>, 1);
+    // B200 (FP64, 30 hits, each thread multiplying its own link) at 1 / 4 / 8
+    // lanes: 6^4 30 / 16 / 12, 8^4 31 / 16 / 14, 12^4 33 / 27 / 32, 16^4 53 / 60 /
+    // 75 (2 lanes are never the fastest).
+    if (links <= 4736) return launch(metropolis_kernel<F, 8>, 8);
+    if (links <= 14208) return launch(metropolis_kernel<F, 4>, 4);
+    return launch(metropolis_kernel<F, 1>, 1);
 }
 
 }  // namespace

@@ -111,3 +111,21 @@ def test_every_lane_count_runs_the_same_chain(oracle, n, hits):
     acc = oracle.gen_metropolis_cb(U, n, BETA, EPS, 1, hits, 21)
     assert round(frac * hits * 4 * oracle.volume(n)) == acc
     assert np.abs(got - U).max() < 1e-12
+
+
+@pytest.mark.parametrize("n", [(2, 2, 2, 2), (6, 6, 6, 6), (12, 10, 12, 10), (18, 10, 10, 18)], ids=str)
+def test_every_link_of_a_warp_accepting(oracle, n):
+    """beta = 0: all 32, 8 or 4 links of a warp (and those of a partial one) take
+    every proposal, the most products a hit has; the oracle's chain (tolerance
+    as above)."""
+    U = oracle.gen_cold(n)
+    oracle.gen_haar_mix(U, n, 0.3, 13, 0)
+    from latticeyangmills_b200 import GluonField
+
+    with GluonField(n, "fp64") as f:
+        f.upload(U)
+        frac = f.generate_metropolis(0.0, EPS, 1, 5, 21, "current")
+        got = f.download()
+    assert oracle.gen_metropolis_cb(U, n, 0.0, EPS, 1, 5, 21) == 5 * 4 * oracle.volume(n)
+    assert frac == 1.0
+    assert np.abs(got - U).max() < 1e-12
