@@ -84,7 +84,9 @@ int ensure_meas(ymflow_ctx* c, int rows);
 cudaError_t enqueue_stage(ymflow_ctx* c, int stage, const void* in, void* out, double eps);
 // Observables of the current field (the context's sites) into measurement row `row` on the device.
 // rows_in: read rows 0 and 1 of its links only (they were written by a stage).
-int enqueue_measure(ymflow_ctx* c, int row, bool rows_in = false);
+// pending (optional): rows before `row` that are still to be folded; a row
+// measured through the plaquette field may join them (fold_rows).
+int enqueue_measure(ymflow_ctx* c, int row, bool rows_in = false, int* pending = nullptr);
 void fill_obs(const ymflow_ctx* c, const double* m, int64_t step, double t, ymflow_obs* o);
 
 // Slab transport (slab.cu): halo exchange of link buffer u[buf] and the sum of a

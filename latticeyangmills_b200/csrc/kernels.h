@@ -140,22 +140,30 @@ cudaError_t launch_exp(const double* q, double* r, int64_t n, cudaStream_t st);
 int obs_blocks(const Geo& g);
 cudaError_t launch_observables(int prec, const void* u, const Geo& g, double* partials, cudaStream_t st);
 cudaError_t launch_obs_finalize(const double* partials, int nblocks, const Geo& g, double* out, cudaStream_t st,
-                                bool chained = false);
+                                bool chained = false, int rows = 1);
 
-// The same row (out[0..3]) through the plaquette field, in three launches: the
-// field of u over `field`'s sites into h (which then holds u's plaquette field,
-// as after launch_plaq_field) with the plaquette sums, energy and charge from
-// it over `own`'s sites, and the fold.  `partials` holds measure_partials
-// doubles.  The energy and charge kernel's blocks stride over the sites beyond
-// kCloverMaxBlocks.
+// The same row through the plaquette field, in three launches: the field of u
+// over `field`'s sites into h (which then holds u's plaquette field, as after
+// launch_plaq_field) with the plaquette sums, then energy and charge from it
+// over `own`'s sites into slot `slot` of the partials (launch_measure_from_field);
+// the fold of slots 0..rows-1 into out[0..4 rows) (launch_fold_rows).  `partials`
+// holds measure_partials doubles.  The energy and charge kernel's blocks stride
+// over the sites beyond kCloverMaxBlocks.
+//
+// A flow call folds its rows kFoldRows at a time: only the host reads them, at
+// the call's end, and a fold (one block's chain, about 4 us) before the next
+// step would keep that step waiting.
+constexpr int kFoldRows = 16;
 constexpr int kCloverMaxBlocks = 148 * 20;
 int plaq_sum_partials(int prec, const Geo& g);
 cudaError_t launch_plaq_field_sum(int prec, const void* u, void* h, const Geo& g, int count0, int count1,
                                   double* partials, cudaStream_t st, bool rows_in = false, bool chained = false);
 int measure_partials(int prec, const Geo& field, const Geo& own);
 cudaError_t launch_measure_from_field(int prec, const void* u, void* h, const Geo& field, const Geo& own,
-                                      double* partials, double* out, cudaStream_t st, bool rows_in = false,
+                                      double* partials, int slot, cudaStream_t st, bool rows_in = false,
                                       bool chained = false);
+cudaError_t launch_fold_rows(int prec, const Geo& field, const Geo& own, const double* partials, int rows, double* out,
+                             cudaStream_t st, bool chained = false);
 
 // .bin layout (site-major, mu, 18 doubles) <-> device layout
 // Sites [first, first + n) between a .bin-layout block (aos points at site

@@ -25,11 +25,13 @@
 
 namespace ym {
 
-// One block of 1024 threads: thread i folds partials i, i+1024, ... in order,
-// then the block tree.  Output (plaq, topc, energy, nonfinite flag).
+// One block of 1024 threads per row: thread i folds partials i, i+1024, ... in
+// order, then the block tree.  Output (plaq, topc, energy, nonfinite flag).
 __global__ void __launch_bounds__(1024) obs_finalize_kernel(const double* partials, int nblocks, double inv_18v,
                                                             double* out) {
     grid_wait();
+    partials += int64_t(blockIdx.x) * 3 * nblocks;
+    out += 4 * blockIdx.x;
     double a = 0.0, b = 0.0, c = 0.0;
 #pragma unroll 4
     for (int i = threadIdx.x; i < nblocks; i += blockDim.x) {
@@ -65,24 +67,23 @@ cudaError_t launch_observables(int prec, const void* u, const Geo& g, double* pa
 }
 
 cudaError_t launch_obs_finalize(const double* partials, int nblocks, const Geo& g, double* out, cudaStream_t st,
-                                bool chained) {
-    return launch_chained(chained, obs_finalize_kernel, 1, 1024, st, partials, nblocks,
+                                bool chained, int rows) {
+    return launch_chained(chained, obs_finalize_kernel, unsigned(rows), 1024, st, partials, nblocks,
                           1.0 / (18.0 * double(g.vglobal)), out);
 }
 
 template <class F>
 static cudaError_t launch_clover_typed(const void* u, const void* h, const Geo& g, int blocks, const double* plaq,
-                                       int nplaq, double* partials, cudaStream_t st) {
+                                       int nplaq, double* partials, bool chained, cudaStream_t st) {
     const F in{const_cast<void*>(u), g.V};
     const ForceField<typename F::Real> hf{const_cast<void*>(h), g.V};
-    clover_field_kernel<F><<<blocks, 96, 0, st>>>(in, hf, g, plaq, nplaq, partials);
-    return cudaGetLastError();
+    return launch_chained(chained, clover_field_kernel<F>, unsigned(blocks), 96, st, in, hf, g, plaq, nplaq, partials);
 }
 
 static int clover_blocks(const Geo& g) { return std::min((g.site1 - g.site0 + 31) / 32, kCloverMaxBlocks); }
 
 int measure_partials(int prec, const Geo& field, const Geo& own) {
-    return plaq_sum_partials(prec, field) + 3 * clover_blocks(own);
+    return plaq_sum_partials(prec, field) + kFoldRows * 3 * clover_blocks(own);
 }
 
 // Contexts on the two-kernel stage measure this way: the field is needed by
@@ -91,23 +92,28 @@ int measure_partials(int prec, const Geo& field, const Geo& own) {
 // 48 0.55 -> 0.39 ms; below, both are a few launches long (8^4 FP64: 9.3 + 2.9
 // us against 4.9 + 6.7 + 2.9, of which the next step saves the first).
 cudaError_t launch_measure_from_field(int prec, const void* u, void* h, const Geo& field, const Geo& own,
-                                      double* partials, double* out, cudaStream_t st, bool rows_in, bool chained) {
+                                      double* partials, int slot, cudaStream_t st, bool rows_in, bool chained) {
     const int np = plaq_sum_partials(prec, field), nc = clover_blocks(own);
-    if (np < 1 || nc < 1) return cudaErrorInvalidValue;
-    cudaError_t e = launch_plaq_field_sum(prec, u, h, field, own.site0, own.site1, partials, st, rows_in, chained);
+    if (np < 1 || nc < 1 || slot < 0 || slot >= kFoldRows) return cudaErrorInvalidValue;
+    const cudaError_t e =
+        launch_plaq_field_sum(prec, u, h, field, own.site0, own.site1, partials, st, rows_in, chained);
     if (e != cudaSuccess) return e;
-    double* const cp = partials + np;
+    double* const cp = partials + np + int64_t(slot) * 3 * nc;
     switch (prec) {
         case kFP64:
-            e = rows_in ? launch_clover_typed<FieldD18Rows>(u, h, own, nc, partials, np, cp, st)
-                        : launch_clover_typed<FieldD18>(u, h, own, nc, partials, np, cp, st);
-            break;
-        case kFP32_18: e = launch_clover_typed<FieldF18>(u, h, own, nc, partials, np, cp, st); break;
-        case kFP32_12: e = launch_clover_typed<FieldF12>(u, h, own, nc, partials, np, cp, st); break;
+            if (rows_in) return launch_clover_typed<FieldD18Rows>(u, h, own, nc, partials, np, cp, chained, st);
+            return launch_clover_typed<FieldD18>(u, h, own, nc, partials, np, cp, chained, st);
+        case kFP32_18: return launch_clover_typed<FieldF18>(u, h, own, nc, partials, np, cp, chained, st);
+        case kFP32_12: return launch_clover_typed<FieldF12>(u, h, own, nc, partials, np, cp, chained, st);
         default: return cudaErrorInvalidValue;
     }
-    if (e != cudaSuccess) return e;
-    return launch_obs_finalize(cp, nc, own, out, st, chained);
+}
+
+cudaError_t launch_fold_rows(int prec, const Geo& field, const Geo& own, const double* partials, int rows, double* out,
+                             cudaStream_t st, bool chained) {
+    if (rows < 1 || rows > kFoldRows) return cudaErrorInvalidValue;
+    return launch_obs_finalize(partials + plaq_sum_partials(prec, field), clover_blocks(own), own, out, st, chained,
+                               rows);
 }
 
 }  // namespace ym

@@ -259,10 +259,15 @@ __global__ void __launch_bounds__(kObsThreads, kObsMinBlocks)
 // six stage launches, 0.28 ms in FP64 (observables_kernel: 0.78), 0.15 in
 // FP32-18 (0.41) and 0.15 in FP32-12 (0.45): this kernel 0.250 / 0.135 / 0.135,
 // the sums in the field kernel 0.023 / 0.009 / 0.007 (the field itself is the
-// next stage's), the fold 0.005.
+// next stage's).  Launched on the field kernel's heels, with its rows folded
+// later (kFoldRows), a measured step is 4-5 us shorter at every size: 12^4 FP64
+// 52.5 -> 48.5 us, 16^4 FP32-12 71 -> 67, 15 x 13 x 17 x 21 FP64 131.4 -> 126.5.
+// (The field kernel with the sums does not release this one before its end:
+// with a release before its last store FP64 16^3 x 32 ran 238.3 us, without
+// 237.3.)
 // ---------------------------------------------------------------------------
 // (down: Geo::steps of the site in the negative directions)
-template <class F>
+template <bool RO, class F>
 __device__ __forceinline__ Herm8<typename F::Real> clover_generator(const F& u,
                                                                     const ForceField<typename F::Real>& hf,
                                                                     const Geo& g, int s, const int down[4], int mu,
@@ -271,11 +276,12 @@ __device__ __forceinline__ Herm8<typename F::Real> clover_generator(const F& u,
     const int p = plane_index(mu, nu);
     const int d_mu = g.pick(down, mu), d_nu = g.pick(down, nu);
     const int s_mm = s + d_mu, s_mn = s + d_nu, s_mm_mn = s_mm + d_nu;
-    Herm8<R> back = hf.load_ro(p, s_mm);
-    herm_conj_add(u.load(nu, s_mm_mn), hf.load_ro(p, s_mm_mn), back);
-    Herm8<R> sum = hf.load_ro(p, s);
-    herm_conj_add(u.load(nu, s_mn), hf.load_ro(p, s_mn), sum);
-    herm_conj_add(u.load(mu, s_mm), back, sum);
+    auto generator = [&](int y) { return RO ? hf.load_ro(p, y) : hf.load(p, y); };
+    Herm8<R> back = generator(s_mm);
+    herm_conj_add(u.template load<RO>(nu, s_mm_mn), generator(s_mm_mn), back);
+    Herm8<R> sum = generator(s);
+    herm_conj_add(u.template load<RO>(nu, s_mn), generator(s_mn), sum);
+    herm_conj_add(u.template load<RO>(mu, s_mm), back, sum);
     return sum;
 }
 
@@ -289,13 +295,13 @@ __device__ __forceinline__ R herm_trace_mul(const Herm8<R>& a, const Herm8<R>& b
 }
 
 // Energy and charge of the plane pair k of site s, (01,23), (02,13) or (03,12).
-template <class F>
+template <bool RO = true, class F>
 __device__ __forceinline__ void clover_pair(const F& u, const ForceField<typename F::Real>& hf, const Geo& g, int s,
                                             const int c[4], int k, double& energy, double& topc) {
     int down[4];
     g.steps(c, -1, down);
-    const auto a = clover_generator(u, hf, g, s, down, 0, k + 1);
-    const auto b = clover_generator(u, hf, g, s, down, k == 0 ? 2 : 1, k == 2 ? 2 : 3);
+    const auto a = clover_generator<RO>(u, hf, g, s, down, 0, k + 1);
+    const auto b = clover_generator<RO>(u, hf, g, s, down, k == 0 ? 2 : 1, k == 2 ? 2 : 3);
     // Re tr(G_a G_b) = -4 tr(S_a S_b); the pairs' signs as in site_observables
     energy = -4.0 * (double(herm_trace_mul(a, a)) + double(herm_trace_mul(b, b)));
     const double t = 4.0 * double(herm_trace_mul(a, b));
@@ -324,6 +330,7 @@ __global__ void __launch_bounds__(96, CloverMinBlocks<F>::value)
     sums[0][threadIdx.x] = sums[1][threadIdx.x] = 0.0;
     const int k = int(threadIdx.x >> 5);
     const int items = (g.site1 - g.site0 + 31) / 32;
+    grid_wait();
     for (int item = blockIdx.x; item < items; item += gridDim.x) {
         const int s = g.site0 + item * 32 + int(threadIdx.x & 31);
         if (s >= g.site1) continue;
@@ -331,7 +338,7 @@ __global__ void __launch_bounds__(96, CloverMinBlocks<F>::value)
         g.coords(s, c);
         if (!g.interior(c)) continue;  // a block's halo sites are its neighbours'
         double e, t;
-        clover_pair(u, hf, g, s, c, k, e, t);
+        clover_pair<false>(u, hf, g, s, c, k, e, t);
         sums[0][threadIdx.x] += e;
         sums[1][threadIdx.x] += t;
     }
@@ -342,6 +349,7 @@ __global__ void __launch_bounds__(96, CloverMinBlocks<F>::value)
         if (j < nplaq) p += plaq[j];
     }
     block_sum3(p, energy, topc);
+    grid_release();
     if (threadIdx.x == 0) {
         partials[3 * blockIdx.x + 0] = p;
         partials[3 * blockIdx.x + 1] = energy;

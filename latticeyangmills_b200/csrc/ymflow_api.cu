@@ -293,8 +293,18 @@ cudaError_t enqueue_stage(ymflow_ctx* c, int stage, const void* in, void* out, d
     return launch_rk_stage(c->prec, stage, in, out, c->z, c->geo, eps, c->block, c->stream);
 }
 
+// Folds the `n` rows up to `last` whose partials enqueue_measure has left.
+static int fold_rows(ymflow_ctx* c, int last, int n) {
+    if (n == 0) return YMFLOW_OK;
+    const bool chained = !c->slab && !c->is_block;
+    YM_CK(c, launch_fold_rows(c->prec, plaq_range(c->geo, c->slab), c->geo, c->partials, n,
+                              c->meas + 4 * (last - n + 1), c->stream, chained),
+          "observables fold");
+    return YMFLOW_OK;
+}
+
 // Observables of the current field into meas row `row` (device).
-int enqueue_measure(ymflow_ctx* c, int row, bool rows_in) {
+int enqueue_measure(ymflow_ctx* c, int row, bool rows_in, int* pending) {
     int r = ensure_partials(c);
     if (r != YMFLOW_OK) return r;
     // Kernels of a whole lattice follow one another on its stream alone, so they
@@ -307,8 +317,11 @@ int enqueue_measure(ymflow_ctx* c, int row, bool rows_in) {
               "observables launch");
     } else if (measures_from_field(c)) {
         YM_CK(c, launch_measure_from_field(c->prec, c->u[c->cur], c->hfield, plaq_range(c->geo, c->slab), c->geo,
-                                           c->partials, c->meas + 4 * row, c->stream, rows_in, chained),
+                                           c->partials, pending ? *pending : 0, c->stream, rows_in, chained),
               "observables launch");
+        if (pending && ++*pending < kFoldRows) return YMFLOW_OK;
+        if ((r = fold_rows(c, row, pending ? *pending : 1)) != YMFLOW_OK) return r;
+        if (pending) *pending = 0;
     } else {
         YM_CK(c, launch_observables(c->prec, c->u[c->cur], c->geo, c->partials, c->stream), "observables launch");
         YM_CK(c, launch_obs_finalize(c->partials, obs_blocks(c->geo), c->geo, c->meas + 4 * row, c->stream),
@@ -774,7 +787,9 @@ int ymflow_flow(ymflow_ctx* c, double eps, int nsteps, int measure_every, int re
     if (reunit) YM_CK(c, cudaMemsetAsync(c->deviation, 0, sizeof(unsigned long long), c->stream), "reset drift");
     if ((r = slab_prepare(c)) != YMFLOW_OK) return r;
     int row = 0;
-    if ((r = enqueue_measure(c, row)) != YMFLOW_OK) return r;
+    int unfolded = 0;
+    int* const pending = c->slab || c->is_block ? nullptr : &unfolded;  // a slab's or block's row is summed over its group
+    if ((r = enqueue_measure(c, row, false, pending)) != YMFLOW_OK) return r;
     row_step[row] = c->step;
     row_t[row] = c->t;
     row++;
@@ -789,13 +804,14 @@ int ymflow_flow(ymflow_ctx* c, double eps, int nsteps, int measure_every, int re
         if (reunit && s % reunit_every == 0)
             YM_CK(c, launch_reunitarize(c->prec, c->u[c->cur], c->geo, c->deviation, c->stream), "reunitarise");
         if ((measure_every > 0 && s % measure_every == 0) || s == nsteps) {
-            if ((r = enqueue_measure(c, row, by_rows)) != YMFLOW_OK) return r;
+            if ((r = enqueue_measure(c, row, by_rows, pending)) != YMFLOW_OK) return r;
             row_step[row] = c->step;
             row_t[row] = c->t;
             row++;
             field_ready = from_field;
         }
     }
+    if ((r = fold_rows(c, row - 1, unfolded)) != YMFLOW_OK) return r;
     YM_CK(c, cudaMemcpyAsync(c->meas_host, c->meas, size_t(rows) * 4 * sizeof(double), cudaMemcpyDeviceToHost,
                              c->stream),
           "measurement copy");

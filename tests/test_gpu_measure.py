@@ -59,3 +59,19 @@ def test_measured_steps_flow_the_same_links(precision, graph):
     for rows, links in out[1:]:
         np.testing.assert_array_equal(links, out[0][1])
         np.testing.assert_array_equal(rows, out[0][0])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32_12"])
+@pytest.mark.parametrize("steps", [14, 15, 16, 32])
+def test_rows_folded_together(precision, steps):
+    """A call folds its rows 16 at a time: each row of a call of 15 (fewer than
+    a fold), 16, 17 and 33 rows is that of its step flowed in a call of its own."""
+    n = (8, 8, 8, 10)
+    with split_context(n, precision) as f, split_context(n, precision) as one:
+        f.init_links("expiah", 0.35, 5)
+        one.init_links("expiah", 0.35, 5)
+        rows = f.flow(0.01, steps, 1)
+        assert len(rows) == steps + 1
+        for k in range(steps):
+            apart = one.flow(0.01, 1, 1)
+            np.testing.assert_array_equal(rows[k : k + 2, 2:5], apart[:, 2:5])
