@@ -188,7 +188,7 @@ __device__ __forceinline__ double propose(uint32_t l0, uint32_t l1, uint32_t swe
     return beta_3 * double(dtr);
 }
 
-// G lanes per link of the (mu, parity) class (1, 4 or 8); link h's site is the
+// G lanes per link of the (mu, parity) class (1, 2, 4 or 8); link h's site is the
 // one of that parity in the x pair (2h, 2h + 1) (extents are even).  The lanes
 // of a link share its staples, then draw the next G proposals against the same
 // link, one each; the first accepted one is taken and the later ones are drawn
@@ -328,14 +328,28 @@ cudaError_t launch_metro_typed(void* u, const Geo& g, int mu, int parity, double
         return launch_chained(true, kernel, (links + per_block - 1) / per_block, kMetroThreads, st, F{u, g.V}, g, mu,
                               parity, beta / 3.0, eps, x0, hits, seed, sweep, accepted);
     };
-    // One thread per link needs about 15,000 links (three warps on each of the
-    // SM's schedulers, in all 148 SMs) before its work rather than its chain of
-    // hits sets the time; fewer links are given more lanes.  us per launch on
-    // B200 (FP64, 30 hits, each thread multiplying its own link) at 1 / 4 / 8
-    // lanes: 6^4 30 / 16 / 12, 8^4 31 / 16 / 14, 12^4 33 / 27 / 32, 16^4 53 / 60 /
-    // 75 (2 lanes are never the fastest).
-    if (links <= 4736) return launch(metropolis_kernel<F, 8>, 8);
-    if (links <= 14208) return launch(metropolis_kernel<F, 4>, 4);
+    // Few links leave the SMs short of warps, and a launch lasts as long as one
+    // link's chain of hits: more lanes per link draw more of the chain at once.
+    // Every count is the fastest until its blocks no longer fit the GPU at once
+    // (6 a SM at 168 registers, 148 SMs; 8 lanes until 2 a SM, where a hit of the
+    // narrower form is as short).  us per launch on B200 (30 hits) at 1 / 2 / 4
+    // / 8 lanes, FP64: 2048 links 33.1 / 22.1 / 15.1 / 13.7, 4096 33.1 / 22.1 /
+    // 16.1 / 16.8, 13824 34.9 / 28.4 / 25.4 / 36.3, 15552 35.1 / 28.9 / 35.5 /
+    // 42.9, 27648 45.4 / 37.8 / 45.5 / 65.0, 29376 46.8 / 53.2 / 52.7 / 68.8;
+    // FP32-12: 2048 27.3 / 18.5 / 13.4 / 11.5, 13824 28.0 / 24.0 / 21.5 / 30.3,
+    // 15552 28.0 / 24.3 / 25.5 / 32.5, 27648 36.4 / 31.0 / 39.4 / 49.3, 29376
+    // 36.6 / 37.9 / 40.2 / 51.7.
+    constexpr unsigned kSms = 148, kResident = 6 * kSms;
+    if (links <= 2 * kSms * (kMetroThreads / 8)) return launch(metropolis_kernel<F, 8>, 8);
+    if (links <= kResident * (kMetroThreads / 4)) return launch(metropolis_kernel<F, 4>, 4);
+    if (links <= kResident * (kMetroThreads / 2)) return launch(metropolis_kernel<F, 2>, 2);
+    // Past one wave of one-lane FP64 blocks the few blocks of the second take a
+    // chain's time alone; half as many links per block even that out until the
+    // second wave is a third full: 57344 links 88.3 / 81.7 us, 65536 99.5 / 89.1,
+    // 73728 102.0 / 92.9, but 90112 108.4 / 117.8.  (FP32 blocks fit 8 a SM and
+    // gain nothing: 77824 links 77.8 / 79.8.)
+    constexpr unsigned kWave = kResident * kMetroThreads;
+    if (sizeof(typename F::Real) == 8 && links > kWave && links <= kWave / 3 * 4) return launch(metropolis_kernel<F, 2>, 2);
     return launch(metropolis_kernel<F, 1>, 1);
 }
 

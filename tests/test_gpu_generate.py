@@ -129,3 +129,21 @@ def test_every_link_of_a_warp_accepting(oracle, n):
     assert oracle.gen_metropolis_cb(U, n, 0.0, EPS, 1, 5, 21) == 5 * 4 * oracle.volume(n)
     assert frac == 1.0
     assert np.abs(got - U).max() < 1e-12
+
+
+@pytest.mark.parametrize("beta", [BETA, 0.0])
+@pytest.mark.parametrize("n", [(8, 8, 8, 10), (14, 14, 14, 22), (16, 16, 16, 28)], ids=str)
+def test_lane_counts_at_larger_lattices(oracle, n, beta):
+    """4 lanes past the 8-lane range, one lane per link (a partial warp), and two
+    lanes past a wave of one-lane blocks: the oracle's chain (tolerance as above)."""
+    U = oracle.gen_cold(n)
+    oracle.gen_haar_mix(U, n, 0.3, 13, 0)
+    from latticeyangmills_b200 import GluonField
+
+    with GluonField(n, "fp64") as f:
+        f.upload(U)
+        frac = f.generate_metropolis(beta, EPS, 1, 3, 21, "current")
+        got = f.download()
+    acc = oracle.gen_metropolis_cb(U, n, beta, EPS, 1, 3, 21)
+    assert round(frac * 3 * 4 * oracle.volume(n)) == acc
+    assert np.abs(got - U).max() < 1e-12
