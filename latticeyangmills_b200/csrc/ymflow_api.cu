@@ -437,8 +437,11 @@ ymflow_ctx* ymflow_create(const int dims[4], int precision, int device, int* sta
     // (FP32-12) and 1.73 against 2.05 (FP64).  Where the FP64 plaquette field
     // (384 bytes per site) does not fit beside the links, FP64 keeps the fused
     // staple kernel.  FP32 lattices of at most 8192 sites, whose steps are
-    // bound by their launches, keep the one-launch fused kernel (8^4 FP32-12:
-    // 0.0164 against 0.0205 ms per step; from 12^4 on the two kernels win).  The one-kernel form with a tile's plane generators in
+    // bound by their launches, keep the one-launch fused kernel (FP32-12, us per
+    // step with one launch per stage / two: 8^3 x 12 17.3 / 18.5, 7 x 9 x 8 x 13
+    // 17.5 / 19.3, 10^4 21.8 / 20.1; measured every step the two kernels, whose
+    // field the measurement shares, are ahead there too, 29.1 / 23.8 at 8^3 x 12;
+    // up to kSmallSites every form is flow_small.cu's).  The one-kernel form with a tile's plane generators in
     // shared memory is prepared (its default tiling) for
     // YMFLOW_OPT_STAGE_FORM 2 and the autotuner, which times every form.
     if (r == YMFLOW_OK && prepare_tile_kernels(c->prec) != cudaSuccess) {
