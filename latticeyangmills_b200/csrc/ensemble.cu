@@ -1082,7 +1082,7 @@ ymflow_ens* ymflow_ensemble_create(int nconf, const int* dims, int precision, in
         e->signature += std::to_string(d[0]) + "x" + std::to_string(d[1]) + "x" + std::to_string(d[2]) + "x" +
                         std::to_string(d[3]) + ";";
     }
-    e->signature += "p" + std::to_string(precision);
+    e->signature += "p" + std::to_string(precision) + "d" + std::to_string(device);
     e->pool_links = uo;
     e->pool_force = zo;
     int r = YMFLOW_OK;
@@ -1100,6 +1100,8 @@ ymflow_ens* ymflow_ensemble_create(int nconf, const int* dims, int precision, in
             e->err.clear();
         }
     }
+    // forms 1 and 3 run only where the pool is: its ensembles share no choice with the others
+    if (!e->h) e->signature += "n";
     for (int c = 0; c < nconf; c++) {  // runs of consecutive configurations with equal extents
         const EnsConf& C = e->confs[c];
         if (c > 0 && std::equal(C.g.n, C.g.n + 4, e->confs[c - 1].g.n)) {
