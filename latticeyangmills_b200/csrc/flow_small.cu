@@ -14,8 +14,20 @@
 //
 // Bound by launch latency and by one wave's chain: loads, one loop's products
 // (4.5 warps per scheduler), a barrier, one link's exponential.  8^4 on B200,
-// us per step / per measured step: FP64 20.6 / 33.6 -> 14.5 / 23.5, FP32-12 (as
-// fused staple kernels) 16.4 / 28 -> 10.6 / 17.6.
+// us per step / per measured step: FP64 20.5 / 35.7 -> 15.1 / 23.8, FP32-12 (as
+// fused staple kernels) 17.4 / 27.5 -> 11.3 / 18.3.
+//
+// The stage's loops are multiplied out in all three rows.  Links drift from
+// SU(3) by their rounding (until a reunitarisation, FP64 ones for good), and a
+// loop whose row 2 is completed from the others carries that drift into its
+// generator (force_from_b_cdag).  The two-kernel stage completes its
+// plaquettes too, but takes a link's upper and lower loops from the same ones,
+// so that the error cancels along the lattice; loops completed one by one do
+// not: after 400 steps of eps = 0.01 from a = 0.35 without reunitarisation, at
+// 8^4, rms error of the links against the flow in higher precision 1.11e-15
+// (FP64) and 6.1e-7 (FP32) in two rows, 7.5e-16 and 4.3e-7 in three, 7.6e-16 and
+// 4.4e-7 in the two-kernel stage.  Two rows run 14.5 (FP64) and 10.7 us (FP32-12)
+// per step; the lower loops as transported plaquettes, as exact, 17.3 and 11.4.
 //
 // Every stage form of a configuration of at most kSmallSites sites runs this
 // kernel, whole lattices, slabs and blocks alike (the rule goes by the whole
@@ -29,7 +41,7 @@ namespace ym {
 namespace {
 
 // Generator of the loop x -> x-nu -> x-nu+mu -> x+mu -> x, begun with
-// U_nu(x-nu)^+ and closed with U_mu(x)^+ (clover leaf Q4).
+// U_nu(x-nu)^+ and closed with U_mu(x)^+ (clover leaf Q4), through two rows.
 template <class F>
 __device__ __forceinline__ Herm8<typename F::Real> lower_loop(const F& u, const Geo& g, int s, const int c[4], int mu,
                                                               int nu) {
@@ -40,6 +52,29 @@ __device__ __forceinline__ Herm8<typename F::Real> lower_loop(const F& u, const 
     mmul_rows2<true, false>(u.template load<false>(nu, w), u.template load<false>(mu, w), t);
     mmul_rows2<false, false>(t, u.template load<false>(nu, w_pm), b);
     return force_from_b2_cdag(b, u.template load<false>(mu, s));
+}
+
+// The stage's loops, every row multiplied out: the plaquette of plane (a, b) and
+// lower_loop's loop.
+template <class F>
+__device__ __forceinline__ Herm8<typename F::Real> stage_plaquette(const F& u, const Geo& g, int s, const int c[4],
+                                                                   int a, int b) {
+    using R = typename F::Real;
+    M3<R> t, x;
+    mmul<false, false>(u.template load<false>(a, s), u.template load<false>(b, g.hop_rt(s, g.coord(c, a), a, +1)), t);
+    mmul<false, true>(t, u.template load<false>(a, g.hop_rt(s, g.coord(c, b), b, +1)), x);
+    return force_from_b_cdag(x, u.template load<false>(b, s));
+}
+template <class F>
+__device__ __forceinline__ Herm8<typename F::Real> stage_lower_loop(const F& u, const Geo& g, int s, const int c[4],
+                                                                    int mu, int nu) {
+    using R = typename F::Real;
+    const int w = g.hop_rt(s, g.coord(c, nu), nu, -1);
+    const int w_pm = g.hop_rt(w, g.coord(c, mu), mu, +1);
+    M3<R> t, x;
+    mmul<true, false>(u.template load<false>(nu, w), u.template load<false>(mu, w), t);
+    mmul<false, false>(t, u.template load<false>(nu, w_pm), x);
+    return force_from_b_cdag(x, u.template load<false>(mu, s));
 }
 
 // Generators of the clover leaves Q2 and Q3 of plane (mu, nu) (observables.cu).
@@ -125,10 +160,10 @@ __global__ void __launch_bounds__(kStageThreads, 1)
     if (active) {
         if (w < 12) {
             const int mu = w / 3, k = w - 3 * mu;
-            loops.put(w, lane, lower_loop(in, g, s, c, mu, k + (k >= mu ? 1 : 0)));
+            loops.put(w, lane, stage_lower_loop(in, g, s, c, mu, k + (k >= mu ? 1 : 0)));
         } else {
             const int p = w - 12;
-            loops.put(w, lane, plane_generator<false>(in, g, s, c, plane_a(p), plane_b(p)));
+            loops.put(w, lane, stage_plaquette(in, g, s, c, plane_a(p), plane_b(p)));
         }
     }
     const int mu = w;

@@ -299,6 +299,38 @@ __device__ __forceinline__ Herm8<R> force_from_b2_cdag(const Rows2<R>& b, const 
     return z;
 }
 
+// The same generator with every row of X multiplied out, 108 multiply-adds, for
+// products whose unitarity is not to be relied on: with h the product's
+// deviation from it, the completed row 2 puts h's entries 02 and 12 into the
+// generator (which vanish for one link, but not for a product), the full
+// product only h times the field strength.
+template <class R>
+__device__ __forceinline__ Herm8<R> force_from_b_cdag(const M3<R>& b, const M3<R>& c) {
+    auto entry = [&](int i, int j) {  // (B C^+)_ij = sum_k b_ik conj(c_jk)
+        R re = R(0), im = R(0);
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            re = fma(b.e[i][k].re, c.e[j][k].re, re);
+            re = fma(b.e[i][k].im, c.e[j][k].im, re);
+            im = fma(b.e[i][k].im, c.e[j][k].re, im);
+            im = fma(-b.e[i][k].re, c.e[j][k].im, im);
+        }
+        return cx(re, im);
+    };
+    Herm8<R> z;
+    const R i0 = entry(0, 0).im, i1 = entry(1, 1).im, i2 = entry(2, 2).im;
+    const R mean = mul_rn(i0 + i1 + i2, R(1.0 / 3.0));
+    z.d0 = mean - i0;
+    z.d1 = mean - i1;
+    const Cx<R> x01 = entry(0, 1), x10 = entry(1, 0);
+    const Cx<R> x02 = entry(0, 2), x20 = entry(2, 0);
+    const Cx<R> x12 = entry(1, 2), x21 = entry(2, 1);
+    z.z01 = cx(R(-0.5) * (x01.im + x10.im), R(0.5) * (x01.re - x10.re));
+    z.z02 = cx(R(-0.5) * (x02.im + x20.im), R(0.5) * (x02.re - x20.re));
+    z.z12 = cx(R(-0.5) * (x12.im + x21.im), R(0.5) * (x12.re - x21.re));
+    return z;
+}
+
 // acc += v^+ h v for a Hermitian traceless h and v in SU(3) (Hermitian and
 // traceless again: its diagonal d0, d1 and upper triangle are formed).  With
 // d2 = h22, v^+ h v = v^+ (h - d2) v + d2, and h - d2 = A + A^+ for the upper
