@@ -239,11 +239,11 @@ YMFLOW_API int ymflow_get_option(const ymflow_ctx* ctx, int key, int64_t* value)
 
 /* The project's autotuner for one context (no counterpart in the reference,
  * whose stage is a fixed sequence of whole-lattice passes,
- * src/Apps/wilsonflow.cpp:141-172): times one RK3 stage in every form and
- * tiling the lattice allows (form 0, form 1, form 2 at every valid (ty, tz)),
- * keeps the fastest, and caches the choice for every context of the same
- * extents, precision and device in the process.  The current links are not
- * changed (stage 0 runs into the other buffer).  Forms agree to rounding, so
+ * src/Apps/wilsonflow.cpp:141-172): times unmeasured RK3 steps, launched as a
+ * flow's, in every form and tiling the lattice allows (form 0, form 1, form 2
+ * at every valid (ty, tz)), keeps the fastest, and caches the choice for every
+ * context of the same extents, precision and device in the process.  The
+ * current links are not changed (every stage runs into the other buffer).  Forms agree to rounding, so
  * a tuned flow can differ from the default one in the last bits.  Writes the
  * chosen form and tile (0, 0 unless form 2).  Not for slab contexts. */
 YMFLOW_API int ymflow_autotune(ymflow_ctx* ctx, double eps, int* stage_form, int* tile_y, int* tile_z);
@@ -383,9 +383,11 @@ YMFLOW_API int ymflow_ensemble_flow(ymflow_ens* ens, double eps, int nsteps, int
 YMFLOW_API int ymflow_ensemble_reset_time(ymflow_ens* ens);
 /* Device-timed RK3 steps of the whole ensemble (no measurements). */
 YMFLOW_API int ymflow_ensemble_time_steps(ymflow_ens* ens, double eps, int nsteps, float* elapsed_ms);
-/* The project's autotuner for an ensemble: times one RK3 stage of the whole
- * ensemble in each form it can take and keeps the fastest, cached for every
- * ensemble of the same sizes and precision in the process:
+/* The project's autotuner for an ensemble: times unmeasured RK3 steps of the
+ * whole ensemble, replayed as a flow's, in each form it can take and keeps the
+ * fastest, cached in the process for every ensemble of the same sizes,
+ * precision and device, those with a plane-generator pool apart from those
+ * without:
  *   - the per-link kernel (FP64) over persistent grids {one CTA per work
  *     item, 1x and 2x the resident CTAs};
  *   - the two-kernel stage, one block per 32-site item (FP64 ensembles where

@@ -171,19 +171,31 @@ bool steps_by_rows(const ymflow_ctx* c) {
 
 constexpr int kRowsIn = 1, kRowsOut = 2;
 
-// The launches of one RK3 step starting from u[from]: per stage the fused
+// The link buffers that the three stages of a step read and write.
+struct StageBuffers {
+    const void* in[3];
+    void* out[3];
+};
+
+// A step from u[from] into the other buffer.
+StageBuffers step_buffers(const ymflow_ctx* c, int from) {
+    void* const a = c->u[from];
+    void* const b = c->u[1 - from];
+    return {{a, b, a}, {b, a, b}};
+}
+
+// The launches of one RK3 step over `io`: per stage the fused
 // stage kernel, or the plaquette-field kernel and the stage kernel built on it
-// (stage_form 1).  field_ready: the plaquette field already holds u[from]'s
-// (stage 0 needs no field kernel).  rows (FP64, stage_form 1): bit 0, u[from]
+// (stage_form 1).  field_ready: the plaquette field already holds io.in[0]'s
+// (stage 0 needs no field kernel).  rows (FP64, stage_form 1): bit 0, io.in[0]
 // was written by a stage of the same call; bit 1, another step of the call
 // follows: the links between a call's steps, and between its stages, are
 // stored and read as their rows 0 and 1 (FieldD18Rows).  ev (optional): three events per stage, before the stage,
 // after its plaquette-field kernel (at once for the fused form) and after it.
-cudaError_t enqueue_step(ymflow_ctx* c, int from, double eps, cudaEvent_t* ev, bool field_ready, int rows) {
-    void* a = c->u[from];
-    void* b = c->u[1 - from];
-    const void* in[3] = {a, b, a};
-    void* out[3] = {b, a, b};
+cudaError_t enqueue_step(ymflow_ctx* c, const StageBuffers& io, double eps, cudaEvent_t* ev, bool field_ready,
+                         int rows) {
+    const void* const* in = io.in;
+    void* const* out = io.out;
     for (int s = 0; s < 3; s++) {
         if (ev) cudaEventRecord(ev[3 * s], c->stream);
         cudaError_t e = cudaSuccess;
@@ -237,6 +249,23 @@ int run_step_slab(ymflow_ctx* c, double eps, cudaEvent_t* ev, bool field_ready) 
     return YMFLOW_OK;
 }
 
+// The step over `io` as an executable graph (stage form 2).
+int capture_step(ymflow_ctx* c, const StageBuffers& io, double eps, cudaGraphExec_t* exec) {
+    cudaGraph_t g = nullptr;
+    YM_CK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal), "begin step capture");
+    cudaError_t le = enqueue_step(c, io, eps, nullptr, false, 0);
+    cudaError_t ee = cudaStreamEndCapture(c->stream, &g);
+    if (le != cudaSuccess) {
+        if (g) cudaGraphDestroy(g);
+        return cuda_fail(c, le, "stage launch during capture");
+    }
+    YM_CK(c, ee, "end step capture");
+    cudaError_t ie = cudaGraphInstantiate(exec, g, 0);
+    cudaGraphDestroy(g);
+    YM_CK(c, ie, "instantiate step graph");
+    return YMFLOW_OK;
+}
+
 // One RK3 step of the current field, step `s` of the `nsteps` (from 1) of a
 // call.  field_ready: the plaquette field holds the current links' (a
 // measurement has just been enqueued, and nothing has changed the links
@@ -255,25 +284,15 @@ int run_step(ymflow_ctx* c, double eps, int s, int nsteps, cudaEvent_t* ev, bool
         if (!c->graph[from] || c->graph_eps[from] != eps || c->graph_block[from] != c->block) {
             if (c->graph[from]) cudaGraphExecDestroy(c->graph[from]);
             c->graph[from] = nullptr;
-            cudaGraph_t g = nullptr;
-            YM_CK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal), "begin step capture");
-            cudaError_t le = enqueue_step(c, from, eps, nullptr, false, 0);
-            cudaError_t ee = cudaStreamEndCapture(c->stream, &g);
-            if (le != cudaSuccess) {
-                if (g) cudaGraphDestroy(g);
-                return cuda_fail(c, le, "stage launch during capture");
-            }
-            YM_CK(c, ee, "end step capture");
-            cudaError_t ie = cudaGraphInstantiate(&c->graph[from], g, 0);
-            cudaGraphDestroy(g);
-            YM_CK(c, ie, "instantiate step graph");
+            const int r = capture_step(c, step_buffers(c, from), eps, &c->graph[from]);
+            if (r != YMFLOW_OK) return r;
             c->graph_eps[from] = eps;
             c->graph_block[from] = c->block;
         }
         YM_CK(c, cudaGraphLaunch(c->graph[from], c->stream), "launch step graph");
     } else {
         const int rows = steps_by_rows(c) ? (s > 1 ? kRowsIn : 0) | (s < nsteps ? kRowsOut : 0) : 0;
-        YM_CK(c, enqueue_step(c, from, eps, ev, field_ready, rows), "stage launch");
+        YM_CK(c, enqueue_step(c, step_buffers(c, from), eps, ev, field_ready, rows), "stage launch");
     }
     c->cur = 1 - from;
     return YMFLOW_OK;
@@ -944,24 +963,36 @@ int ymflow_time_steps(ymflow_ctx* c, double eps, int nsteps, float* elapsed_ms, 
 
 namespace {
 
-// Milliseconds per stage-0 launch in the context's current form, stage 0
-// running from the current links into the other buffer: the current field
-// is untouched and the generator buffer only written (every step's stage 0
-// writes it before stages 1 and 2 read it).
-int time_stage0(ymflow_ctx* c, double eps, int reps, float* ms) {
-    const void* a = c->u[c->cur];
-    void* b = c->u[1 - c->cur];
-    auto launch = [&]() -> cudaError_t {
-        return enqueue_stage(c, 0, a, b, eps);
+// Milliseconds per unmeasured step in the context's current form, launched as
+// run_step launches the steps inside a call (chained; FP64 links as two rows;
+// form 2 replayed), but every stage running from the current links into the
+// other buffer: the current field is untouched and the generator buffer, which
+// every step's stage 0 writes, is scratch.
+int time_step(ymflow_ctx* c, double eps, float* ms) {
+    void* const a = c->u[c->cur];
+    void* const b = c->u[1 - c->cur];
+    const StageBuffers io = {{a, a, a}, {b, b, b}};
+    const int rows = steps_by_rows(c) ? kRowsIn | kRowsOut : 0;
+    cudaGraphExec_t exec = nullptr;
+    int r = YMFLOW_OK;
+    if (c->use_graph && c->stage_form == 2) r = capture_step(c, io, eps, &exec);
+    auto timed = [&](int reps) -> int {
+        YM_CK(c, cudaEventRecord(c->ev0, c->stream), "event record");
+        for (int i = 0; i < reps; i++)
+            YM_CK(c, exec ? cudaGraphLaunch(exec, c->stream) : enqueue_step(c, io, eps, nullptr, false, rows),
+                  "autotune launch");
+        YM_CK(c, cudaEventRecord(c->ev1, c->stream), "event record");
+        YM_CK(c, cudaEventSynchronize(c->ev1), "autotune timing");
+        YM_CK(c, cudaEventElapsedTime(ms, c->ev0, c->ev1), "elapsed time");
+        *ms /= float(reps);
+        return YMFLOW_OK;
     };
-    for (int i = 0; i < 2; i++) YM_CK(c, launch(), "autotune warm-up");
-    YM_CK(c, cudaEventRecord(c->ev0, c->stream), "event record");
-    for (int i = 0; i < reps; i++) YM_CK(c, launch(), "autotune launch");
-    YM_CK(c, cudaEventRecord(c->ev1, c->stream), "event record");
-    YM_CK(c, cudaEventSynchronize(c->ev1), "autotune timing");
-    YM_CK(c, cudaEventElapsedTime(ms, c->ev0, c->ev1), "elapsed time");
-    *ms /= float(reps);
-    return YMFLOW_OK;
+    if (r == YMFLOW_OK) r = timed(1);  // warm-up
+    if (r == YMFLOW_OK) r = timed(2);
+    // short steps again, enough of them to outlast the first launches' latency
+    if (r == YMFLOW_OK && *ms < 1.f) r = timed(20);
+    if (exec) cudaGraphExecDestroy(exec);
+    return r;
 }
 
 struct TuneChoice {
@@ -1006,6 +1037,7 @@ int ymflow_autotune(ymflow_ctx* c, double eps, int* stage_form, int* tile_y, int
     }
     const bool had_hfield = c->hfield != nullptr;
     std::vector<TuneChoice> cands = {{0, 0}, {1, 0}};
+    if (small_lattice(c->geo)) cands = {{c->stage_form == 1 ? 1 : 0, 0}};  // forms 0 and 1 run the same kernel
     for (int ty = 1; ty <= c->geo.n[1]; ty++)
         for (int tz = 1; tz <= c->geo.n[2]; tz++)
             for (int lpt : {1, 2, 4})
@@ -1029,7 +1061,7 @@ int ymflow_autotune(ymflow_ctx* c, double eps, int* stage_form, int* tile_y, int
             int r = apply(cands[i]);
             if (r != YMFLOW_OK) continue;  // e.g. no device memory for the plaquette field
             float ms = 0.f;
-            r = time_stage0(c, eps, 5, &ms);
+            r = time_step(c, eps, &ms);
             if (r != YMFLOW_OK) return r;
             if (tmin[i] < 0.f || ms < tmin[i]) tmin[i] = ms;
             if (!any || tmin[i] < best_ms) {
