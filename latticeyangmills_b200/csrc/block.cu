@@ -174,7 +174,7 @@ ymflow_ctx* ymflow_create_block(const int global_dims[4], const int origin[4], c
         vglobal *= global_dims[d];
     }
     if (vglobal >= (int64_t(1) << 31)) return bad("lattice volume must be below 2^31 sites");
-    ymflow_ctx* c = ymflow_create(local, precision, device, status);
+    ymflow_ctx* c = create_context(local, vglobal, precision, device, status);
     if (!c) return nullptr;
     c->is_block = true;
     c->tile_ok = false;  // the shared-memory stage is for whole lattices; blocks keep form 0 / 1

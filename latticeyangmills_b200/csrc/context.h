@@ -78,6 +78,9 @@ int cuda_fail(ymflow_ctx* c, cudaError_t e, const char* what);
         if (e_ != cudaSuccess) return ::ym::cuda_fail(ctx, e_, what); \
     } while (0)
 
+// A context of a lattice of extents `dims`: a whole configuration (config_sites
+// 0), or the local lattice of a part of one of `config_sites` sites.
+ymflow_ctx* create_context(const int dims[4], int64_t config_sites, int precision, int device, int* status);
 int ensure_meas(ymflow_ctx* c, int rows);
 // One RK3 stage (0, 1, 2) of the context's stage form from link buffer `in`
 // into `out` over all of the context's sites.

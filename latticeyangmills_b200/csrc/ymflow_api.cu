@@ -397,7 +397,11 @@ int ymflow_device_count(int* count) {
     return YMFLOW_OK;
 }
 
-ymflow_ctx* ymflow_create(const int dims[4], int precision, int device, int* status) {
+}  // extern "C"
+
+namespace ym {
+
+ymflow_ctx* create_context(const int dims[4], int64_t config_sites, int precision, int device, int* status) {
     auto set = [&](int s, const std::string& m) {
         if (status) *status = s;
         g_create_error = m;
@@ -455,12 +459,16 @@ ymflow_ctx* ymflow_create(const int dims[4], int precision, int device, int* sta
     // stored plaquette field: at 32^4 on B200 0.77 against 1.16 ms per step
     // (FP32-12) and 1.73 against 2.05 (FP64).  Where the FP64 plaquette field
     // (384 bytes per site) does not fit beside the links, FP64 keeps the fused
-    // staple kernel.  FP32 lattices of at most 8192 sites, whose steps are
-    // bound by their launches, keep the one-launch fused kernel (FP32-12, us per
-    // step with one launch per stage / two: 8^3 x 12 17.3 / 18.5, 7 x 9 x 8 x 13
-    // 17.5 / 19.3, 10^4 21.8 / 20.1; measured every step the two kernels, whose
-    // field the measurement shares, are ahead there too, 29.1 / 23.8 at 8^3 x 12;
-    // up to kSmallSites every form is flow_small.cu's).  The one-kernel form with a tile's plane generators in
+    // staple kernel.  FP32 configurations of at most 8192 sites, whose steps are
+    // bound by their launches, keep the one-launch fused kernel; by the whole
+    // configuration's volume, so that its slabs and blocks, however cut, take
+    // the same form as one another and as the whole lattice.  (us per step with
+    // one launch per stage / two, FP32-12: 8^3 x 12 16.7 / 17.5, 7 x 9 x 8 x 13 17.3 /
+    // 18.3, 10^4 21.0 / 19.9; FP32-18: 18.6 / 18.6, 19.2 / 19.7, 22.9 / 20.9.  The
+    // line is drawn for steps without a measurement: measured every step the
+    // two kernels, whose field the measurement shares, are ahead below it too,
+    // 29.3 / 22.9 and 30.7 / 24.1 at 8^3 x 12.  Up to kSmallSites forms 0 and 1 are
+    // flow_small.cu's.)  The one-kernel form with a tile's plane generators in
     // shared memory is prepared (its default tiling) for
     // YMFLOW_OPT_STAGE_FORM 2 and the autotuner, which times every form.
     if (r == YMFLOW_OK && prepare_tile_kernels(c->prec) != cudaSuccess) {
@@ -468,7 +476,7 @@ ymflow_ctx* ymflow_create(const int dims[4], int precision, int device, int* sta
         r = cuda_fail(c, e == cudaSuccess ? cudaErrorInvalidValue : e, "tile kernel set-up");
     }
     if (r == YMFLOW_OK) c->tile_ok = default_tile(c, &c->tile);
-    const bool launch_bound = c->prec != YMFLOW_FP64 && V <= 8192;
+    const bool launch_bound = c->prec != YMFLOW_FP64 && (config_sites > 0 ? config_sites : V) <= 8192;
     if (r == YMFLOW_OK && !launch_bound) {
         r = dev_alloc(c, &c->hfield, plane_field_bytes(c->prec, V), "plaquette field");
         if (r == YMFLOW_OK) {
@@ -489,6 +497,14 @@ ymflow_ctx* ymflow_create(const int dims[4], int precision, int device, int* sta
     }
     if (status) *status = YMFLOW_OK;
     return c;
+}
+
+}  // namespace ym
+
+extern "C" {
+
+ymflow_ctx* ymflow_create(const int dims[4], int precision, int device, int* status) {
+    return create_context(dims, 0, precision, device, status);
 }
 
 ymflow_ctx* ymflow_create_slab(const int global_dims[4], int t0, int nt, int precision, int device, int* status) {
@@ -519,7 +535,7 @@ ymflow_ctx* ymflow_create_slab(const int global_dims[4], int t0, int nt, int pre
         return nullptr;
     }
     const int local[4] = {global_dims[0], global_dims[1], global_dims[2], nt + 2};
-    ymflow_ctx* c = ymflow_create(local, precision, device, status);
+    ymflow_ctx* c = create_context(local, vs * global_dims[3], precision, device, status);
     if (!c) return nullptr;
     c->slab = true;
     c->geo.tile_groups = 0;  // the interior range starts at a halo slice: plain order
