@@ -21,8 +21,10 @@
 #include <atomic>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <system_error>
 #include <thread>
+#include <type_traits>
 
 namespace ym {
 
@@ -44,10 +46,11 @@ struct Slots {
     size_t earned = 0;     // see kEarnSlots
 };
 
-Slots& slots() {
-    static Slots* s = new Slots;  // never destroyed: contexts may outlive static destruction
-    return *s;
-}
+// Neither allocated (its first user is a C entry) nor destroyed (contexts may
+// outlive static destruction).
+static_assert(std::is_trivially_destructible<Slots>::value, "Slots outlives static destruction");
+Slots g_slots;
+Slots& slots() { return g_slots; }
 
 bool pinned_or_device(const void* p) {
     cudaPointerAttributes a;
@@ -89,7 +92,7 @@ cudaError_t upload_chunks(int device, char* dev, const char* host, size_t bytes,
     return e;
 }
 
-// One worker's chunks of a download; `ready` marks the device data.
+// One worker's chunks of a download.
 cudaError_t download_chunks(int device, char* host, const char* dev, size_t bytes, cudaStream_t st, char* slot, int w,
                             int n) {
     cudaError_t e = cudaSetDevice(device);
@@ -117,7 +120,8 @@ cudaError_t download_chunks(int device, char* host, const char* dev, size_t byte
 }
 
 // Runs chunks(w, n) on n workers, the calling thread among them; a thread that
-// cannot be started leaves its share to the caller.
+// cannot be started, for want of a thread or of memory, leaves its share to the
+// caller: no exception leaves through the C entries.
 template <class Chunks>
 cudaError_t on_workers(int n, const Chunks& chunks) {
     std::thread threads[kMaxWorkers];
@@ -130,6 +134,7 @@ cudaError_t on_workers(int n, const Chunks& chunks) {
         try {
             threads[w] = std::thread(work, w);
         } catch (const std::system_error&) {
+        } catch (const std::bad_alloc&) {
         }
     }
     work(0);
