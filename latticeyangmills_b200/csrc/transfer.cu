@@ -67,6 +67,20 @@ int workers_for(size_t bytes) {
     return std::max(1, std::min({kMaxWorkers, cores / 2, chunks}));
 }
 
+// Ends a worker's use of its slots: they are free for the next transfer once the
+// copies of its last two events are done, or, after an error, whatever the
+// stream holds (the failed call may have been the record of a copy's event).
+cudaError_t release_slots(cudaEvent_t done[2], cudaStream_t st, cudaError_t e) {
+    if (e != cudaSuccess) cudaStreamSynchronize(st);
+    for (int i = 0; i < 2; i++) {
+        if (!done[i]) continue;
+        const cudaError_t r = cudaEventSynchronize(done[i]);
+        if (e == cudaSuccess) e = r;
+        cudaEventDestroy(done[i]);
+    }
+    return e;
+}
+
 // One worker's chunks (w, w + n, w + 2 n, ...) of an upload.
 cudaError_t upload_chunks(int device, char* dev, const char* host, size_t bytes, cudaStream_t st, char* slot, int w,
                           int n) {
@@ -83,13 +97,7 @@ cudaError_t upload_chunks(int device, char* dev, const char* host, size_t bytes,
         e = cudaMemcpyAsync(dev + off, p, m, cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess) e = cudaEventRecord(done[k & 1], st);
     }
-    for (int i = 0; i < 2; i++) {  // the slots are free for the next transfer
-        if (!done[i]) continue;
-        const cudaError_t r = cudaEventSynchronize(done[i]);
-        if (e == cudaSuccess) e = r;
-        cudaEventDestroy(done[i]);
-    }
-    return e;
+    return release_slots(done, st, e);
 }
 
 // One worker's chunks of a download.
@@ -111,12 +119,7 @@ cudaError_t download_chunks(int device, char* host, const char* dev, size_t byte
         if (e == cudaSuccess) e = cudaEventSynchronize(done[k & 1]);
         if (e == cudaSuccess) std::memcpy(host + off, slot + size_t(k & 1) * kChunk, std::min(kChunk, bytes - off));
     }
-    for (int i = 0; i < 2; i++) {
-        if (!done[i]) continue;
-        cudaEventSynchronize(done[i]);  // a fetch in flight still writes its slot
-        cudaEventDestroy(done[i]);
-    }
-    return e;
+    return release_slots(done, st, e);  // a fetch in flight still writes its slot
 }
 
 // Runs chunks(w, n) on n workers, the calling thread among them; a thread that

@@ -142,7 +142,7 @@ def harness(tmp_path_factory):
     return d / "harness"
 
 
-@pytest.mark.parametrize("mode", ["plain", "no memory for a user", "no memory for threads"])
+@pytest.mark.parametrize("mode", ["plain", "no memory for a user", "no memory for threads", "no event record"])
 def test_transfers_are_exact_and_do_not_throw(harness, mode):
     res = subprocess.run([str(harness), mode], capture_output=True, text=True, timeout=120)
     assert res.returncode == 0, (res.returncode, res.stdout, res.stderr)
