@@ -36,7 +36,7 @@ launches, over the stage kernel's time in the uninstrumented steps, `frac`;
 the whole step's fraction, `step_frac_8d`; the DRAM bytes the ncu captures in
 profiles/ count, over the compulsory ones; `field_kernel` the plaquette-field
 kernel of the two-kernel stage on its own bytes),
-`alu_roofline` (the reference algorithm's flops over the step's kernel time,
+`alu_roofline` (the stage form's own flops over the step's kernel time,
 against the measured FP32 or FP64 FMA peak),
 `accuracy_vs_fp64` (t^2 E and Q at t = 4), `ensemble` (64 configurations of
 four sizes) and `cpu_baseline` (the reference's own code on one host core).
@@ -88,11 +88,14 @@ def split_bytes_per_link(prec: str):
     return su + 1.5 * sz, 2 * su + 1.5 * sz + 4 * sz / 3.0
 
 
-# Algorithmic flops of one link through one RK3 stage, as the reference's
-# algorithm counts them: 12 staple products + U Omega + Q^2 + e^{iQ} U, 198 flops
-# per 3x3 complex product, plus about 300 scalar flops (projection, RK combine,
-# tr Q^3, Cayley-Hamilton coefficients, f0 + f1 Q + f2 Q^2).
-FLOPS_PER_LINK_STAGE = 15 * 198 + 300
+# Flops of one link through one RK3 stage in each form, two per multiply-add of
+# the form's own algorithm.  Forms 1 and 2: 1.5 plaquette generators (two
+# two-row products, a completed row and the closing one: 263 each), three
+# transports (113 each), and the exponential, the update and the RK combination
+# (about 240).  Form 0: twelve staple products (108 each) and the entries of
+# U Omega (90) in place of the first two.
+FLOPS_PER_LINK_STAGE = {0: 2 * (12 * 108 + 90 + 240), 1: 2 * (1.5 * 263 + 3 * 113 + 240),
+                        2: 2 * (1.5 * 263 + 3 * 113 + 240)}
 
 
 STAGE_KERNELS = {
@@ -536,11 +539,11 @@ def our_arm(args, dist: Dist):
                       "design_bytes_per_launch": field_b * links, "avg_launch_ms_events": field_s * 1e3,
                       "design_frac": field_b * links / field_s / 1e9 / peak,
                       "share_of_kernel_time": field_ms / (field_ms + stage_ms)}
-    # arithmetic roofline: the reference algorithm's flops over the step's kernel
+    # arithmetic roofline: the stage form's own flops over the step's kernel
     # time, against the measured CUDA-core FMA peak
     fma_tf = ctypes.c_double(0.0)
     N.check(N.load().ymflow_fma_peak(dev, N.FP64 if prec == "fp64" else N.FP32_18, ctypes.byref(fma_tf)))
-    alu_achieved = links * FLOPS_PER_LINK_STAGE / (plain_ms / 1e3 / (3 * args.steps)) / 1e12
+    alu_achieved = links * FLOPS_PER_LINK_STAGE[form] / (plain_ms / 1e3 / (3 * args.steps)) / 1e12
 
     # accuracy of the mixed form against FP64 at t = 4 (400 steps), same seeded field
     accuracy = None
@@ -634,7 +637,7 @@ def our_arm(args, dist: Dist):
             "alu_roofline": {"bound": "fp64 fma" if prec == "fp64" else "fp32 fma", "achieved": alu_achieved,
                              "peak": fma_tf.value, "unit": "TFLOP/s", "frac": alu_achieved / fma_tf.value,
                              "peak_kind": "measured (ymflow_fma_peak, 8 independent FMA chains per thread)",
-                             "flops_per_link_update": 3 * FLOPS_PER_LINK_STAGE},
+                             "flops_per_link_update": 3 * FLOPS_PER_LINK_STAGE[form]},
             "accuracy_vs_fp64": accuracy,
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": nbytes / args.steps,
                     "d2h_bytes_per_step": rows_bytes / args.steps,

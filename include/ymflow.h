@@ -194,8 +194,10 @@ YMFLOW_API int ymflow_time_steps(ymflow_ctx* ctx, double eps, int nsteps, float*
 
 /* The same with the kernels of the two-kernel stage (YMFLOW_OPT_STAGE_FORM 1)
  * timed apart: field_ms (optional) receives the summed duration of the
- * plaquette-field kernels (0 for the fused form), stage_ms (optional) that of
- * the stage kernels, each from events around every launch. */
+ * plaquette-field kernels, stage_ms (optional) that of the stage kernels, each
+ * from events around every launch.  Stages without a plaquette-field kernel
+ * (forms 0 and 2, and configurations of at most 4736 sites in form 1) leave the
+ * gap between two events in field_ms, a few us per stage. */
 YMFLOW_API int ymflow_time_kernels(ymflow_ctx* ctx, double eps, int nsteps, float* elapsed_ms, float* field_ms,
                                    float* stage_ms);
 
@@ -219,6 +221,10 @@ YMFLOW_API int ymflow_time_kernels(ymflow_ctx* ctx, double eps, int nsteps, floa
  *       plaquette generators into shared memory, recompute the lower (y, z)
  *       faces, stream along t and finish the links from there (whole-lattice
  *       contexts only; ymflow_autotune times it against the others).
+ * A configuration of at most 4736 sites (one block of 32 per SM) runs the same
+ * kernel in forms 0 and 1, one launch per stage and one per measurement, with
+ * its own rounding; the option keeps the form that was set (form 1 also its
+ * field), without effect on such a flow.  Form 2 runs there as elsewhere.
  * YMFLOW_OPT_TILE: form 2's tiling, value = (lean << 36) | (lpt << 32) |
  * (ty << 16) | tz: ty must divide the y extent, tz the z extent, Lx ty must be
  * a multiple of 32 and Lx ty tz within 64..512 sites; each thread advances

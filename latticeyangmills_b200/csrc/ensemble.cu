@@ -436,7 +436,8 @@ struct EnsRunLaunch {
 };
 
 // One stage of one run: its plaquette-field launch (field: not where the pool
-// holds uin's already), then its stage launch, chained to it.
+// holds uin's already), then its stage launch (unchained, as the branches of
+// the step graph that they become).
 template <class F, class FO = F>
 static cudaError_t launch_ens_run_typed(int stage, void* uin, void* uout, void* z, void* h, const EnsRunLaunch& L,
                                         bool field, double eps, cudaStream_t st) {

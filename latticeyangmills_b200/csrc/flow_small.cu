@@ -29,7 +29,7 @@
 // 4.4e-7 in the two-kernel stage.  Two rows run 14.5 (FP64) and 10.7 us (FP32-12)
 // per step; the lower loops as transported plaquettes, as exact, 17.3 and 11.4.
 //
-// Every stage form of a configuration of at most kSmallSites sites runs this
+// Stage forms 0 and 1 of a configuration of at most kSmallSites sites run this
 // kernel, whole lattices, slabs and blocks alike (the rule goes by the whole
 // configuration's volume), so decomposed flows stay bit-identical to whole ones.
 #include "flow_device.cuh"

@@ -43,7 +43,7 @@ cudaError_t launch_chained(bool chained, void (*kernel)(P...), unsigned grid, un
     return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
-// Small configurations (flow_small.cu): every stage form and the observables
+// Small configurations (flow_small.cu): stage forms 0 and 1 and the observables
 // run one kernel each whose threads take one plaquette loop, instead of the
 // kernels below.  By the whole configuration's volume, so that its slabs and
 // blocks take the same.  The line is one block per SM (148 x 32 sites): past it

@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(kObsThreads, kObsMinBlocks)
 //   V = U_nu(x-nu),  W = U_mu(x-mu),  Y = U_nu(x-mu-nu):
 // three transports of 113 multiply-adds per plane in place of four products
 // of four links (about 1000).  Bound by latency and arithmetic (FP64 pipe at
-// about 53 %), not by HBM.  A measured step at 32^4 on B200 spends, beyond its
+// 54 %, 14 warps per SM waiting for loads), not by HBM (60 %).  A measured step at 32^4 on B200 spends, beyond its
 // six stage launches, 0.28 ms in FP64 (observables_kernel: 0.78), 0.15 in
 // FP32-18 (0.41) and 0.15 in FP32-12 (0.45): this kernel 0.250 / 0.135 / 0.135,
 // the sums in the field kernel 0.023 / 0.009 / 0.007 (the field itself is the

@@ -6,9 +6,11 @@
 // thread.  Here up to kMaxWorkers threads each move every n-th chunk through
 // two pinned slots of their own, so the copies to and from the slots (and the
 // page faults) run side by side while the DMA engine moves other chunks.  On a
-// B200 host with 16 cores, upload / download of a field in the .bin layout: 75.5
-// MB 6.0 / 15.4 -> 2.4 / 5.1 ms, 604 MB 54 / 124 -> 14 / 39 ms (chunks of 2 MB
-// 13 / 36, of 512 KB 20 / 43, at 32 and 8 MB of slots).
+// B200 host with 16 cores, upload of a field in the .bin layout / download into
+// a fresh array / into one whose pages are there: 75.5 MB 6.6-7.3 / 15-16 / 3.9-4.9
+// -> 2.2-2.4 / 3.6-4.7 / 2.5-3.0 ms, 604 MB 55-59 / 121-127 / 32-36 -> 14 / 35-38 /
+// 19-24 ms (604 MB in chunks of 2 MB 13 and, fresh, 36, of 512 KB 20 and 43, at 32
+// and 8 MB of slots).
 //
 // Transfers below kDirectBytes, from or to memory that is pinned already, and
 // those that find the slots in use by another thread's transfer go to the
