@@ -43,6 +43,7 @@ struct ymflow_ctx {
     std::vector<cudaEvent_t> events;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int block = 128;
+    int kernels_form = -1;            // the stage form whose kernels are loaded (load_flow_kernels)
     bool use_graph = true;
     bool loaded = false;
     int64_t step = 0;

@@ -108,19 +108,23 @@ static cudaError_t launch_ens_typed(int stage, void* uin, void* uout, void* z, c
     const R e = R(stage == 0 ? eps * 0.25 : eps);
     char *a = (char*)uin, *b = (char*)uout, *zz = (char*)z;
     if (grid >= nitems) {
+        auto flat = [&](auto kernel) {
+            return launch_chained(false, kernel, unsigned(nitems), unsigned(block), st, a, b, zz, confs, nconf, e);
+        };
         switch (stage) {
-            case 0: ens_flat_kernel<F, 0><<<nitems, block, 0, st>>>(a, b, zz, confs, nconf, e); break;
-            case 1: ens_flat_kernel<F, 1><<<nitems, block, 0, st>>>(a, b, zz, confs, nconf, e); break;
-            default: ens_flat_kernel<F, 2><<<nitems, block, 0, st>>>(a, b, zz, confs, nconf, e); break;
+            case 0: return flat(ens_flat_kernel<F, 0>);
+            case 1: return flat(ens_flat_kernel<F, 1>);
+            default: return flat(ens_flat_kernel<F, 2>);
         }
-        return cudaGetLastError();
     }
+    auto launch = [&](auto kernel) {
+        return launch_chained(false, kernel, unsigned(grid), unsigned(block), st, a, b, zz, confs, nconf, nitems, e);
+    };
     switch (stage) {
-        case 0: ens_stage_kernel<F, 0><<<grid, block, 0, st>>>(a, b, zz, confs, nconf, nitems, e); break;
-        case 1: ens_stage_kernel<F, 1><<<grid, block, 0, st>>>(a, b, zz, confs, nconf, nitems, e); break;
-        default: ens_stage_kernel<F, 2><<<grid, block, 0, st>>>(a, b, zz, confs, nconf, nitems, e); break;
+        case 0: return launch(ens_stage_kernel<F, 0>);
+        case 1: return launch(ens_stage_kernel<F, 1>);
+        default: return launch(ens_stage_kernel<F, 2>);
     }
-    return cudaGetLastError();
 }
 
 // The two-kernel stage over the work list: a 192-thread block per 32-site item
@@ -274,10 +278,12 @@ static cudaError_t launch_ens_measure_typed(void* u, void* h, const EnsConf* con
                                             double* partials, double* out, cudaStream_t st) {
     char *a = (char*)u, *hh = (char*)h;
     double* items = partials + 6 * int64_t(nitems);
-    ens_plaq_sum_kernel<F><<<plaq_item_blocks<F>(nitems), 192, 0, st>>>(a, hh, confs, nconf, nitems, partials);
-    ens_clover_kernel<F><<<nitems, 96, 0, st>>>(a, hh, confs, nconf, partials, items);
-    ens_fold_kernel<<<nconf, 256, 0, st>>>(confs, items, out);
-    return cudaGetLastError();
+    cudaError_t r = launch_chained(false, ens_plaq_sum_kernel<F>, plaq_item_blocks<F>(nitems), 192, st, a, hh, confs,
+                                   nconf, nitems, partials);
+    if (r == cudaSuccess)
+        r = launch_chained(false, ens_clover_kernel<F>, unsigned(nitems), 96, st, a, hh, confs, nconf, partials, items);
+    if (r == cudaSuccess) r = launch_chained(false, ens_fold_kernel, unsigned(nconf), 256, st, confs, items, out);
+    return r;
 }
 
 // Every configuration's row (out + 4 c) through the plane-generator pool h,
@@ -445,13 +451,17 @@ static cudaError_t launch_ens_run_typed(int stage, void* uin, void* uout, void* 
     const R e = R(stage == 0 ? eps * 0.25 : eps);
     const int items = L.r.nconf * L.r.nblk;
     char *a = (char*)uin + L.uoff, *b = (char*)uout + L.uoff, *zz = (char*)z + L.zoff, *hh = (char*)h + L.hoff;
-    if (field) ens_run_plaq_kernel<F><<<plaq_item_blocks<F>(items), 192, 0, st>>>(a, hh, L.r);
+    cudaError_t r = cudaSuccess;
+    if (field) r = launch_chained(false, ens_run_plaq_kernel<F>, plaq_item_blocks<F>(items), 192, st, a, hh, L.r);
+    if (r != cudaSuccess) return r;
+    auto launch = [&](auto kernel) {
+        return launch_chained(false, kernel, unsigned(items), 128, st, a, b, zz, hh, L.r, e);
+    };
     switch (stage) {
-        case 0: ens_run_split_kernel<F, 0, FO><<<items, 128, 0, st>>>(a, b, zz, hh, L.r, e); break;
-        case 1: ens_run_split_kernel<F, 1, FO><<<items, 128, 0, st>>>(a, b, zz, hh, L.r, e); break;
-        default: ens_run_split_kernel<F, 2, FO><<<items, 128, 0, st>>>(a, b, zz, hh, L.r, e); break;
+        case 0: return launch(ens_run_split_kernel<F, 0, FO>);
+        case 1: return launch(ens_run_split_kernel<F, 1, FO>);
+        default: return launch(ens_run_split_kernel<F, 2, FO>);
     }
-    return cudaGetLastError();
 }
 
 // What a two-kernel stage of an ensemble reads and leaves: field, as above;
@@ -694,6 +704,8 @@ struct ymflow_ens {
     int block = 128;
     int grid = 0;  // persistent CTAs (0: one per work item)
     bool use_graph = true;
+    bool graphs_fit = true;  // no step graph of this call was refused for want of memory
+    int kernels_form = -1;   // the form whose kernels are loaded (load_ens_kernels)
     bool tuned = false;
     bool form_chosen = false;  // set_tuning was called, or the first flow has settled the form
     std::vector<char> loaded;
@@ -712,7 +724,10 @@ int efail(ymflow_ens* e, int code, const std::string& m) {
     if (e) e->err = m;
     return code;
 }
-int ecuda(ymflow_ens* e, cudaError_t c, const char* what) { return efail(e, status_of(c), cuda_message(c, what)); }
+int ecuda(ymflow_ens* e, cudaError_t c, const char* what) {
+    cudaGetLastError();  // reported here: the next call's launches do not find it again
+    return efail(e, status_of(c), cuda_message(c, what));
+}
 
 #define YE_CK(ens, call, what)                                     \
     do {                                                           \
@@ -911,7 +926,8 @@ int capture_ens_step(ymflow_ens* e, const EnsBuffers& bufs, const EnsStepIo& ste
 
 // The steps that repeat within a call are replayed as graphs (one per buffer
 // and with or without a measurement before); its first and last are launched
-// as they are.
+// as they are, and all where there is no memory for a graph (a call that has
+// begun leaves FP64 links as two rows between its steps, so it goes on).
 int run_ens_step(ymflow_ens* e, double eps, int s, int nsteps, bool field_ready = false) {
     const int from = e->cur;
     EnsStepIo step;
@@ -922,22 +938,29 @@ int run_ens_step(ymflow_ens* e, double eps, int s, int nsteps, bool field_ready 
             step.rows_out = s < nsteps;
         }
     }
-    if (e->use_graph && s > 1 && s < nsteps) {
+    bool replayed = false;
+    if (e->use_graph && e->graphs_fit && s > 1 && s < nsteps) {
         EnsGraph& G = e->graphs[from + (step.field_ready ? 2 : 0)];
         if (!G.exec || G.eps != eps || G.block != e->block || G.grid != e->grid || G.io != step.key()) {
             if (G.exec) cudaGraphExecDestroy(G.exec);
             G.exec = nullptr;
             const int r = capture_ens_step(e, ens_step_buffers(e, from), step, eps, &G.exec);
-            if (r != YMFLOW_OK) return r;
+            if (r != YMFLOW_OK && r != YMFLOW_ERR_OOM) return r;
             G.eps = eps;
             G.block = e->block;
             G.grid = e->grid;
             G.io = step.key();
         }
-        YE_CK(e, cudaGraphLaunch(G.exec, e->stream), "launch step graph");
-    } else {
-        YE_CK(e, enqueue_ens_step(e, ens_step_buffers(e, from), step, eps), "stage launch");
+        const cudaError_t l = G.exec ? cudaGraphLaunch(G.exec, e->stream) : cudaErrorMemoryAllocation;
+        if (l != cudaSuccess && l != cudaErrorMemoryAllocation) return ecuda(e, l, "launch step graph");
+        replayed = l == cudaSuccess;
+        if (!replayed) {
+            cudaGetLastError();
+            e->err.clear();
+            e->graphs_fit = false;
+        }
     }
+    if (!replayed) YE_CK(e, enqueue_ens_step(e, ens_step_buffers(e, from), step, eps), "stage launch");
     e->cur = 1 - from;
     return YMFLOW_OK;
 }
@@ -1008,35 +1031,58 @@ void settle_form(ymflow_ens* e) {
     e->by_runs = sites >= kSitesPerRun * int64_t(e->runs.size());
 }
 
+// Loads the kernels of a call's steps and measurements (LoadOnly); the tile form's
+// were loaded when the ensemble was created.
+int load_ens_kernels(ymflow_ens* e) {
+    const int form = e->tile ? 2 : e->split ? (e->by_runs ? 3 : 1) : (e->grid > 0 ? 4 : 0);
+    if (form == 2 || e->kernels_form == form) return YMFLOW_OK;
+    const bool rows = e->prec == YMFLOW_FP64 && two_kernel_form(e);
+    LoadOnly load;
+    for (int i = 0; i < (rows ? 3 : 1); i++) {  // a call's first step, those inside it, its last
+        EnsStepIo step;
+        step.rows_in = rows && i > 0;
+        step.rows_out = rows && i < 2;
+        YE_CK(e, enqueue_ens_step(e, ens_step_buffers(e, e->cur), step, 0.0), "stage kernels");
+    }
+    for (int i = 0; i < (rows ? 2 : 1); i++) {
+        const int r = enqueue_ens_measure(e, 0, i == 1);
+        if (r != YMFLOW_OK) return r;
+    }
+    e->kernels_form = form;
+    return YMFLOW_OK;
+}
+
 void* conf_links(const ymflow_ens* e, int c) { return (char*)e->u[e->cur] + e->confs[c].uoff; }
 
 // Milliseconds per unmeasured step in the ensemble's current form, replayed as
 // run_ens_step replays the steps inside a call (FP64 two-kernel forms: links as
 // two rows), but every stage running from the current links into the other
-// pool: tuning does not disturb the flow state.  Negative: a launch failed.
-float time_ens_step(ymflow_ens* e, double eps) {
+// pool: tuning does not disturb the flow state.
+int time_ens_step(ymflow_ens* e, double eps, float* ms) {
     void* const a = e->u[e->cur];
     void* const b = e->u[1 - e->cur];
     EnsStepIo step;
     step.rows_in = step.rows_out = two_kernel_form(e);
     cudaGraphExec_t exec = nullptr;
-    if (capture_ens_step(e, {{a, a, a}, {b, b, b}}, step, eps, &exec) != YMFLOW_OK) return -1.f;
-    auto timed = [&](int reps) {
-        cudaEventRecord(e->ev0, e->stream);
+    const EnsBuffers io = {{a, a, a}, {b, b, b}};
+    int r = capture_ens_step(e, io, step, eps, &exec);
+    if (r == YMFLOW_ERR_OOM) r = YMFLOW_OK;  // launched directly, as a flow's then are
+    auto timed = [&](int reps) -> int {
+        YE_CK(e, cudaEventRecord(e->ev0, e->stream), "event record");
         for (int i = 0; i < reps; i++)
-            if (cudaGraphLaunch(exec, e->stream) != cudaSuccess) return -1.f;
-        cudaEventRecord(e->ev1, e->stream);
-        float ms = -1.f;
-        if (cudaEventSynchronize(e->ev1) != cudaSuccess || cudaEventElapsedTime(&ms, e->ev0, e->ev1) != cudaSuccess)
-            return -1.f;
-        return ms / float(reps);
+            YE_CK(e, exec ? cudaGraphLaunch(exec, e->stream) : enqueue_ens_step(e, io, step, eps), "tuning launch");
+        YE_CK(e, cudaEventRecord(e->ev1, e->stream), "event record");
+        YE_CK(e, cudaEventSynchronize(e->ev1), "tuning");
+        YE_CK(e, cudaEventElapsedTime(ms, e->ev0, e->ev1), "elapsed time");
+        *ms /= float(reps);
+        return YMFLOW_OK;
     };
-    float ms = timed(1);  // warm-up
-    if (ms >= 0.f) ms = timed(2);
+    if (r == YMFLOW_OK) r = timed(1);  // warm-up
+    if (r == YMFLOW_OK) r = timed(2);
     // short steps again, enough of them to outlast the first launches' latency
-    if (ms >= 0.f && ms < 1.f) ms = timed(20);
-    cudaGraphExecDestroy(exec);
-    return ms;
+    if (r == YMFLOW_OK && *ms < 1.f) r = timed(20);
+    if (exec) cudaGraphExecDestroy(exec);
+    return r;
 }
 
 }  // namespace
@@ -1283,6 +1329,8 @@ int ymflow_ensemble_flow(ymflow_ens* e, double eps, int nsteps, int measure_ever
     if (reunit) YE_CK(e, cudaMemsetAsync(e->deviation, 0, sizeof(unsigned long long), e->stream), "reset drift");
     int row = 0;
     settle_form(e);
+    e->graphs_fit = true;
+    if ((r = load_ens_kernels(e)) != YMFLOW_OK) return r;
     if ((r = enqueue_ens_measure(e, row, false)) != YMFLOW_OK) return r;
     rs[row] = e->step;
     rt[row] = e->t;
@@ -1345,8 +1393,10 @@ int ymflow_ensemble_time_steps(ymflow_ens* e, double eps, int nsteps, float* ela
     for (int c = 0; c < e->nconf; c++)
         if (!e->loaded[c]) return efail(e, YMFLOW_ERR_STATE, "configuration not loaded");
     DeviceGuard guard(e->device);
-    YE_CK(e, cudaEventRecord(e->ev0, e->stream), "event");
     settle_form(e);
+    e->graphs_fit = true;
+    if (const int r = load_ens_kernels(e)) return r;
+    YE_CK(e, cudaEventRecord(e->ev0, e->stream), "event");
     for (int s = 0; s < nsteps; s++) {
         int r = run_ens_step(e, eps, s + 1, nsteps);
         if (r != YMFLOW_OK) return r;
@@ -1425,8 +1475,9 @@ int ymflow_ensemble_autotune(ymflow_ens* e, double eps, int* block_out, int* gri
                 int r = set_block(e, ch.block);
                 if (r != YMFLOW_OK) return r;
             }
-            const float ms = time_ens_step(e, eps);
-            if (ms < 0.f) return ecuda(e, cudaGetLastError(), "tuning launch");
+            float ms = 0.f;
+            const int r = time_ens_step(e, eps, &ms);
+            if (r != YMFLOW_OK) return r;
             tmin[i] = std::min(tmin[i], ms);
             if (tmin[i] < best) {
                 best = tmin[i];

@@ -23,6 +23,21 @@ inline size_t plane_field_bytes(int prec, int64_t V) { return size_t(6 * padded_
 // whether field.cuh's 32-bit offsets (16-byte units) reach every link of V sites
 inline bool volume_addressable(int prec, int64_t V) { return link_field_bytes(prec, V) / 16 < (size_t(1) << 32); }
 
+// While one lives, launch_chained loads the kernels of this thread's launches and
+// launches none.  A kernel is loaded at its first use and needs device memory
+// then; a flow loads its own before its first step, so that a full device
+// refuses it with its links as they were.
+struct LoadOnly {
+    LoadOnly() { depth()++; }
+    ~LoadOnly() { depth()--; }
+    LoadOnly(const LoadOnly&) = delete;
+    LoadOnly& operator=(const LoadOnly&) = delete;
+    static int& depth() {
+        static thread_local int d = 0;
+        return d;
+    }
+};
+
 // Launches `kernel` so that it may start while the kernel before it on the
 // stream drains (programmatic dependent launch): its blocks are placed as the
 // other's finish (grid_release) and its index arithmetic runs; it waits
@@ -31,6 +46,10 @@ inline bool volume_addressable(int prec, int64_t V) { return link_field_bytes(pr
 template <class... P, class... A>
 cudaError_t launch_chained(bool chained, void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t st,
                            A... args) {
+    if (LoadOnly::depth() > 0) {
+        cudaFuncAttributes a;
+        return cudaFuncGetAttributes(&a, kernel);
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);

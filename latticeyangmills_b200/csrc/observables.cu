@@ -51,19 +51,16 @@ int obs_blocks(const Geo& g) {
 cudaError_t launch_observables(int prec, const void* u, const Geo& g, double* partials, cudaStream_t st) {
     const unsigned nb = unsigned(obs_blocks(g));
     if (nb == 0) return cudaErrorInvalidValue;
+    auto launch = [&](auto f) {
+        return launch_chained(false, observables_kernel<decltype(f)>, nb, kObsThreads, st, f, g, partials);
+    };
+    void* const links = const_cast<void*>(u);
     switch (prec) {
-        case kFP64:
-            observables_kernel<<<nb, kObsThreads, 0, st>>>(FieldD18{const_cast<void*>(u), g.V}, g, partials);
-            break;
-        case kFP32_18:
-            observables_kernel<<<nb, kObsThreads, 0, st>>>(FieldF18{const_cast<void*>(u), g.V}, g, partials);
-            break;
-        case kFP32_12:
-            observables_kernel<<<nb, kObsThreads, 0, st>>>(FieldF12{const_cast<void*>(u), g.V}, g, partials);
-            break;
+        case kFP64: return launch(FieldD18{links, g.V});
+        case kFP32_18: return launch(FieldF18{links, g.V});
+        case kFP32_12: return launch(FieldF12{links, g.V});
         default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
 }
 
 cudaError_t launch_obs_finalize(const double* partials, int nblocks, const Geo& g, double* out, cudaStream_t st,

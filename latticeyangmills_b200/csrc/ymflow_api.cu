@@ -27,7 +27,10 @@ int fail(ymflow_ctx* c, int code, const std::string& msg) {
     return code;
 }
 
-int cuda_fail(ymflow_ctx* c, cudaError_t e, const char* what) { return fail(c, status_of(e), cuda_message(e, what)); }
+int cuda_fail(ymflow_ctx* c, cudaError_t e, const char* what) {
+    cudaGetLastError();  // reported here: the next call's launches do not find it again
+    return fail(c, status_of(e), cuda_message(e, what));
+}
 
 }  // namespace ym
 
@@ -350,6 +353,24 @@ int enqueue_measure(ymflow_ctx* c, int row, bool rows_in, int* pending) {
     return YMFLOW_OK;
 }
 
+
+// Loads the kernels of a call's steps and measurements (LoadOnly): whole lattices
+// in forms 0 and 1.  (Form 2's were loaded when the context was created.)
+int load_flow_kernels(ymflow_ctx* c) {
+    if (c->slab || c->is_block || c->stage_form == 2 || c->kernels_form == c->stage_form) return YMFLOW_OK;
+    const bool by_rows = steps_by_rows(c);
+    LoadOnly load;
+    for (int rows : {kRowsOut, kRowsIn | kRowsOut, kRowsIn}) {  // a call's first step, those inside it, its last
+        YM_CK(c, enqueue_step(c, step_buffers(c, c->cur), 0.0, nullptr, false, by_rows ? rows : 0), "stage kernels");
+        if (!by_rows) break;
+    }
+    for (bool rows_in : {false, true}) {
+        const int r = enqueue_measure(c, 0, rows_in && by_rows);
+        if (r != YMFLOW_OK) return r;
+    }
+    c->kernels_form = c->stage_form;
+    return YMFLOW_OK;
+}
 
 void fill_obs(const ymflow_ctx* c, const double* m, int64_t step, double t, ymflow_obs* o) {
     o->step = int32_t(step);
@@ -821,6 +842,7 @@ int ymflow_flow(ymflow_ctx* c, double eps, int nsteps, int measure_every, int re
     if (r != YMFLOW_OK) return r;
     std::vector<int64_t> row_step(rows);
     std::vector<double> row_t(rows);
+    if ((r = load_flow_kernels(c)) != YMFLOW_OK) return r;
     const bool reunit = c->prec != YMFLOW_FP64 && reunit_every > 0;
     if (reunit) YM_CK(c, cudaMemsetAsync(c->deviation, 0, sizeof(unsigned long long), c->stream), "reset drift");
     if ((r = slab_prepare(c)) != YMFLOW_OK) return r;
@@ -932,6 +954,7 @@ int ymflow_time_kernels(ymflow_ctx* c, double eps, int nsteps, float* elapsed_ms
     if (!c->loaded) return fail(c, YMFLOW_ERR_STATE, "no links loaded");
     DeviceGuard guard(c->device);
     if (int r = slab_prepare(c)) return r;
+    if (int r = load_flow_kernels(c)) return r;
     const bool per_kernel = field_ms || stage_ms;
     const size_t nev = per_kernel ? size_t(9) * nsteps : 0;
     while (c->events.size() < nev) {
@@ -992,6 +1015,7 @@ int time_step(ymflow_ctx* c, double eps, float* ms) {
     cudaGraphExec_t exec = nullptr;
     int r = YMFLOW_OK;
     if (c->use_graph && c->stage_form == 2) r = capture_step(c, io, eps, &exec);
+    if (r == YMFLOW_ERR_OOM) r = YMFLOW_OK;  // launched directly
     auto timed = [&](int reps) -> int {
         YM_CK(c, cudaEventRecord(c->ev0, c->stream), "event record");
         for (int i = 0; i < reps; i++)
