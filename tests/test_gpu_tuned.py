@@ -28,7 +28,7 @@ def test_tuned_contexts_are_not_slower(n, precision):
         np.testing.assert_array_equal(tuned.download(), U)
         a, b = step_us(lambda k: plain.time_steps(0.01, k)[0], lambda k: tuned.time_steps(0.01, k)[0])
     print(n, precision, "untuned", a, "tuned", form, b)
-    assert b < 1.1 * a  # the clock's and the timing's spread
+    assert b < 1.2 * a  # the clock's and the host's spread; a wrong form costs 1.3 and more
 
 
 @pytest.mark.parametrize("sizes", [[(6, 6, 6, 6)] * 5, [(8, 8, 8, 8)] * 6 + [(6, 10, 12, 14)] * 4], ids=["one", "two"])
@@ -47,4 +47,4 @@ def test_tuned_ensembles_are_not_slower(sizes, precision):
         a, b = step_us(lambda k: plain.time_steps(0.01, k), lambda k: tuned.time_steps(0.01, k))
         forms = plain.tuning(), tuned.tuning()
     print(precision, "untuned", forms[0], a, "tuned", forms[1], b)
-    assert b < 1.1 * a
+    assert b < 1.2 * a
